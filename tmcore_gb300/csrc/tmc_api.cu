@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "tmc_ensemble.cuh"
+#include "tmc_fp64.cuh"
 #include "tmc_kernels.cuh"
 #include "tmc_mlp.cuh"
 #include "tmc_prep.h"
@@ -202,10 +203,12 @@ struct Engine : EngineBase {
   T* gd_e[2] = {};
   T* u[2] = {};
   T* Fq[2] = {};
+  double *sq[2] = {}, *hu[2] = {}, *ke[2] = {}, *ud[2] = {};  // FP64 path (StageIO)
+  double* ratio = nullptr;
   double *gd_acc = nullptr, *gd_tend = nullptr, *ghs = nullptr;
   T* q_acc = nullptr;
   T *iap_acc = nullptr, *iap_tend = nullptr, *E = nullptr;
-  T *pv_v = nullptr, *vor = nullptr, *gd_v = nullptr, *pv_c = nullptr, *v_e = nullptr, *pv_e = nullptr;
+  T *pv_v = nullptr, *vor = nullptr, *gd_v = nullptr, *pv_c = nullptr, *pv_e = nullptr;
   T *dpv = nullptr, *pvf = nullptr, *dpvf = nullptr;  // conservative APVM
   // generic integrators: tendency slots (gd FP64; iap_u and tracer mass in T)
   double* tgd[4] = {};
@@ -220,7 +223,8 @@ struct Engine : EngineBase {
   // per-member sizes (members are stored one after another)
   size_t qsz() const { return (size_t)h->M.nc * (h->O.n_tracers > 0 ? h->O.n_tracers : 1); }
   size_t fqsz() const {
-    return (h->O.n_tracers > 0 && h->O.tr_order >= 3) ? (size_t)h->M.ne * h->O.n_tracers : 1;
+    const bool edge_terms = h->O.tr_order >= 3 || std::is_same<T, double>::value;
+    return (h->O.n_tracers > 0 && edge_terms) ? (size_t)h->M.ne * h->O.n_tracers : 1;
   }
 
   int alloc() override {
@@ -250,7 +254,6 @@ struct Engine : EngineBase {
     vor = h->dalloc<T>(nv);
     gd_v = h->dalloc<T>(nv);
     pv_c = h->dalloc<T>(nc);
-    v_e = h->dalloc<T>(ne);
     pv_e = h->dalloc<T>(ne);
     if (!std::is_same<T, double>::value) {
       for (int i = 0; i < 3; ++i) {
@@ -259,6 +262,16 @@ struct Engine : EngineBase {
       }
     }
     if (!pv_e || !F[1] || !Fq[1]) return TMC_E_CUDA;
+    if (std::is_same<T, double>::value) {
+      for (int i = 0; i < 2; ++i) {
+        sq[i] = h->dalloc<double>(ne);
+        hu[i] = h->dalloc<double>(ne);
+        ke[i] = h->dalloc<double>(ne);
+        ud[i] = h->dalloc<double>(ne);
+        if (!sq[i] || !hu[i] || !ke[i] || !ud[i]) return TMC_E_CUDA;
+      }
+      if (!(ratio = h->dalloc<double>(nq))) return TMC_E_CUDA;
+    }
     if (h->O.pv_scheme == 2) {
       dpv = h->dalloc<T>(ne);
       pvf = h->dalloc<T>(ne);
@@ -323,12 +336,20 @@ struct Engine : EngineBase {
     s.u_nx = fuse ? u[1 - set] : nullptr;
     s.F_nx = fuse ? F[1 - set] : nullptr;
     s.Fq_nx = fuse ? Fq[1 - set] : nullptr;
+    s.sq = sq[set];
+    s.hu = hu[set];
+    s.ke = ke[set];
+    s.ud = ud[set];
+    s.sq_nx = sq[1 - set];
+    s.hu_nx = hu[1 - set];
+    s.ke_nx = ke[1 - set];
+    s.ud_nx = ud[1 - set];
+    s.ratio = ratio;
     s.E = E;
     s.pv_v = pv_v;
     s.vor = vor;
     s.gd_v = gd_v;
     s.pv_c = pv_c;
-    s.v_e = v_e;
     s.pv_e = pv_e;
     s.ghs = ghs;
     s.dpv = dpv;
@@ -1296,6 +1317,7 @@ int tmc_create(const tmc_mesh_desc* mesh, const tmc_params* params, tmc_handle**
     };
     std::vector<double> invA(hm.areaCell.size());
     for (size_t i = 0; i < invA.size(); ++i) invA[i] = 1.0 / hm.areaCell[i];
+    M.invAreaCell = h->upload(invA);
     M.weightsOnEdge_f = h->upload(f32(hm.weightsOnEdge));
     M.dcEdge_f = h->upload(f32(hm.dcEdge));
     M.dvEdge_f = h->upload(f32(hm.dvEdge));
@@ -1306,7 +1328,15 @@ int tmc_create(const tmc_mesh_desc* mesh, const tmc_params* params, tmc_handle**
     M.invAreaCell_f = h->upload(inv32(hm.areaCell));
     M.areaCell_f = h->upload(f32(hm.areaCell));
     M.areaTriangle_f = h->upload(f32(hm.areaTriangle));
-    M.invAreaCell = h->upload(invA);
+  } else {
+    auto inv64 = [](const std::vector<double>& v) {
+      std::vector<double> o(v.size());
+      for (size_t i = 0; i < v.size(); ++i) o[i] = f64::recip_host(v[i]);
+      return o;
+    };
+    M.invAreaCell = h->upload(inv64(hm.areaCell));
+    M.invAreaTriangle = h->upload(inv64(hm.areaTriangle));
+    M.invDcEdge = h->upload(inv64(hm.dcEdge));
   }
   M.cell2 = upload_stencil(h.get(), hm.cell2);
   M.cell3 = upload_stencil(h.get(), hm.cell3);
@@ -1656,12 +1686,12 @@ int tmc_time_integrate(tmc_handle* h, const double* gd_old, const double* iap_u_
       return h->cuda_check("H2D");
     cudaEventRecord(h->cev[1 + i], cs);
   }
-  // The step's edge preparation reads gd and iap_u only (second-order tracers
-  // are fluxed in the cell pass): with such tracers it runs before their
+  // The FP32 step's edge preparation reads gd and iap_u only (second-order
+  // tracers are fluxed in the cell pass): with such tracers it runs before their
   // copy has arrived, beside it.  Where the fused program allows (FP32, 1, 2
   // or 4 tracers), so does all of stage 1 but its tracer terms, which follow
   // the tracers' arrival.
-  const bool prep_early = trc && h->O.tr_order < 3 && !h->generic;
+  const bool prep_early = trc && h->O.tr_order < 3 && !h->generic && h->p.precision == TMC_FP32;
   const bool split = trc && h->eng->can_split();
   h->have_state = true;
   h->prep_valid = false;

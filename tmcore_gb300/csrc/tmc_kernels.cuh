@@ -73,7 +73,7 @@ struct DevMesh {
   // kUpW32 (null otherwise: the generic stencil loop runs)
   const int2* vert2_iw;
   // FP32 path: FP32-rounded copies of the metrics used in FP32 arithmetic
-  // and FP64 reciprocals of the areas used in FP64 arithmetic (null in FP64 mode)
+  // (null in FP64 mode)
   const float* weightsOnEdge_f;
   const float* dcEdge_f;
   const float* dvEdge_f;
@@ -84,7 +84,11 @@ struct DevMesh {
   const float* invAreaCell_f;
   const float* areaCell_f;
   const float* areaTriangle_f;
+  // FP64 reciprocals, rounded to nearest (invAreaCell in both modes; the FP64
+  // path divides by these metrics with f64::div_r)
   const double* invAreaCell;
+  const double* invAreaTriangle;
+  const double* invDcEdge;
   // vector reconstruction (history): coefficients [3][me][nc], cos/sin lat, lon [4][nc]
   const double* recon;
   const double* cell_trig;
@@ -182,8 +186,13 @@ struct StageIO {
   // intermediates
   T* gd_e;
   T* u;
-  T* F;   // u * gd_e
-  T* Fq;  // [ntr][ne]
+  T* F;   // u * gd_e (FP64 path: times dvEdge)
+  T* Fq;  // [ntr][ne] (FP64 path: every order, times dvEdge)
+  // FP64 path: sqrt(gd_e), (u/2)/sqrt(gd_e), u^2 areaEdge, u dcEdge, and the
+  // tracers' mixing ratios [ntr][nc] of the next stage's state
+  double *sq, *hu, *ke, *ud;
+  double *sq_nx, *hu_nx, *ke_nx, *ud_nx;
+  double* ratio;
   // the next stage's gd_e, u, F, Fq, written by k_edge_flux (stages 1-3) and
   // k_final_edges (next step): the edge preparation of the next stage fused
   // into the pass that produces its iap_u (null: not fused)
@@ -196,7 +205,6 @@ struct StageIO {
   T* vor;
   T* gd_v;
   T* pv_c;
-  T* v_e;
   T* pv_e;
   const double* ghs;
   // conservative APVM (pv_scheme 2): correction direction and the two
@@ -249,7 +257,6 @@ struct StageIO {
     s.vor = off(vor, v);
     s.gd_v = off(gd_v, v);
     s.pv_c = off(pv_c, c);
-    s.v_e = off(v_e, e);
     s.pv_e = off(pv_e, e);
     s.ghs = off(ghs, c);
     s.dpv = off(dpv, e);

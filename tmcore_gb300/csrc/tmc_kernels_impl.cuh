@@ -41,6 +41,7 @@
 
 #include <type_traits>
 
+#include "tmc_fp64.cuh"
 #include "tmc_kernels.cuh"
 
 namespace tmc {
@@ -126,6 +127,12 @@ __device__ __forceinline__ T met(const double* d, const float* f, size_t i) {
     return f[i];
 }
 
+// acc + a b of a global sum
+__device__ __forceinline__ float fma_acc(float a, float b, float acc) { return acc + a * b; }
+__device__ __forceinline__ double fma_acc(double a, double b, double acc) { return __fma_rn(a, b, acc); }
+__device__ __forceinline__ float halve(float x) { return 0.5f * x; }
+__device__ __forceinline__ double halve(double x) { return f64::half(x); }
+
 template <class T>
 __device__ __forceinline__ T sgn1(T x) {
   return copysign(T(1), x);
@@ -194,6 +201,10 @@ __device__ __forceinline__ void block_store_ff(const float (&hi)[N], const float
        ++_k, i += blockDim.x)                                                          \
     if (i < (n))
 
+// x / 12
+__device__ __forceinline__ float over12(float x) { return x / 12.f; }
+__device__ __forceinline__ double over12(double x) { return f64::div_r(x, 12.0, 1.0 / 12.0); }
+
 // Upwind correction of an edge value from two-sided polynomial-fit stencils
 // (operators_mod.F90:423-472 for cells, :359-412 for vertices).  `f(i)`
 // returns the field at stencil point i as T; ctr0/ctr1 are the two centres.
@@ -207,6 +218,7 @@ __device__ __forceinline__ T upwind_edge(const DStencil& S2, const DStencil& S4,
       const T fc = f(s == 0 ? ctr0 : ctr1);
       T acc = T(0);
       const int n = S2.count[(size_t)s * ne + e];
+#pragma unroll 4
       for (int j = 0; j < n; ++j) {
         const size_t k = ((size_t)j * 2 + s) * ne + e;
         acc = acc + T(S2.w[k]) * (f(S2.idx[k]) - fc);
@@ -216,7 +228,7 @@ __device__ __forceinline__ T upwind_edge(const DStencil& S2, const DStencil& S4,
       else
         d1 = acc;
     }
-    fe = fe - dist * dist * ((d0 + d1) - sgn1(sgn_of) * coef2 * (d1 - d0)) / T(12);
+    fe = fe - over12(dist * dist * ((d0 + d1) - sgn1(sgn_of) * coef2 * (d1 - d0)));
   } else if (order == 5 || order == 6) {
     T a0, a1, b0, b1;
 #pragma unroll
@@ -272,50 +284,100 @@ struct CellSrc {
   const float* gdf;
   const T* q;
   const float* qr;
+  const double* ratio;  // FP64: mixing ratios [ntr][nc], or null (divide q by gd)
 };
+
+// The edge quantities of a stage that an edge preparation writes.
+template <class T>
+struct EdgeSet {
+  T *gd_e, *u, *F, *Fq;
+  double *sq, *hu, *ke, *ud;  // FP64 path
+};
+template <class T>
+__device__ __forceinline__ EdgeSet<T> edge_set(const StageIO<T>& S) {
+  return {S.gd_e, S.u, S.F, S.Fq, S.sq, S.hu, S.ke, S.ud};
+}
+template <class T>
+__device__ __forceinline__ EdgeSet<T> next_edge_set(const StageIO<T>& S) {
+  return {S.gd_e_nx, S.u_nx, S.F_nx, S.Fq_nx, S.sq_nx, S.hu_nx, S.ke_nx, S.ud_nx};
+}
 
 // Edge preparation of one edge (operators_mod.F90:93-104 c2e, :423-472 upwind
 // correction with the sign of iap_u, :168-176 inverse IAP; the mass flux
 // u*gd_edge of tmcore_swm_mod.F90:135; for tracers of order >= 3 the sg11
 // edge value of adv_scheme_sg11_mod.F90:42-45 times the mass flux).
 // g1, g2 are the two cells' gd in T, already loaded by the caller.
+//
+// FP64: the terms that the cell, vertex and flux passes sum are formed here,
+// once per edge instead of once per use (two cells, two vertices, and the
+// flux pass's square root and quotient over again): the signed sums of those
+// passes take them with a sign flip, so the products' roundings are the
+// reference's.  F holds u gd_edge dvEdge, Fq the tracers' terms, ke u^2
+// areaEdge, ud u dcEdge, sq sqrt(gd_edge) and hu (u/2)/sqrt(gd_edge).  At
+// about 64 cycles per warp-wide FP64 instruction the extra 64 bytes per edge
+// are the cheaper side: a level-8 step with four tracers 5.29 -> 2.89 ms
+// with the reciprocal quotients (tmc_fp64.cuh).
+// ratios: C.ratio holds the tracers' mixing ratios of the two cells, else
+// they are divided here (a state set from outside).
 template <class T>
 __device__ __forceinline__ void prep_edge(const DevMesh& M, const ModelOpt& O, int e, int c1, int c2, T ia, T g1,
-                                          T g2, const CellSrc<T>& C, T* gd_e, T* u, T* F, T* Fq) {
-  T ge = T(0.5) * (g1 + g2);
-  if (O.adv_order >= 3) {
-    if constexpr (kF64<T>) {
+                                          T g2, const CellSrc<T>& C, const EdgeSet<T>& X) {
+  if constexpr (kF64<T>) {
+    double ge = f64::half(g1 + g2);
+    if (O.adv_order >= 3) {
       const double* gd = C.gd;
       ge = upwind_edge<T>(M.cell2, M.cell4, O.adv_order, T(O.cell_coef2), T(O.cell_coef4), M.ne, e, c1, c2, ge, ia,
                           M.dcEdge[e], [gd](int i) { return gd[i]; });
-    } else {
+    }
+    const double dv = M.dvEdge[e], dc = M.dcEdge[e], ae = M.areaEdge[e];
+    const f64::SqrtR sq = f64::sqrt_r(ge);
+    const double uu = f64::div_r(ia, sq.s, sq.r);
+    const double Fv = uu * ge;
+    X.gd_e[e] = ge;
+    X.u[e] = uu;
+    X.F[e] = Fv * dv;
+    X.sq[e] = sq.s;
+    X.hu[e] = f64::div_r(f64::half(uu), sq.s, sq.r);
+    X.ke[e] = uu * uu * ae;
+    X.ud[e] = uu * dc;
+    for (int k = 0; k < O.n_tracers; ++k) {
+      double qe;
+      if (C.ratio) {
+        const double* r = C.ratio + (size_t)k * M.nc;
+        qe = f64::half(r[c1] + r[c2]);
+      } else {
+        const double* q = C.q + (size_t)k * M.nc;
+        qe = f64::half(q[c1] / g1 + q[c2] / g2);
+      }
+      if (O.tr_order >= 3) {
+        const double* q = C.q + (size_t)k * M.nc;
+        const double* gd = C.gd;
+        qe = upwind_edge<T>(M.cell2, M.cell4, O.tr_order, T(O.tr_coef2), T(O.tr_coef4), M.ne, e, c1, c2, qe, ia, dc,
+                            [q, gd](int i) { return q[i] / gd[i]; });
+      }
+      X.Fq[(size_t)k * M.ne + e] = Fv * qe * dv;
+    }
+  } else {
+    T ge = T(0.5) * (g1 + g2);
+    if (O.adv_order >= 3) {
       const float* gd = C.gdf;
       ge = upwind_edge<T>(M.cell2, M.cell4, O.adv_order, T(O.cell_coef2), T(O.cell_coef4), M.ne, e, c1, c2, ge, ia,
                           M.dcEdge_f[e], [gd](int i) { return gd[i]; });
     }
-  }
-  const T sq = sqrt(ge);
-  const T uu = ia / sq;
-  const T Fv = uu * ge;
-  gd_e[e] = ge;
-  u[e] = uu;
-  F[e] = Fv;
-  // second-order tracers are fluxed by k_cell directly (no per-edge flux stored)
-  for (int k = 0; k < (O.tr_order >= 3 ? O.n_tracers : 0); ++k) {
-    T qe;
-    if constexpr (kF64<T>) {
-      const double* q = C.q + (size_t)k * M.nc;
-      const double* gd = C.gd;
-      qe = 0.5 * (q[c1] / g1 + q[c2] / g2);
-      qe = upwind_edge<T>(M.cell2, M.cell4, O.tr_order, T(O.tr_coef2), T(O.tr_coef4), M.ne, e, c1, c2, qe, ia,
-                          M.dcEdge[e], [q, gd](int i) { return q[i] / gd[i]; });
-    } else {
+    const T sq = sqrt(ge);
+    const T uu = ia / sq;
+    const T Fv = uu * ge;
+    X.gd_e[e] = ge;
+    X.u[e] = uu;
+    X.F[e] = Fv;
+    // second-order tracers are fluxed by k_cell directly (no per-edge flux stored)
+    for (int k = 0; k < (O.tr_order >= 3 ? O.n_tracers : 0); ++k) {
       const float* qr = C.qr + (size_t)k * M.nc;
-      qe = 0.5f * (qr[c1] + qr[c2]);
+      T qe = 0.5f * (qr[c1] + qr[c2]);
       qe = upwind_edge<T>(M.cell2, M.cell4, O.tr_order, T(O.tr_coef2), T(O.tr_coef4), M.ne, e, c1, c2, qe, ia,
                           M.dcEdge_f[e], [qr](int i) { return qr[i]; });
+      X.Fq[(size_t)k * M.ne + e] = Fv * qe;
     }
-    Fq[(size_t)k * M.ne + e] = Fv * qe;
   }
 }
 
@@ -334,7 +396,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_edge_prep(DevMesh M, ModelOpt O, 
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
   double en = 0.0;
-  const CellSrc<T> C{S.gd_in, S.gdf_in, S.q_in, S.qr_in};
+  const CellSrc<T> C{S.gd_in, S.gdf_in, S.q_in, S.qr_in, nullptr};
   TMC_FOR_EPT(e, M.ne) {
     const int c1 = M.cellsOnEdge[e], c2 = M.cellsOnEdge[M.ne + e];
     const T ia = S.iap_in[e];
@@ -346,7 +408,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_edge_prep(DevMesh M, ModelOpt O, 
       g1 = S.gdf_in[c1];
       g2 = S.gdf_in[c2];
     }
-    prep_edge<T>(M, O, e, c1, c2, ia, g1, g2, C, S.gd_e, S.u, S.F, S.Fq);
+    prep_edge<T>(M, O, e, c1, c2, ia, g1, g2, C, edge_set(S));
     if (diag) {
       if constexpr (kF64<T>)
         en = en + energy_term<T>(M, e, ia);
@@ -373,6 +435,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_cell(DevMesh M, ModelOpt O, Stage
   double mass = 0.0, enc = 0.0;
   TMC_FOR_EPT(c, M.nc) {
     double t;  // gd tendency, FP64 in both modes
+    double rA = 0.0;  // FP64: 1 / areaCell
     T tT, ke;
     int eidx[kME], cidx[kME];
     float nsg[kME];
@@ -388,18 +451,20 @@ __global__ void __launch_bounds__(kMaxBlock) k_cell(DevMesh M, ModelOpt O, Stage
       tprev = (mode >= 2) ? S.tendf[c] : 0.f;
     const double gdin = diag ? S.gd_in[c] : 0.0, ghsd = diag ? S.ghs[c] : 0.0;
     if constexpr (kF64<T>) {
-      // operators_mod.F90:40-55 (div_operator of u*gd_edge) and :206-221, in order
+      // operators_mod.F90:40-55 (div_operator of u*gd_edge) and :206-221, in
+      // order, from the edges' terms (prep_edge): one addition per edge and sum
       double s = 0.0, k = 0.0;
+#pragma unroll 6
       for (int i = 0; i < n; ++i) {
         const int e = M.edgesOnCell[(size_t)i * M.nc + c];
-        const double uu = S.u[e];
-        s = s + (double)M.nSign[(size_t)i * M.nc + c] * S.F[e] * M.dvEdge[e];
-        k = k + uu * uu * M.areaEdge[e];
+        s = s + f64::with_sign(S.F[e], M.nSign[(size_t)i * M.nc + c]);
+        k = k + S.ke[e];
       }
       const double A = M.areaCell[c];
-      t = (-s) / A;
+      rA = M.invAreaCell[c];
+      t = f64::div_r(-s, A, rA);
       tT = t;
-      ke = (k * 0.25) / A;
+      ke = f64::div_r(f64::half(f64::half(k)), A, rA);
       S.E[c] = ke + S.gd_in[c] + S.ghs[c];
       (void)eidx;
       (void)cidx;
@@ -450,18 +515,18 @@ __global__ void __launch_bounds__(kMaxBlock) k_cell(DevMesh M, ModelOpt O, Stage
           break;
         case 2:
         case 3: {
-          rip = rip + tprev * t * Ad;
-          S.gd_acc[c] = gacc + 2.0 * t;
+          rip = __fma_rn(tprev * t, Ad, rip);
+          S.gd_acc[c] = __fma_rn(2.0, t, gacc);  // 2 t is exact
           tb[c] = t;
           gnext = gold + rk.a_dt * t;
           S.gd_next[c] = gnext;
           break;
         }
         case 4: {
-          rip = rip + tprev * t * Ad;
-          const double tn = (gacc + t) / 6.0;
+          rip = __fma_rn(tprev * t, Ad, rip);
+          const double tn = f64::div_r(gacc + t, 6.0, 1.0 / 6.0);
           S.gd_acc[c] = tn;
-          r44 = r44 + tn * tn * Ad;
+          r44 = __fma_rn(tn * tn, Ad, r44);
           tb[c] = t;
           break;
         }
@@ -504,6 +569,9 @@ __global__ void __launch_bounds__(kMaxBlock) k_cell(DevMesh M, ModelOpt O, Stage
     }
     // tracers, kTr at a time: loads and divergences first, then the stores
     constexpr int kTr = 4;
+    double rg = 0.0;  // FP64: 1 / the next stage's gd
+    if constexpr (kF64<T>)
+      if (O.n_tracers > 0 && mode >= 1 && mode <= 3) rg = f64::recip(gnext);
     for (int q0 = 0; q0 < O.n_tracers; q0 += kTr) {
       T tq[kTr], qo[kTr], qa[kTr];
 #pragma unroll
@@ -517,27 +585,18 @@ __global__ void __launch_bounds__(kMaxBlock) k_cell(DevMesh M, ModelOpt O, Stage
         // Second-order tracers take the edge value from the two cells directly,
         // q_edge = (q(c1) + q(c2))/2, so no per-edge tracer flux is stored;
         // higher orders read the fluxes k_edge_prep wrote with the upwind
-        // correction.
-        const bool direct = (O.tr_order == 2);
+        // correction.  The FP64 path sums the edges' terms of prep_edge.
         if constexpr (kF64<T>) {
           double sq = 0.0;
-          const double qs = direct ? S.q_in[qi] / S.gd_in[c] : 0.0;
+#pragma unroll 6
           for (int i = 0; i < n; ++i) {
             const int e = M.edgesOnCell[(size_t)i * M.nc + c];
-            double flux;
-            if (direct) {
-              const int nb = M.cellsOnCell[(size_t)i * M.nc + c];
-              const double qn = S.q_in[(size_t)q * M.nc + nb] / S.gd_in[nb];
-              flux = S.F[e] * (0.5 * (qs + qn));
-            } else {
-              flux = S.Fq[(size_t)q * M.ne + e];
-            }
-            sq = sq + (double)M.nSign[(size_t)i * M.nc + c] * flux * M.dvEdge[e];
+            sq = sq + f64::with_sign(S.Fq[(size_t)q * M.ne + e], M.nSign[(size_t)i * M.nc + c]);
           }
-          tq[j] = (-sq) / M.areaCell[c];
+          tq[j] = f64::div_r(-sq, M.areaCell[c], rA);
         } else {
           float sq = 0.f;
-          if (direct) {
+          if (O.tr_order == 2) {
             const float qs = S.qr_in[qi];
 #pragma unroll
             for (int i = 0; i < kME; ++i) {
@@ -567,27 +626,33 @@ __global__ void __launch_bounds__(kMaxBlock) k_cell(DevMesh M, ModelOpt O, Stage
             break;
           case 2:
           case 3:
-            S.q_acc[qi] = qa[j] + T(2) * tq[j];
+            if constexpr (kF64<T>)
+              S.q_acc[qi] = __fma_rn(2.0, tq[j], qa[j]);
+            else
+              S.q_acc[qi] = qa[j] + T(2) * tq[j];
             qnext = qo[j] + adt * tq[j];
             if constexpr (kF64<T>) S.q_next[qi] = qnext;
             break;
           case 4:
             if constexpr (kF64<T>)
-              S.q_acc[qi] = (qa[j] + tq[j]) / 6.0;
+              S.q_acc[qi] = f64::div_r(qa[j] + tq[j], 6.0, 1.0 / 6.0);
             else
               S.q_acc[qi] = (qa[j] + tq[j]) * (1.0f / 6.0f);
             break;
           default:
             S.q_acc[qi] = tq[j];
         }
-        if constexpr (!kF64<T>) {
-          if (mode >= 1 && mode <= 3) S.qr_next[qi] = qnext / (float)gnext;
+        if (mode >= 1 && mode <= 3) {
+          if constexpr (kF64<T>)
+            S.ratio[qi] = f64::div_r(qnext, gnext, rg);
+          else
+            S.qr_next[qi] = qnext / (float)gnext;
         }
       }
     }
     if (diag) {
-      mass = mass + gdin * Ad;
-      enc = enc + (gdin * gdin + 2.0 * gdin * ghsd) * Ad;
+      mass = __fma_rn(gdin, Ad, mass);
+      enc = __fma_rn(gdin * __fma_rn(2.0, ghsd, gdin), Ad, enc);
     }
   }
   if (rk.mode >= 2) {
@@ -618,21 +683,20 @@ __global__ void __launch_bounds__(kMaxBlock) k_vertex(DevMesh M, ModelOpt O, Sta
 #pragma unroll
       for (int i = 0; i < 3; ++i)
         gv = gv + S.gd_in[M.cellsOnVertex[(size_t)i * M.nv + v]] * M.kite[(size_t)i * M.nv + v];
-      const double At = M.areaTriangle[v];
-      gv = gv / At;
+      const double At = M.areaTriangle[v], rAt = M.invAreaTriangle[v];
+      gv = f64::div_r(gv, At, rAt);
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const int e = M.edgesOnVertex[(size_t)i * M.nv + v];
-        s = s + (double)M.tSign[(size_t)i * M.nv + v] * S.u[e] * M.dcEdge[e];
-      }
-      const double vo = (-s) / At;
-      const double pv = (M.fVertex[v] + vo) / gv;
+      for (int i = 0; i < 3; ++i)
+        s = s + f64::with_sign(S.ud[M.edgesOnVertex[(size_t)i * M.nv + v]], M.tSign[(size_t)i * M.nv + v]);
+      const double vo = f64::div_r(-s, At, rAt);
+      const double ab = M.fVertex[v] + vo;
+      const double pv = f64::div_r(ab, gv, f64::recip(gv));
       S.pv_v[v] = pv;
       if (S.vor) S.vor[v] = vo;
       if (S.gd_v) S.gd_v[v] = gv;
       if (diag) {
-        pe = pe + gv * (pv * pv) * At;
-        av = av + (vo + M.fVertex[v]) * At;
+        pe = __fma_rn(ab * pv, At, pe);  // gd_vertex pv^2 areaTriangle
+        av = __fma_rn(ab, At, av);
       }
     }
   } else {
@@ -723,7 +787,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_edge_pv(DevMesh M, ModelOpt O, St
       v2[j] = e < M.ne ? M.verticesOnEdge[M.ne + e] : 0;
     }
 #pragma unroll
-    for (int j = 0; j < kEPT; ++j) pe[j] = T(0.5) * (S.pv_v[v1[j]] + S.pv_v[v2[j]]);
+    for (int j = 0; j < kEPT; ++j) pe[j] = halve(S.pv_v[v1[j]] + S.pv_v[v2[j]]);
 #pragma unroll
     for (int j = 0; j < kEPT; ++j) {
       const int e = e0 + j * blockDim.x;
@@ -734,15 +798,15 @@ __global__ void __launch_bounds__(kMaxBlock) k_edge_pv(DevMesh M, ModelOpt O, St
   TMC_FOR_EPT(e, M.ne) {
     const int v1 = M.verticesOnEdge[e], v2 = M.verticesOnEdge[M.ne + e];
     const T p1 = S.pv_v[v1], p2 = S.pv_v[v2];
-    T pe = T(0.5) * (p1 + p2);
+    T pe = halve(p1 + p2);
     T ve = T(0);
     if (need_v) {
       const int n = M.nEdgesOnEdge[e];
+#pragma unroll 5
       for (int i = 0; i < n; ++i) {
         const size_t k = (size_t)i * M.ne + e;
         ve = ve + S.u[M.edgesOnEdge[k]] * met<T>(M.weightsOnEdge, M.weightsOnEdge_f, k);
       }
-      if (S.v_e) S.v_e[e] = ve;
     }
     if (O.pv_scheme == 1) {
       if (O.apvm_weight != 0.0) {
@@ -831,7 +895,6 @@ __global__ void __launch_bounds__(256, TMC_UP32_MINB) k_edge_pv_up32(DevMesh M, 
   const float dist = __ldg(M.dvEdge_f + e);
   const float pe = 0.5f * (p1 + p2) -
                    dist * dist * ((d[0] + d[1]) - sgn1(ve) * (float)O.vert_coef2 * (d[1] - d[0])) / 12.f;
-  if (S.v_e) S.v_e[e] = ve;
   S.pv_e[e] = pe;
 }
 
@@ -1064,8 +1127,15 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
     // would wait a full memory round trip.
     const int c1 = M.cellsOnEdge[e], c2 = M.cellsOnEdge[M.ne + e];
     const T pe = S.pv_e[e];
-    const T uu = S.u[e];
-    const T ge = S.gd_e[e];
+    T uu = T(0), ge = T(0), sq = T(0), hu = T(0);
+    if constexpr (kF64<T>) {
+      sq = S.sq[e];
+      hu = S.hu[e];
+      if (O.adv_order >= 3) uu = S.u[e];
+    } else {
+      uu = S.u[e];
+      ge = S.gd_e[e];
+    }
     const T tp = (mode >= 2) ? S.iap_tend[e] : T(0);
     const T accv = (mode >= 2) ? S.iap_acc[e] : T(0);
     const T oldv = (mode >= 1 && mode <= 3) ? S.iap_old[e] : T(0);
@@ -1085,15 +1155,18 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
     T s = T(0), tge, dEdx, dc;
     if constexpr (kF64<T>) {
       // calc_tangent_vor_flux (operators_mod.F90:239-260), in order
+      // (its factor 1/2 taken out of the sum: powers of two round alike)
       const int n = M.nEdgesOnEdge[e];
+#pragma unroll 5
       for (int i = 0; i < n; ++i) {
         const size_t k = (size_t)i * M.ne + e;
         const int ep = M.edgesOnEdge[k];
-        s = s + M.weightsOnEdge[k] * S.u[ep] * S.gd_e[ep] * 0.5 * (pe + S.pv_e[ep]);
+        s = s + M.weightsOnEdge[k] * S.u[ep] * S.gd_e[ep] * (pe + S.pv_e[ep]);
       }
+      s = f64::half(s);
       dc = M.dcEdge[e];
-      dEdx = (S.E[c2] - S.E[c1]) / dc;
-      tge = 0.5 * (S.gd_tend[c1] + S.gd_tend[c2]);
+      dEdx = f64::div_r(S.E[c2] - S.E[c1], dc, M.invDcEdge[e]);
+      tge = f64::half(S.gd_tend[c1] + S.gd_tend[c2]);
     } else {
       int ep[kME2];
       float w[kME2];
@@ -1141,8 +1214,13 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
       }
     }
     // calc_u_tend_on_edge (tmcore_swm_mod.F90:155-201)
-    const T sq = sqrt(ge);
-    const T it = sq * ut + T(0.5) * uu / sq * tge;
+    T it;
+    if constexpr (kF64<T>) {
+      it = sq * ut + hu * tge;  // sqrt(gd_edge) and (u/2) / sqrt(gd_edge) of prep_edge
+    } else {
+      sq = sqrt(ge);
+      it = sq * ut + T(0.5) * uu / sq * tge;
+    }
     T* tb = S.iap_tend;
     T inext = T(0);  // iap_u of the next stage (update_state, tmcore_swm_mod.F90:210)
     switch (mode) {
@@ -1156,29 +1234,32 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
         break;
       case 2:
       case 3: {
-        rip = rip + tp * it * ae;
-        S.iap_acc[e] = accv + T(2) * it;
+        rip = fma_acc(tp * it, ae, rip);
+        if constexpr (kF64<T>)
+          S.iap_acc[e] = __fma_rn(2.0, it, accv);  // 2 t is exact
+        else
+          S.iap_acc[e] = accv + T(2) * it;
         tb[e] = it;
         inext = oldv + T(rk.a_dt) * it;
         break;
       }
       case 4: {
-        rip = rip + tp * it * ae;
+        rip = fma_acc(tp * it, ae, rip);
         T tn;
         if constexpr (kF64<T>)
-          tn = (accv + it) / 6.0;
+          tn = f64::div_r(accv + it, 6.0, 1.0 / 6.0);
         else
           tn = (accv + it) * (1.0f / 6.0f);
         S.iap_acc[e] = tn;
-        r44 = r44 + tn * tn * ae;
+        r44 = fma_acc(tn * tn, ae, r44);
         tb[e] = it;
         break;
       }
     }
     if (fuse) {
       // edge preparation of the next stage from its gd and iap_u
-      const CellSrc<T> C{S.gd_next, S.gdf_next, S.q_next, S.qr_next};
-      prep_edge<T>(M, O, e, c1, c2, inext, gn1, gn2, C, S.gd_e_nx, S.u_nx, S.F_nx, S.Fq_nx);
+      const CellSrc<T> C{S.gd_next, S.gdf_next, S.q_next, S.qr_next, S.ratio};
+      prep_edge<T>(M, O, e, c1, c2, inext, gn1, gn2, C, next_edge_set(S));
     } else if (mode >= 1 && mode <= 3) {
       S.iap_next[e] = inext;
     }
@@ -1227,6 +1308,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_final_cells(DevMesh M, ModelOpt O
     if constexpr (!kF64<T>) const_cast<float*>(S.gdf_in)[i] = (float)g[j];
   }
   T* qq = const_cast<T*>(S.q_old);
+  double rg[kEPT];  // FP64: 1 / gd
   for (int q = 0; q < O.n_tracers; ++q) {
     T qn[kEPT];
 #pragma unroll
@@ -1235,13 +1317,20 @@ __global__ void __launch_bounds__(kMaxBlock) k_final_cells(DevMesh M, ModelOpt O
       const size_t qi = (size_t)q * M.nc + i;
       qn[j] = i < M.nc ? qq[qi] + T(bdt) * S.q_acc[qi] : T(0);
     }
+    if constexpr (kF64<T>)
+      if (q == 0)
+#pragma unroll
+        for (int j = 0; j < kEPT; ++j) rg[j] = f64::recip(g[j]);
 #pragma unroll
     for (int j = 0; j < kEPT; ++j) {
       const int i = i0 + j * blockDim.x;
       if (i >= M.nc) continue;
       const size_t qi = (size_t)q * M.nc + i;
       qq[qi] = qn[j];
-      if constexpr (!kF64<T>) const_cast<float*>(S.qr_in)[qi] = qn[j] / (float)g[j];
+      if constexpr (kF64<T>)
+        S.ratio[qi] = f64::div_r(qn[j], g[j], rg[j]);
+      else
+        const_cast<float*>(S.qr_in)[qi] = qn[j] / (float)g[j];
     }
   }
 }
@@ -1258,7 +1347,7 @@ __global__ void __launch_bounds__(kB ? kMemberBlock : kMaxBlock, kB ? TMC_FINAL_
   const double* diag = kB ? diag0 + (size_t)blockIdx.y * kDiagStride : diag0;
   const double bdt = diag[9];
   double en = 0.0;
-  const CellSrc<T> C{S.gd_old, S.gdf_in, S.q_old, S.qr_in};
+  const CellSrc<T> C{S.gd_old, S.gdf_in, S.q_old, S.qr_in, S.ratio};
   // loads of all kEPT edges first (see k_final_cells)
   const int e0 = blockIdx.x * (kEPT * blockDim.x) + threadIdx.x;
   T* iap = const_cast<T*>(S.iap_old);
@@ -1289,10 +1378,10 @@ __global__ void __launch_bounds__(kB ? kMemberBlock : kMaxBlock, kB ? TMC_FINAL_
     const int e = e0 + j * blockDim.x;
     if (e >= M.ne) continue;
     iap[e] = ia[j];
-    prep_edge<T>(M, O, e, c1[j], c2[j], ia[j], g1[j], g2[j], C, S.gd_e, S.u, S.F, S.Fq);
+    prep_edge<T>(M, O, e, c1[j], c2[j], ia[j], g1[j], g2[j], C, edge_set(S));
     // energy_term (tmcore_swm_mod.F90:229) with areaEdge already loaded
     if constexpr (kF64<T>)
-      en = en + ia[j] * ia[j] * ae[j];
+      en = __fma_rn(ia[j] * ia[j], ae[j], en);
     else
       two_sum_acc(eh, el, ia[j] * ia[j] * ae[j]);
   }
