@@ -64,3 +64,33 @@ def test_tracer_terms_match_oracle(tracers, order):
     assert np.max(np.abs(a[0] / g.get_state()[0] - 0.75)) < 1e-14
     g.close()
     o.close()
+
+
+@pytest.mark.parametrize("level", [1, 4, 6])
+@pytest.mark.parametrize("scale", [1.0, 1e-60, 1e-140, 1e80])
+def test_invariants_match_exact_sums(level, scale):
+    """Mass, energy and absolute vorticity (integer block sums; FP64 sums for
+    extreme exponents) against exactly rounded sums of the same terms.  Terms
+    carry at most three roundings of 2^-53 and a thread adds four of them, so
+    16 2^-53 of the sum of magnitudes bounds the difference."""
+    import math
+
+    from tmcore_gb300.gpu import REF_OMEGA, REF_RADIUS, TMCoreGPU
+
+    m = mesh.icos_mesh(level)
+    gd, iap, ghs = _state(m, scale, False)
+    g = TMCoreGPU(m, dt=600.0, pv_scheme=1, apvm_weight=0.0)
+    g.set_initial(gd, np.zeros(m.nEdges), ghs)
+    g.set_state(gd, iap)
+    mass, energy, _, av = g.diag()[:4]
+    r2 = REF_RADIUS ** 2
+    A, Ae, At = m.areaCell * r2, (m.dvEdge * m.dcEdge) * r2, m.areaTriangle * r2
+    tol = 16 * 2.0 ** -53
+    t = gd * A
+    assert abs(mass - math.fsum(t)) <= tol * math.fsum(abs(t))
+    t = np.concatenate([(gd * gd + 2.0 * gd * ghs) * A, iap * iap * Ae])
+    assert abs(energy - math.fsum(t)) <= tol * math.fsum(abs(t))
+    _, vor = g.get_vertex()
+    t = (vor + 2.0 * REF_OMEGA * np.sin(m.latVertex)) * At
+    assert abs(av * math.fsum(At) - math.fsum(t)) <= tol * math.fsum(abs(t)) + 2.0 ** -51 * abs(math.fsum(t))
+    g.close()

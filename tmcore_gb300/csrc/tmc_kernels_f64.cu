@@ -15,39 +15,42 @@ struct FinalizeArgs {
   int split;  // blocks per region (1..kFinSplit)
 };
 
-// Fixed-order double-double sum of `count` per-block partials (hi, lo pairs),
-// by one block; lane 0 of warp 0 returns it.
-__device__ DD region_sum_pair(const double* reg, int count) {
+// The sum of `count` per-block partials (hi, lo pairs) by one block, as a
+// (hi, lo) pair in the lanes of warp 0: per-thread FP64 sums of a few
+// partials, then integer sums of the threads (f64::warp_sum).
+__device__ f64::HiLo region_sum_pair(const double* reg, int count) {
   double hi = 0.0, lo = 0.0;
   for (int i = threadIdx.x; i < count; i += blockDim.x) {
     hi = __dadd_rn(hi, reg[2 * i]);
     lo = __dadd_rn(lo, reg[2 * i + 1]);
   }
-  __shared__ DD sm[32];
+  __shared__ double sm[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  DD w = warp_reduce_dd(DD{hi, lo});
-  if (lane == 0) sm[warp] = w;
-  __syncthreads();
-  if (warp == 0) {
-    w = (lane < nw) ? sm[lane] : DD{0.0, 0.0};
-    w = warp_reduce_dd(w);
+  const f64::HiLo w = f64::split(f64::warp_sum(hi));
+  const double l = f64::value(f64::warp_sum(lo));
+  if (lane == 0) {
+    sm[warp] = w.hi;
+    sm[16 + warp] = w.lo + l;
   }
-  return w;
+  __syncthreads();
+  f64::HiLo out{0.0, 0.0};
+  if (warp == 0) out = f64::split(f64::warp_sum((lane & 15) < nw ? sm[lane] : 0.0));
+  return out;
 }
 __device__ double region_sum_dd(const double* reg, int count) {
-  const DD w = region_sum_pair(reg, count);
+  const f64::HiLo w = region_sum_pair(reg, count);
   return w.hi + w.lo;
 }
 
 // a.split blocks per partial region (kFinSplit for one model, fewer for a
-// batch of members), each a fixed-order double-double reduction of a contiguous
-// 1/a.split of the region's per-block partials into P.fin; the last block to
-// finish (atomic counter, no waiting) combines each region's a.split sums in
-// order (one thread per region), then the
+// batch of members), each the sum of a contiguous 1/a.split of the region's
+// per-block partials into P.fin; the last block to finish (atomic counter, no
+// waiting) combines each region's a.split sums (a warp per region) and the
 // region sums into beta and the invariants (time_scheme_mod.F90:144-150;
-// tmcore_swm_mod.F90:215-255), and re-arms the counter.  With one block per
-// region the widest region (15,360 partials at level 9) cost ~15,000 cycles
-// of one SM's 2-lane FP64 pipe, and the launch 28 us.
+// tmcore_swm_mod.F90:215-255), and re-arms the counter.  The sums across
+// lanes are exact integer sums: with double-double shuffle trees on the
+// 2-lane FP64 pipe this launch took 24 us at every mesh size; a level-6 FP32
+// step went from 118.3 to 102.8 us with the integer sums.
 __global__ void __launch_bounds__(256) k_finalize(Partials P0, FinalizeArgs a, double* out0, double* res0,
                                                   unsigned int* counter0) {
   // one member per blockIdx.y: its partials, outputs, region sums and counter
@@ -61,7 +64,7 @@ __global__ void __launch_bounds__(256) k_finalize(Partials P0, FinalizeArgs a, d
   if (want) {
     const int count = a.counts[r], chunk = (count + a.split - 1) / a.split;
     const int i0 = min(count, part * chunk), i1 = min(count, i0 + chunk);
-    const DD v = region_sum_pair(P.region(r) + 2 * (size_t)i0, i1 - i0);
+    const f64::HiLo v = region_sum_pair(P.region(r) + 2 * (size_t)i0, i1 - i0);
     if (threadIdx.x == 0) {
       P.fin[2 * (r * kFinSplit + part)] = v.hi;
       P.fin[2 * (r * kFinSplit + part) + 1] = v.lo;
@@ -76,22 +79,28 @@ __global__ void __launch_bounds__(256) k_finalize(Partials P0, FinalizeArgs a, d
   if (!last) return;
   __threadfence();
   __shared__ double rs[kFinalizeRegions];
-  if (threadIdx.x < kFinalizeRegions) {
-    const int q = threadIdx.x;
-    DD acc{0.0, 0.0};
-    if ((q <= R_44_E) ? a.step : a.diag)
-      for (int k = 0; k < a.split; ++k)  // L2 loads: the other blocks wrote them
-        acc = dd_add(acc, DD{__ldcg(P.fin + 2 * (q * kFinSplit + k)), __ldcg(P.fin + 2 * (q * kFinSplit + k) + 1)});
-    rs[q] = acc.hi + acc.lo;
-    res[q] = rs[q];
+  static_assert(2 * kFinSplit <= 32, "a warp combines one region's sums");
+  const int lane = threadIdx.x & 31;
+  for (int q = threadIdx.x >> 5; q < kFinalizeRegions; q += blockDim.x >> 5) {
+    const bool on = ((q <= R_44_E) ? a.step : a.diag) && lane < 2 * a.split;
+    // L2 loads: the other blocks wrote them
+    const double s = f64::value(f64::warp_sum(on ? __ldcg(P.fin + 2 * q * kFinSplit + lane) : 0.0));
+    if (lane == 0) rs[q] = res[q] = s;
   }
   __syncthreads();
-  if (threadIdx.x != 0) return;
+  if (threadIdx.x >= 32) return;
   const double* rv = rs;
+  // lane k: R[k] = <t_k, t_k+1> (k < 3), R[3] = <t_new, t_new>
+  double Rk = 0.0;
   if (a.step) {
-    double R[4];
-    for (int k = 0; k < 3; ++k) R[k] = (rv[R_IP_E + 2 * k] + rv[R_IP_C + 2 * k]) / a.totalArea;
-    R[3] = (rv[R_44_E] + rv[R_44_C]) / a.totalArea;
+    const int re = lane < 3 ? R_IP_E + 2 * lane : R_44_E, rc = lane < 3 ? R_IP_C + 2 * lane : R_44_C;
+    Rk = (rv[re] + rv[rc]) / a.totalArea;
+  }
+  double R[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) R[k] = __shfl_sync(0xffffffffu, Rk, k);
+  if (threadIdx.x != 0) return;
+  if (a.step) {
     double beta = 1.0;
     if (a.conserve) {
       if (a.scheme == 1)  // CRK3: R[0] = <t1,t2>, R[1] = <t1,t3>, R[2] = <t2,t3>
@@ -136,9 +145,8 @@ void launch_finalize(Partials P, const int* counts_host, double totalArea, doubl
   // would leave one block's FP64 additions on one SM's 2-lane FP64 pipe, so
   // each region is split over kFinSplit blocks.  A batch of members already
   // has a block per region and member; splitting it as much multiplies the
-  // blocks' fixed cost of a double-double block reduction (512 level-6
-  // members: 0.2 -> 4 ms per step), so the split shrinks with the members
-  // (about kFinSplit x the regions' blocks in all).
+  // blocks' fixed cost, so the split shrinks with the members (about
+  // kFinSplit x the regions' blocks in all).
   const int nm = members > 1 ? members : 1;
   a.split = kFinSplit / nm > 1 ? kFinSplit / nm : 1;
   // scratch after the kDiagLen outputs: R_COUNT region sums, then the counter

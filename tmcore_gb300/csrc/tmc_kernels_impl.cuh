@@ -52,40 +52,24 @@ constexpr int kCellBlock = 256;    // block size limit of the FP32 cell pass (re
 constexpr int kME = 6;    // unrolled maxEdges of the FP32 path
 constexpr int kME2 = 10;  // unrolled maxEdges2 of the FP32 path
 
-// ---------------------------------------------------------------------------
-// double-double accumulation (Knuth TwoSum), never contracted into FMA
-// ---------------------------------------------------------------------------
-struct DD {
-  double hi, lo;
-};
-__device__ __forceinline__ DD dd_add(DD a, DD b) {
-  double s = __dadd_rn(a.hi, b.hi);
-  double bb = __dsub_rn(s, a.hi);
-  double e = __dadd_rn(__dsub_rn(a.hi, __dsub_rn(s, bb)), __dsub_rn(b.hi, bb));
-  e = __dadd_rn(e, __dadd_rn(a.lo, b.lo));
-  double hi = __dadd_rn(s, e);
-  double lo = __dsub_rn(e, __dsub_rn(hi, s));
-  return {hi, lo};
-}
-__device__ __forceinline__ DD warp_reduce_dd(DD v) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    DD o;
-    o.hi = __shfl_down_sync(0xffffffffu, v.hi, off);
-    o.lo = __shfl_down_sync(0xffffffffu, v.lo, off);
-    v = dd_add(v, o);
-  }
-  return v;
-}
-
 // Reduce N per-thread partial sums over the block and store region[r[k]][block]
-// as (sum, 0).  Warps sum their lanes with a shuffle tree in A (double or
-// float), warp 0 sums the warp sums the same way; the compensated
-// (double-double) combination happens across blocks in k_finalize.  No
-// double-double arithmetic here: warp 0 of every block sits on the same SM
-// sub-partition, and GB300 issues FP64 at 1/64 of the FP32 rate, so a
-// double-double tail per block serialises behind the whole kernel.  Every
-// thread of the block must call this (it synchronises).
+// as (sum, 0).  FP32 sums: warps sum their lanes with a shuffle tree, warp 0
+// sums the warp sums the same way.  FP64 sums: both levels in integers
+// (f64::warp_sum), which leaves the FP64 pipe to the kernel's arithmetic: a
+// shuffle tree costs five warp-wide FP64 instructions per warp and value, and
+// warp 0 of every block sits on the same SM sub-partition, so an FP64 tail per
+// block serialises behind the whole kernel.  The combination across blocks is
+// k_finalize's.  Every thread of the block must call this (it synchronises).
+template <class A>
+__device__ __forceinline__ A lanes_sum(A w) {
+  if constexpr (sizeof(A) == 8) {
+    return f64::value(f64::warp_sum(w));
+  } else {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) w += __shfl_down_sync(0xffffffffu, w, off);
+    return w;
+  }
+}
 template <class A, int N>
 __device__ __forceinline__ void block_store(const A (&v)[N], const Partials& P, const int (&r)[N], int slot = -1) {
   if (slot < 0) slot = blockIdx.x;
@@ -93,18 +77,14 @@ __device__ __forceinline__ void block_store(const A (&v)[N], const Partials& P, 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
 #pragma unroll
   for (int k = 0; k < N; ++k) {
-    A w = v[k];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) w += __shfl_down_sync(0xffffffffu, w, off);
+    const A w = lanes_sum(v[k]);
     if (lane == 0) sm[k][warp] = w;
   }
   __syncthreads();
   if (warp == 0) {
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-      A w = (lane < nw) ? sm[k][lane] : A(0);
-#pragma unroll
-      for (int off = kMaxBlock / 64; off > 0; off >>= 1) w += __shfl_down_sync(0xffffffffu, w, off);
+      const A w = lanes_sum((lane < nw) ? sm[k][lane] : A(0));
       if (lane == 0) {
         double* reg = P.region(r[k]);
         reg[2 * slot] = (double)w;

@@ -22,9 +22,31 @@
 
 namespace {
 
-using tmc::DD;
-using tmc::dd_add;
-using tmc::warp_reduce_dd;
+// ---------------------------------------------------------------------------
+// double-double accumulation (Knuth TwoSum), never contracted into FMA
+// ---------------------------------------------------------------------------
+struct DD {
+  double hi, lo;
+};
+__device__ __forceinline__ DD dd_add(DD a, DD b) {
+  double s = __dadd_rn(a.hi, b.hi);
+  double bb = __dsub_rn(s, a.hi);
+  double e = __dadd_rn(__dsub_rn(a.hi, __dsub_rn(s, bb)), __dsub_rn(b.hi, bb));
+  e = __dadd_rn(e, __dadd_rn(a.lo, b.lo));
+  double hi = __dadd_rn(s, e);
+  double lo = __dsub_rn(e, __dsub_rn(hi, s));
+  return {hi, lo};
+}
+__device__ __forceinline__ DD warp_reduce_dd(DD v) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    DD o;
+    o.hi = __shfl_down_sync(0xffffffffu, v.hi, off);
+    o.lo = __shfl_down_sync(0xffffffffu, v.lo, off);
+    v = dd_add(v, o);
+  }
+  return v;
+}
 
 constexpr int kThreads = 256;
 constexpr int kPerThread = 4;
