@@ -124,6 +124,11 @@ struct tmc_handle {
   // block size per pass of the fused step (cell, vertex, edge_pv, edge_flux,
   // final), chosen by tmc_autotune; the partial-sum counts follow them
   int bsp[5] = {256, 256, 256, 256, 256};
+  int ept[5] = {kEPT, kEPT, kEPT, kEPT, kEPT};  // elements per thread per pass
+  // factors of the inner products and vertex terms of the invariants (FP32,
+  // passes of one element per thread)
+  float *ipc = nullptr, *ipe = nullptr, *vterm = nullptr;
+  Blk blk(int pass) const { return Blk(bsp[pass], ept[pass]); }
   // learned PV-on-edge closure (FP32 path): network, per-member switch, wait status
   const tmc_mlp* closure = nullptr;
   tmc::mlp::Net closure_net{};
@@ -345,6 +350,9 @@ struct Engine : EngineBase {
     s.ke_nx = ke[1 - set];
     s.ud_nx = ud[1 - set];
     s.ratio = ratio;
+    s.ipc = h->ipc;
+    s.ipe = h->ipe;
+    s.vterm = h->vterm;
     s.E = E;
     s.pv_v = pv_v;
     s.vor = vor;
@@ -391,7 +399,20 @@ struct Engine : EngineBase {
   // pass keeps it current.
   void launch_prep() override {
     StageIO<T> s = io(0);
-    launch_edge_prep<T>(h->M, h->O, s, h->P, true, h->bsp[P_FINAL], h->st);
+    launch_edge_prep<T>(h->M, h->O, s, h->P, true, h->blk(P_FINAL), h->st);
+  }
+
+  // beta (step) and the invariants (diag) of the fused program's passes
+  void launch_sums(bool step, bool diag) {
+    const DevMesh& M = h->M;
+    Products X{};
+    if constexpr (std::is_same<T, float>::value) {
+      X = Products{M.nc, M.ne, M.nv, h->ipc, h->ipe, h->vterm, M.areaCell_f, M.areaEdge_f, M.areaTriangle_f,
+                   M.fVertex_f, M.areaCell, gd[0], ghs, gdf[0], ghsf, iap[0],
+                   !step || !launch_cell_is_fast(h->O), !step};
+    }
+    launch_finalize(h->P, h->counts, h->hm.totalArea, h->hm.sumAreaTriangle, h->O.dt, step, diag,
+                    h->p.conserve_energy != 0 && step, h->d_diag, h->st, 2, h->members, X.c ? &X : nullptr);
   }
 
   // one CRK4 step (time_scheme_mod.F90:109-154); state(old) updated in place.
@@ -405,10 +426,9 @@ struct Engine : EngineBase {
     const ModelOpt& O = h->O;
     const double dt = O.dt;
     for (int k = first_stage; k <= 4; ++k) launch_stage(k, diag && k == 1, false, flux_ev, ev_pos);
-    launch_finalize(h->P, h->counts, h->hm.totalArea, h->hm.sumAreaTriangle, dt, true, diag,
-                    h->p.conserve_energy != 0, h->d_diag, h->st, 2, h->members);
+    launch_sums(true, diag);
     if (flux_ev && h->timed_pass == P_FINAL) cudaEventRecord((*flux_ev)[(*ev_pos)++], h->st);
-    launch_final_update<T>(M, O, io(0), h->d_diag, h->P, h->bsp[P_FINAL], h->st);
+    launch_final_update<T>(M, O, io(0), h->d_diag, h->P, h->blk(P_FINAL), h->st);
     if (flux_ev && h->timed_pass == P_FINAL) cudaEventRecord((*flux_ev)[(*ev_pos)++], h->st);
   }
 
@@ -423,7 +443,6 @@ struct Engine : EngineBase {
     s.vor = nullptr;  // vorticity and gd on vertices are kept only by the diagnostic pass
     s.gd_v = nullptr;
     RKStage rk{k, adt[k]};
-    const int* b = h->bsp;
     auto mark = [&](int pass) {
       if (flux_ev && h->timed_pass == pass) cudaEventRecord((*flux_ev)[(*ev_pos)++], h->st);
     };
@@ -435,22 +454,24 @@ struct Engine : EngineBase {
     if (no_tracers) {
       ModelOpt O0 = O;
       O0.n_tracers = 0;
-      launch_cell<T>(M, O0, s, rk, h->P, dg, b[P_CELL], h->st);
+      launch_cell<T>(M, O0, s, rk, h->P, dg, h->blk(P_CELL), h->st);
     } else {
-      launch_cell<T>(M, O, s, rk, h->P, dg, b[P_CELL], h->st);
+      launch_cell<T>(M, O, s, rk, h->P, dg, h->blk(P_CELL), h->st);
     }
     mark(P_CELL);
     mark(P_VERTEX);
-    launch_vertex<T>(M, O, s, h->P, dg, b[P_VERTEX], side);
+    // in FP32 one vertex per thread at every size, but for the invariants' sums
+    const bool one = std::is_same<T, float>::value && h->members == 1 && !dg;
+    launch_vertex<T>(M, O, s, h->P, dg, one ? Blk(h->bsp[P_VERTEX], 1) : h->blk(P_VERTEX), side);
     mark(P_VERTEX);
     mark(P_PV);
-    launch_edge_pv<T>(M, O, s, b[P_PV], side);
+    launch_edge_pv<T>(M, O, s, h->blk(P_PV), side);
     if (branch) h->join_side();
-    if (O.pv_scheme == 2) launch_cons_apvm<T>(M, O, s, h->P, h->d_diag, b[P_VERTEX], h->st);
+    if (O.pv_scheme == 2) launch_cons_apvm<T>(M, O, s, h->P, h->d_diag, h->bsp[P_VERTEX], h->st);
     launch_closure_pass(s, k);
     mark(P_PV);
     mark(P_FLUX);
-    launch_edge_flux<T>(M, O, s, rk, h->P, b[P_FLUX], h->st);
+    launch_edge_flux<T>(M, O, s, rk, h->P, h->blk(P_FLUX), h->st);
     mark(P_FLUX);
   }
 
@@ -471,7 +492,7 @@ struct Engine : EngineBase {
   // stage 1's tracer terms: its F (edge set 0) and next gd (slot 1) stay as
   // the stage left them until stage 2
   void launch_late_tracers() override {
-    launch_tracers_fast<T>(h->M, h->O, io(1), RKStage{1, 0.5 * h->O.dt}, h->bsp[P_CELL], h->st);
+    launch_tracers_fast<T>(h->M, h->O, io(1), RKStage{1, 0.5 * h->O.dt}, h->blk(P_CELL), h->st);
   }
 
   // the learned closure on this stage's pv_edge (FP32 path)
@@ -492,7 +513,7 @@ struct Engine : EngineBase {
     if constexpr (std::is_same<T, float>::value) {
       launch_diag_pass(false);
       StageIO<T> s = io(0);
-      launch_edge_pv<T>(h->M, h->O, s, h->bsp[P_PV], h->st);
+      launch_edge_pv<T>(h->M, h->O, s, h->blk(P_PV), h->st);
       if (h->O.pv_scheme == 2) launch_cons_apvm<T>(h->M, h->O, s, h->P, h->d_diag, h->bsp[P_VERTEX], h->st);
       launch_closure_features(h->M, s, h->cur, feat, pv, h->st);
     }
@@ -647,12 +668,10 @@ struct Engine : EngineBase {
     }
     StageIO<T> s = io(0);
     RKStage rk{0, 0.0};
-    launch_edge_prep<T>(h->M, h->O, s, h->P, true, h->bsp[P_FINAL], h->st);
-    launch_cell<T>(h->M, h->O, s, rk, h->P, true, h->bsp[P_CELL], h->st);
-    launch_vertex<T>(h->M, h->O, s, h->P, true, h->bsp[P_VERTEX], h->st);
-    if (finalize)
-      launch_finalize(h->P, h->counts, h->hm.totalArea, h->hm.sumAreaTriangle, h->O.dt, false, true,
-                      h->p.conserve_energy != 0, h->d_diag, h->st, 2, h->members);
+    launch_edge_prep<T>(h->M, h->O, s, h->P, true, h->blk(P_FINAL), h->st);
+    launch_cell<T>(h->M, h->O, s, rk, h->P, true, h->blk(P_CELL), h->st);
+    launch_vertex<T>(h->M, h->O, s, h->P, true, h->blk(P_VERTEX), h->st);
+    if (finalize) launch_sums(false, true);
   }
 
   // spatial_operators on the state in slot 1 -> gd_tend, iap_tend (uses edge set 0)
@@ -664,12 +683,12 @@ struct Engine : EngineBase {
     s.gdf_in = gdf[1];
     s.qr_in = qr[1];
     RKStage rk{0, 0.0};
-    launch_edge_prep<T>(h->M, h->O, s, h->P, false, h->bs, h->st);
-    launch_cell<T>(h->M, h->O, s, rk, h->P, false, h->bs, h->st);
-    launch_vertex<T>(h->M, h->O, s, h->P, false, h->bs, h->st);
-    launch_edge_pv<T>(h->M, h->O, s, h->bs, h->st);
+    launch_edge_prep<T>(h->M, h->O, s, h->P, false, h->blk(P_FINAL), h->st);
+    launch_cell<T>(h->M, h->O, s, rk, h->P, false, h->blk(P_CELL), h->st);
+    launch_vertex<T>(h->M, h->O, s, h->P, false, h->blk(P_VERTEX), h->st);
+    launch_edge_pv<T>(h->M, h->O, s, h->blk(P_PV), h->st);
     if (h->O.pv_scheme == 2) launch_cons_apvm<T>(h->M, h->O, s, h->P, h->d_diag, h->bs, h->st);
-    launch_edge_flux<T>(h->M, h->O, s, rk, h->P, h->bs, h->st);
+    launch_edge_flux<T>(h->M, h->O, s, rk, h->P, h->blk(P_FLUX), h->st);
   }
 
   void state_slot0(void** g, void** i, void** qq, void** gh) override {
@@ -1054,15 +1073,54 @@ int build_graph(tmc_handle* h, bool diag, cudaGraphExec_t* out, int first_stage 
 
 // partial counts per region: the grid of the passes that write it
 void set_counts(tmc_handle* h) {
-  const int bc = grid_for(h->M.nc, h->bsp[P_CELL]), bf = grid_for(h->M.ne, h->bsp[P_FLUX]),
-            bfin = grid_for(h->M.ne, h->bsp[P_FINAL]), bv = grid_for(h->M.nv, h->bsp[P_VERTEX]);
-  static const int cells[6] = {R_IP_C, R_IP_C + 2, R_IP_C + 4, R_44_C, R_MASS, R_EN_C};
+  const int bc = grid_for(h->M.nc, h->blk(P_CELL)), bf = grid_for(h->M.ne, h->blk(P_FLUX)),
+            bfin = grid_for(h->M.ne, h->blk(P_FINAL)), bv = grid_for(h->M.nv, h->blk(P_VERTEX));
+  static const int cells[4] = {R_IP_C, R_IP_C + 2, R_IP_C + 4, R_44_C};
   static const int edges[4] = {R_IP_E, R_IP_E + 2, R_IP_E + 4, R_44_E};
   static const int verts[5] = {R_PE, R_AV, R_C1, R_C2, R_C3};
-  for (int r : cells) h->counts[r] = bc;
-  for (int r : edges) h->counts[r] = bf;
-  h->counts[R_EN_E] = bfin;
-  for (int r : verts) h->counts[r] = bv;
+  // the sums of k_finalize_products come in blocks of 256 x kEPT elements
+  const int bci = h->ipc ? grid_for(h->M.nc, 256) : bc, bfi = h->ipe ? grid_for(h->M.ne, 256) : bf;
+  for (int r : cells) h->counts[r] = bci;
+  h->counts[R_MASS] = h->counts[R_EN_C] = bci;
+  for (int r : edges) h->counts[r] = bfi;
+  h->counts[R_EN_E] = h->ipe ? bfi : bfin;
+  for (int r : verts) h->counts[r] = h->vterm ? grid_for(h->M.nv, 256) : bv;
+}
+
+// Elements per thread (1 or kEPT) and default block size of each pass of the
+// fused single-model step, by element count.  Four elements per thread leave
+// SMs without a block on a small mesh (level 6: 120 blocks of 256 edges x 4
+// on 152 SMs) and run a thread's elements one after another; one element per
+// thread costs a large mesh the loads in flight and the warps' start-up.
+// Measured per step, four -> one: level 5 FP64 227 -> 89 us, FP32 74 -> 47;
+// level 6 FP64 with upwind pv 475 -> 300, FP32 103 -> 84.  The lines, us per
+// pass, four / one:
+//   FP64 flux      491k edges 115.6 / 96.2, 1.97M 342.9 / 344.7 (final, upwind pv alike)
+//   FP64 cell      655k cells, four tracers 182.5 / 139.4
+//   FP64 vertex    328k 28.9 / 25.4, 1.31M 71.0 / 73.6
+//   FP32 flux      123k edges 10.5 / 8.8, 491k 18.8 / 21.5 (final alike)
+//   centred pv     123k equal, 491k 6.9 / 10.0 in FP32, 8.8 / 9.6 in FP64
+//   FP32 cell      164k 15.8 / 13.2, 655k 31.2 / 29.8, 2.6M 132.9 / 140.9 (655k stays at four:
+//                  its inner products would come as 10 MB of factors)
+//   FP32 vertex    one is the faster at every size (1.31M 25.0 / 22.9, 5.2M 68.9 / 67.5; launch_stage)
+// One element per thread takes blocks of 128 threads, and of 64 in FP64 while
+// those number under 16 per SM (level 6, upwind pv: 300 us against 312 with
+// 128 and 343 with 256).
+void choose_launch_shapes(tmc_handle* h, bool default_blocks) {
+  const bool f64 = h->p.precision == TMC_FP64;
+  const int nc = h->M.nc, ne = h->M.ne, nv = h->M.nv;
+  const int big = 1000000, small = 300000;
+  const int n[P_COUNT] = {nc, nv, ne, ne, ne};
+  int line[P_COUNT];
+  line[P_CELL] = f64 ? big : small;
+  line[P_VERTEX] = f64 ? big : small;
+  line[P_PV] = f64 && h->O.pv_scheme == 3 ? big : small;
+  line[P_FLUX] = line[P_FINAL] = f64 ? big : small;
+  for (int k = 0; k < P_COUNT; ++k) {
+    if (n[k] >= line[k]) continue;
+    h->ept[k] = 1;
+    if (default_blocks) h->bsp[k] = f64 && n[k] < 64 * 16 * h->sms ? 64 : 128;
+  }
 }
 
 void ensure_prep(tmc_handle* h) {
@@ -1233,6 +1291,8 @@ int tmc_create(const tmc_mesh_desc* mesh, const tmc_params* params, tmc_handle**
   const int tro = p.tracer_adv_order ? p.tracer_adv_order : p.adv_order;
   if (tro < 2 || tro > 6) return bad("tracer_adv_order must be 2..6");
   if (p.precision != TMC_FP64 && p.precision != TMC_FP32) return bad("precision must be TMC_FP64 or TMC_FP32");
+  cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, p.device);
+  cudaGetLastError();
   h->bs = p.block_size > 0 ? p.block_size : 256;
   if (h->bs % 32 != 0 || h->bs > 512) return bad("block_size must be a multiple of 32 up to 512");
   if (p.members > 1 && h->bs > 256) return bad("block_size must be at most 256 for ensembles");
@@ -1400,6 +1460,19 @@ int tmc_create(const tmc_mesh_desc* mesh, const tmc_params* params, tmc_handle**
   // the FP32 cell pass is compiled for at most 256 threads per block (its
   // register budget leaves room for 3 blocks per SM)
   if (p.precision == TMC_FP32) h->bsp[P_CELL] = std::min(h->bsp[P_CELL], 256);
+  if (!h->generic && h->members == 1) choose_launch_shapes(h.get(), p.block_size == 0);
+  if (p.precision == TMC_FP32 && h->members == 1) {
+    if (h->ept[P_CELL] == 1) h->ipc = h->dalloc<float>((size_t)4 * hm.nc);
+    if (h->ept[P_FLUX] == 1) h->ipe = h->dalloc<float>((size_t)4 * hm.ne);
+    if (h->ept[P_VERTEX] == 1) h->vterm = h->dalloc<float>((size_t)2 * hm.nv);
+    if ((h->ept[P_CELL] == 1 && !h->ipc) || (h->ept[P_FLUX] == 1 && !h->ipe) ||
+        (h->ept[P_VERTEX] == 1 && !h->vterm)) {
+      h->err = "device allocation failed";
+      cudaGetLastError();
+      *out = h.release();
+      return TMC_E_CUDA;
+    }
+  }
   set_counts(h.get());
   const int bc = grid_for(hm.nc, h->bs);
   for (int r = 0; r < R_COUNT; ++r) h->gen_counts[r] = h->counts[r];
@@ -1414,7 +1487,6 @@ int tmc_create(const tmc_mesh_desc* mesh, const tmc_params* params, tmc_handle**
     return TMC_E_CUDA;
   }
   cudaMemset(h->d_diag, 0, sizeof(double) * kDiagStride * h->members);
-  cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, p.device);
   h->d_member_on = h->dalloc<int>(h->members);
   h->d_closure_err = h->dalloc<int>(1);
   if (!h->d_member_on || !h->d_closure_err) {

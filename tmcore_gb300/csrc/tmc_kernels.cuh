@@ -33,7 +33,7 @@
 
 namespace tmc {
 
-constexpr int kEPT = 4;  // elements per thread
+constexpr int kEPT = 4;  // elements per thread (one on small meshes, see Blk)
 constexpr int kUpW32 = 16;  // widest vertex fit stencil of the packed FP32 upwind pv kernel
 
 struct DStencil {
@@ -193,6 +193,10 @@ struct StageIO {
   double *sq, *hu, *ke, *ud;
   double *sq_nx, *hu_nx, *ke_nx, *ud_nx;
   double* ratio;
+  // FP32 path, one element per thread: factors of the CRK4 inner products
+  // [4][nc] and [4][ne] (t1 t2, t2 t3, t3 t4, t_new t_new), and [2][nv] the
+  // vertex terms of potential enstrophy and vorticity; see Products
+  float *ipc, *ipe, *vterm;
   // the next stage's gd_e, u, F, Fq, written by k_edge_flux (stages 1-3) and
   // k_final_edges (next step): the edge preparation of the next stage fused
   // into the pass that produces its iap_u (null: not fused)
@@ -272,40 +276,65 @@ inline unsigned nmem(const StageIO<T>& S) {
   return S.members > 1 ? (unsigned)S.members : 1u;
 }
 
+// Launch shape of a pass: threads per block and elements per thread, 1 or
+// kEPT.  One on a mesh too small to fill the GPU otherwise (elements_per_thread).
+struct Blk {
+  int bs, ept;
+  Blk(int b, int e = kEPT) : bs(b), ept(e) {}
+};
+
 // ---- launchers (instantiated in tmc_kernels_f64.cu / _f32.cu) ----
 template <class T>
-void launch_edge_prep(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Partials P, bool diag, int bs,
+void launch_edge_prep(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Partials P, bool diag, Blk b,
                       cudaStream_t st);
 template <class T>
 void launch_cell(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Partials P, bool diag,
-                 int bs, cudaStream_t st);
+                 Blk b, cudaStream_t st);
+// whether launch_cell takes the FP32 fast pass in a CRK4 stage
+inline bool launch_cell_is_fast(const ModelOpt& O) {
+  const int n = O.n_tracers;
+  return n == 0 || (O.tr_order == 2 && (n == 1 || n == 2 || n == 4));
+}
 // FP32, single member, 1, 2 or 4 second-order tracers: the tracer terms of
 // the cell pass of stage rk, after a tracer-free cell pass of that stage
 // (launch_cell with n_tracers 0); a no-op otherwise
 template <class T>
-void launch_tracers_fast(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, int bs,
+void launch_tracers_fast(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Blk b,
                          cudaStream_t st);
 template <class T>
-void launch_vertex(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Partials P, bool diag, int bs,
+void launch_vertex(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Partials P, bool diag, Blk b,
                    cudaStream_t st);
 template <class T>
-void launch_edge_pv(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, int bs, cudaStream_t st);
+void launch_edge_pv(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Blk b, cudaStream_t st);
 template <class T>
-void launch_edge_flux(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Partials P, int bs,
+void launch_edge_flux(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Partials P, Blk b,
                       cudaStream_t st);
 // final update (beta-scaled) of cells, then of edges together with the edge
 // preparation of the next step's first stage and its energy partials
 template <class T>
 void launch_final_update(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, const double* diag, Partials P,
-                         int bs, cudaStream_t st);
+                         Blk b, cudaStream_t st);
 // number of blocks a launcher uses for n elements
-__host__ __device__ inline int grid_for(int n, int bs) { return (n + bs * kEPT - 1) / (bs * kEPT); }
+__host__ __device__ inline int grid_for(int n, int bs, int ept = kEPT) { return (n + bs * ept - 1) / (bs * ept); }
+inline int grid_for(int n, const Blk& b) { return grid_for(n, b.bs, b.ept); }
 
 // reduction of partial regions into diag[]; counts per region.  scheme: the
 // beta formula (1 CRK3, 2 CRK4, 3 PC2; time_scheme_mod.F90:94-100,144-150,174-180)
+// What k_finalize_products sums after FP32 passes of one element per thread:
+// the stored factors of the inner products with the areas that weigh them, and
+// the invariants of state(old) from its arrays.  A null c, e or v: that kind's
+// passes stored block sums.
+struct Products {
+  int nc, ne, nv;
+  const float *c, *e, *v;  // [4][nc], [4][ne], [2][nv]
+  const float *areaCell_f, *areaEdge_f, *areaTriangle_f, *fVertex_f;
+  const double *areaCell, *gd, *ghs;
+  const float *gdf, *ghsf, *iap;
+  bool enc64, ene64;  // the cells' (edges') energy terms in FP64 (k_cell, k_edge_prep), else FP32, compensated
+};
 void launch_finalize(Partials P, const int* counts_host, double totalArea, double sumAreaTriangle, double dt,
                      bool step, bool diag, bool conserve, double* diag_out, cudaStream_t st, int scheme = 2,
-                     int members = 1);
+                     int members = 1, const Products* products = nullptr);
 
 // conservative APVM (pv_scheme 2) after k_edge_pv: both tangent fluxes, their
 // curls and the three global sums, epsilon, and the correction of pv_edge

@@ -2,6 +2,8 @@
 // element follows the reference's IEEE operation order), the reduction
 // finaliser, the FP32 shadow helpers and the single-operator kernels used for
 // parity.
+#include <algorithm>
+
 #include "tmc_kernels_impl.cuh"
 
 namespace tmc {
@@ -40,6 +42,48 @@ __device__ f64::HiLo region_sum_pair(const double* reg, int count) {
 __device__ double region_sum_dd(const double* reg, int count) {
   const f64::HiLo w = region_sum_pair(reg, count);
   return w.hi + w.lo;
+}
+
+// beta and the invariants from the region sums rv, by warp 0
+__device__ __forceinline__ void finish_step(const FinalizeArgs& a, const double* rv, double* out) {
+  if (threadIdx.x >= 32) return;
+  const int lane = threadIdx.x;
+  // lane k: R[k] = <t_k, t_k+1> (k < 3), R[3] = <t_new, t_new>
+  double Rk = 0.0;
+  if (a.step) {
+    const int re = lane < 3 ? R_IP_E + 2 * lane : R_44_E, rc = lane < 3 ? R_IP_C + 2 * lane : R_44_C;
+    Rk = (rv[re] + rv[rc]) / a.totalArea;
+  }
+  double R[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) R[k] = __shfl_sync(0xffffffffu, Rk, k);
+  if (threadIdx.x != 0) return;
+  if (a.step) {
+    double beta = 1.0;
+    if (a.conserve) {
+      if (a.scheme == 1)  // CRK3: R[0] = <t1,t2>, R[1] = <t1,t3>, R[2] = <t2,t3>
+        beta = R[3] != 0.0 ? (2.0 * R[0] - R[1] + 2.0 * R[2]) / (3.0 * R[3]) : 1.0;
+      else if (a.scheme == 3)  // PC2: R[0] = <t_old,t_new>, R[3] = <t_new,t_new>
+        beta = (R[0] != 0.0 && R[3] != 0.0) ? R[0] / R[3] : 1.0;
+      else  // CRK4
+        beta = R[3] != 0.0 ? (R[0] + R[1] + R[2]) / (3.0 * R[3]) : 1.0;
+      // time_scheme_mod.F90:145 (CRK4) and :94-100 (CRK3) divide 0 / 0 when the
+      // tendency is zero everywhere (a state at rest); beta = 1 there, as the
+      // reference's PC2 has it (:178)
+    }
+    out[4] = beta;
+    out[5] = R[0];
+    out[6] = R[1];
+    out[7] = R[2];
+    out[8] = R[3];
+    out[9] = beta * a.dt;
+  }
+  if (a.diag) {
+    out[0] = rv[R_MASS];
+    out[1] = rv[R_EN_E] + rv[R_EN_C];
+    out[2] = rv[R_PE];
+    out[3] = rv[R_AV] / a.sumAreaTriangle;
+  }
 }
 
 // a.split blocks per partial region (kFinSplit for one model, fewer for a
@@ -88,50 +132,132 @@ __global__ void __launch_bounds__(256) k_finalize(Partials P0, FinalizeArgs a, d
     if (lane == 0) rs[q] = res[q] = s;
   }
   __syncthreads();
-  if (threadIdx.x >= 32) return;
-  const double* rv = rs;
-  // lane k: R[k] = <t_k, t_k+1> (k < 3), R[3] = <t_new, t_new>
-  double Rk = 0.0;
-  if (a.step) {
-    const int re = lane < 3 ? R_IP_E + 2 * lane : R_44_E, rc = lane < 3 ? R_IP_C + 2 * lane : R_44_C;
-    Rk = (rv[re] + rv[rc]) / a.totalArea;
-  }
-  double R[4];
+  finish_step(a, rs, out);
+  if (threadIdx.x == 0) *counter = 0u;
+}
+
+// The same after passes of one element per thread, for small FP32 models: the
+// blocks first form the block sums those passes did not store, 256 threads of
+// four elements with the fused multiply-adds, shuffle tree and block tree of
+// the passes of kEPT elements per thread, so beta and the invariants do not
+// depend on the passes' launch shapes; the last block to finish combines all
+// regions, a warp each.
+__device__ __forceinline__ void sum_products(const Partials& P, const float* f, const float* area, int n, int slot,
+                                             const int (&r)[4]) {
+  const int i0 = slot * (kEPT * 256) + threadIdx.x;
+  float w[kEPT], x[4][kEPT], v[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-  for (int k = 0; k < 4; ++k) R[k] = __shfl_sync(0xffffffffu, Rk, k);
-  if (threadIdx.x != 0) return;
-  if (a.step) {
-    double beta = 1.0;
-    if (a.conserve) {
-      if (a.scheme == 1)  // CRK3: R[0] = <t1,t2>, R[1] = <t1,t3>, R[2] = <t2,t3>
-        beta = R[3] != 0.0 ? (2.0 * R[0] - R[1] + 2.0 * R[2]) / (3.0 * R[3]) : 1.0;
-      else if (a.scheme == 3)  // PC2: R[0] = <t_old,t_new>, R[3] = <t_new,t_new>
-        beta = (R[0] != 0.0 && R[3] != 0.0) ? R[0] / R[3] : 1.0;
-      else  // CRK4
-        beta = R[3] != 0.0 ? (R[0] + R[1] + R[2]) / (3.0 * R[3]) : 1.0;
-      // time_scheme_mod.F90:145 (CRK4) and :94-100 (CRK3) divide 0 / 0 when the
-      // tendency is zero everywhere (a state at rest); beta = 1 there, as the
-      // reference's PC2 has it (:178)
+  for (int j = 0; j < kEPT; ++j) {
+    const int i = i0 + j * 256;
+    w[j] = i < n ? area[i] : 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x[k][j] = i < n ? f[(size_t)k * n + i] : 0.f;
+  }
+#pragma unroll
+  for (int j = 0; j < kEPT; ++j)
+    if (i0 + j * 256 < n)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = __fmaf_rn(x[k][j], w[j], v[k]);
+  block_store<float, 4>(v, P, r, slot);
+}
+__global__ void __launch_bounds__(256) k_finalize_products(Partials P, FinalizeArgs a, Products X, int nbc, int nbe,
+                                                           int nbv, double* out, double* res, unsigned int* counter) {
+  const int b = blockIdx.x;
+  if (b < nbc) {
+    if (a.step) {
+      const int r[4] = {R_IP_C, R_IP_C + 2, R_IP_C + 4, R_44_C};
+      sum_products(P, X.c, X.areaCell_f, X.nc, b, r);
     }
-    out[4] = beta;
-    out[5] = R[0];
-    out[6] = R[1];
-    out[7] = R[2];
-    out[8] = R[3];
-    out[9] = beta * a.dt;
+    if (a.diag) {
+      double mass = 0.0, enc = 0.0;
+      float eh = 0.f, el = 0.f;
+      for (int j = 0; j < kEPT; ++j) {
+        const int i = b * (kEPT * 256) + j * 256 + threadIdx.x;
+        if (i >= X.nc) break;
+        const double g = X.gd[i], A = X.areaCell[i];
+        mass = __fma_rn(g, A, mass);
+        if (X.enc64) {
+          enc = __fma_rn(g * __fma_rn(2.0, X.ghs[i], g), A, enc);
+        } else {
+          const float gf = X.gdf[i];
+          two_sum_acc(eh, el, gf * (gf + 2.f * X.ghsf[i]) * X.areaCell_f[i]);
+        }
+      }
+      const double v[2] = {mass, X.enc64 ? enc : (double)eh + (double)el};
+      const int r[2] = {R_MASS, R_EN_C};
+      block_store<double, 2>(v, P, r, b);
+    }
+  } else if (b < nbc + nbe) {
+    const int slot = b - nbc;
+    if (a.step) {
+      const int r[4] = {R_IP_E, R_IP_E + 2, R_IP_E + 4, R_44_E};
+      sum_products(P, X.e, X.areaEdge_f, X.ne, slot, r);
+    }
+    if (a.diag) {
+      double en = 0.0;
+      float eh = 0.f, el = 0.f;
+      for (int j = 0; j < kEPT; ++j) {
+        const int i = slot * (kEPT * 256) + j * 256 + threadIdx.x;
+        if (i >= X.ne) break;
+        const float t = X.iap[i] * X.iap[i] * X.areaEdge_f[i];
+        if (X.ene64)
+          en += (double)t;
+        else
+          two_sum_acc(eh, el, t);
+      }
+      const int r[1] = {R_EN_E};
+      if (X.ene64) {
+        const double v[1] = {en};
+        block_store<double, 1>(v, P, r, slot);
+      } else {
+        const float h[1] = {eh}, l[1] = {el};
+        block_store_ff<1>(h, l, P, r, slot);
+      }
+    }
+  } else if (b < nbc + nbe + nbv) {
+    const int slot = b - nbc - nbe;
+    float ph = 0.f, pl = 0.f, ah = 0.f, al = 0.f;
+    for (int j = 0; j < kEPT; ++j) {
+      const int i = slot * (kEPT * 256) + j * 256 + threadIdx.x;
+      if (i >= X.nv) break;
+      two_sum_acc(ph, pl, X.v[i]);
+      two_sum_acc(ah, al, X.v[(size_t)X.nv + i]);
+      two_sum_acc(ah, al, X.fVertex_f[i] * X.areaTriangle_f[i]);
+    }
+    const float h[2] = {ph, ah}, l[2] = {pl, al};
+    const int r[2] = {R_PE, R_AV};
+    block_store_ff<2>(h, l, P, r, slot);
   }
-  if (a.diag) {
-    out[0] = rv[R_MASS];
-    out[1] = rv[R_EN_E] + rv[R_EN_C];
-    out[2] = rv[R_PE];
-    out[3] = rv[R_AV] / a.sumAreaTriangle;
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = (atomicAdd(counter, 1u) == gridDim.x - 1);
   }
-  *counter = 0u;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  __shared__ double rs[kFinalizeRegions];
+  const int lane = threadIdx.x & 31;
+  for (int q = threadIdx.x >> 5; q < kFinalizeRegions; q += blockDim.x >> 5) {
+    const bool on = (q <= R_44_E) ? a.step : a.diag;
+    double hi = 0.0, lo = 0.0;
+    for (int i = lane; on && i < a.counts[q]; i += 32) {
+      const double2 p = __ldcg(reinterpret_cast<const double2*>(P.region(q)) + i);
+      hi = __dadd_rn(hi, p.x);
+      lo = __dadd_rn(lo, p.y);
+    }
+    const f64::HiLo h = f64::split(f64::warp_sum(hi));
+    const double s = h.hi + (h.lo + f64::value(f64::warp_sum(lo)));
+    if (lane == 0) rs[q] = res[q] = s;
+  }
+  __syncthreads();
+  finish_step(a, rs, out);
+  if (threadIdx.x == 0) *counter = 0u;
 }
 
 void launch_finalize(Partials P, const int* counts_host, double totalArea, double sumAreaTriangle, double dt,
                      bool step, bool diag, bool conserve, double* diag_out, cudaStream_t st, int scheme,
-                     int members) {
+                     int members, const Products* products) {
   FinalizeArgs a;
   for (int r = 0; r < R_COUNT; ++r) a.counts[r] = counts_host[r];
   a.totalArea = totalArea;
@@ -152,6 +278,13 @@ void launch_finalize(Partials P, const int* counts_host, double totalArea, doubl
   // scratch after the kDiagLen outputs: R_COUNT region sums, then the counter
   double* res = diag_out + kDiagLen;
   unsigned int* counter = reinterpret_cast<unsigned int*>(diag_out + kDiagLen + R_COUNT);
+  if (products) {
+    const int nbc = products->c ? grid_for(products->nc, 256) : 0, nbe = products->e ? grid_for(products->ne, 256) : 0;
+    const int nbv = products->v && diag ? grid_for(products->nv, 256) : 0;
+    k_finalize_products<<<std::max(nbc + nbe + nbv, 1), 256, 0, st>>>(P, a, *products, nbc, nbe, nbv, diag_out, res,
+                                                                      counter);
+    return;
+  }
   k_finalize<<<dim3(kFinalizeRegions * a.split, members > 1 ? members : 1), 256, 0, st>>>(P, a, diag_out, res,
                                                                                          counter);
 }

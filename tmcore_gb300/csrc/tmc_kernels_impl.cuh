@@ -98,6 +98,13 @@ __device__ __forceinline__ void block_store(const A (&v)[N], const Partials& P, 
 template <class T>
 constexpr bool kF64 = std::is_same<T, double>::value;
 
+// The FP32 passes of one element per thread store the factors of the CRK4
+// inner products and the vertex terms of the invariants, and no block sums:
+// k_finalize_products sums them, and the other invariants from the state, in
+// the order of the passes of kEPT elements per thread.
+template <class T, int EPT>
+constexpr bool kProducts = !kF64<T> && EPT == 1;
+
 // metric in the arithmetic type: FP64 array in FP64 mode, FP32 copy otherwise
 template <class T>
 __device__ __forceinline__ T met(const double* d, const float* f, size_t i) {
@@ -136,8 +143,8 @@ __device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float p) {
 // busy time.  Every thread of the block must call this (it synchronises).
 template <int N>
 __device__ __forceinline__ void block_store_ff(const float (&hi)[N], const float (&lo)[N], const Partials& P,
-                                               const int (&r)[N]) {
-  const int slot = blockIdx.x;
+                                               const int (&r)[N], int slot = -1) {
+  if (slot < 0) slot = blockIdx.x;
   __shared__ float sh[N][kMaxBlock / 32], sl[N][kMaxBlock / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
 #pragma unroll
@@ -175,11 +182,12 @@ __device__ __forceinline__ void block_store_ff(const float (&hi)[N], const float
   __syncthreads();
 }
 
-// block-strided loop: thread handles i = base + k*blockDim.x, k < kEPT
-#define TMC_FOR_EPT(i, n)                                                              \
-  for (int _k = 0, i = blockIdx.x * (kEPT * blockDim.x) + threadIdx.x; _k < kEPT; \
-       ++_k, i += blockDim.x)                                                          \
+// block-strided loop: thread handles i = base + k*blockDim.x, k < EPT
+#define TMC_FOR_N(EPT, i, n)                                                          \
+  for (int _k = 0, i = blockIdx.x * (EPT * blockDim.x) + threadIdx.x; _k < EPT; \
+       ++_k, i += blockDim.x)                                                         \
     if (i < (n))
+#define TMC_FOR_EPT(i, n) TMC_FOR_N(kEPT, i, n)
 
 // x / 12
 __device__ __forceinline__ float over12(float x) { return x / 12.f; }
@@ -371,13 +379,13 @@ __device__ __forceinline__ T energy_term(const DevMesh& M, int e, T ia) {
 
 // Stand-alone edge preparation of a state slot (the first stage after the
 // state was set, the diagnostic pass, spatial_operators).
-template <class T, bool kB>
+template <class T, bool kB, int EPT>
 __global__ void __launch_bounds__(kMaxBlock) k_edge_prep(DevMesh M, ModelOpt O, StageIO<T> S0, Partials P0, int diag) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
   double en = 0.0;
   const CellSrc<T> C{S.gd_in, S.gdf_in, S.q_in, S.qr_in, nullptr};
-  TMC_FOR_EPT(e, M.ne) {
+  TMC_FOR_N(EPT, e, M.ne) {
     const int c1 = M.cellsOnEdge[e], c2 = M.cellsOnEdge[M.ne + e];
     const T ia = S.iap_in[e];
     T g1, g2;
@@ -389,14 +397,14 @@ __global__ void __launch_bounds__(kMaxBlock) k_edge_prep(DevMesh M, ModelOpt O, 
       g2 = S.gdf_in[c2];
     }
     prep_edge<T>(M, O, e, c1, c2, ia, g1, g2, C, edge_set(S));
-    if (diag) {
+    if (!kProducts<T, EPT> && diag) {
       if constexpr (kF64<T>)
         en = en + energy_term<T>(M, e, ia);
       else
         en += (double)energy_term<T>(M, e, ia);
     }
   }
-  if (diag) {
+  if (!kProducts<T, EPT> && diag) {
     const double v[1] = {en};
     const int r[1] = {R_EN_E};
     block_store<double, 1>(v, P, r);
@@ -406,14 +414,14 @@ __global__ void __launch_bounds__(kMaxBlock) k_edge_prep(DevMesh M, ModelOpt O, 
 // ---------------------------------------------------------------------------
 // cell: div of mass flux, kinetic energy, E, RK update of gd and tracers
 // ---------------------------------------------------------------------------
-template <class T, bool kB>
+template <class T, bool kB, int EPT>
 __global__ void __launch_bounds__(kMaxBlock) k_cell(DevMesh M, ModelOpt O, StageIO<T> S0, RKStage rk, Partials P0,
                                                     int diag) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
   T rip = T(0), r44 = T(0);
   double mass = 0.0, enc = 0.0;
-  TMC_FOR_EPT(c, M.nc) {
+  TMC_FOR_N(EPT, c, M.nc) {
     double t;  // gd tendency, FP64 in both modes
     double rA = 0.0;  // FP64: 1 / areaCell
     T tT, ke;
@@ -528,7 +536,10 @@ __global__ void __launch_bounds__(kMaxBlock) k_cell(DevMesh M, ModelOpt O, Stage
           break;
         case 2:
         case 3: {
-          rip += tprev * tT * Af;
+          if constexpr (kProducts<T, EPT>)
+            S.ipc[(size_t)(mode - 2) * M.nc + c] = tprev * tT;
+          else
+            rip += tprev * tT * Af;
           S.gd_acc[c] = gacc + 2.0 * t;
           tb[c] = tT;
           gnext = gold + rk.a_dt * t;
@@ -537,11 +548,16 @@ __global__ void __launch_bounds__(kMaxBlock) k_cell(DevMesh M, ModelOpt O, Stage
           break;
         }
         case 4: {
-          rip += tprev * tT * Af;
           const double tn = (gacc + t) * (1.0 / 6.0);
           S.gd_acc[c] = tn;
           const float tnf = (float)tn;
-          r44 += tnf * tnf * Af;
+          if constexpr (kProducts<T, EPT>) {
+            S.ipc[(size_t)2 * M.nc + c] = tprev * tT;
+            S.ipc[(size_t)3 * M.nc + c] = tnf * tnf;
+          } else {
+            rip += tprev * tT * Af;
+            r44 += tnf * tnf * Af;
+          }
           tb[c] = tT;
           break;
         }
@@ -630,17 +646,17 @@ __global__ void __launch_bounds__(kMaxBlock) k_cell(DevMesh M, ModelOpt O, Stage
         }
       }
     }
-    if (diag) {
+    if (!kProducts<T, EPT> && diag) {
       mass = __fma_rn(gdin, Ad, mass);
       enc = __fma_rn(gdin * __fma_rn(2.0, ghsd, gdin), Ad, enc);
     }
   }
-  if (rk.mode >= 2) {
+  if (!kProducts<T, EPT> && rk.mode >= 2) {
     const T v[2] = {rip, r44};
     const int r[2] = {R_IP_C + 2 * (rk.mode - 2), R_44_C};
     block_store<T, 2>(v, P, r);
   }
-  if (diag) {
+  if (!kProducts<T, EPT> && diag) {
     const double v[2] = {mass, enc};
     const int r[2] = {R_MASS, R_EN_C};
     block_store<double, 2>(v, P, r);
@@ -650,14 +666,14 @@ __global__ void __launch_bounds__(kMaxBlock) k_cell(DevMesh M, ModelOpt O, Stage
 // ---------------------------------------------------------------------------
 // vertex: gd on vertices, vorticity, potential vorticity
 // ---------------------------------------------------------------------------
-template <class T, bool kB>
+template <class T, bool kB, int EPT>
 __global__ void __launch_bounds__(kMaxBlock) k_vertex(DevMesh M, ModelOpt O, StageIO<T> S0, Partials P0, int diag) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
   double pe = 0.0, av = 0.0;      // FP64 path
   float ph = 0.f, pl = 0.f, ah = 0.f, al = 0.f;  // FP32 path: compensated sums
   if constexpr (kF64<T>) {
-    TMC_FOR_EPT(v, M.nv) {
+    TMC_FOR_N(EPT, v, M.nv) {
       // operators_mod.F90:106-123 (c2v), :76-91 (curl), :262-270 (pv)
       double s = 0.0, gv = 0.0;
 #pragma unroll
@@ -685,7 +701,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_vertex(DevMesh M, ModelOpt O, Sta
     // Every load is a read-only (non-coherent) load: nothing this kernel
     // stores aliases them, which lets the compiler issue a vertex's loads
     // ahead of the previous vertex's stores.
-    TMC_FOR_EPT(v, M.nv) {
+    TMC_FOR_N(EPT, v, M.nv) {
       int ci[3], ei[3];
       float kt[3], ts[3];
 #pragma unroll
@@ -716,14 +732,19 @@ __global__ void __launch_bounds__(kMaxBlock) k_vertex(DevMesh M, ModelOpt O, Sta
         // potential enstrophy and absolute vorticity (tmcore_swm_mod.F90:233-255)
         // from FP32 terms with compensated sums: FP64 terms made this launch
         // FP64-pipe bound
-        two_sum_acc(ph, pl, gv * (pv * pv) * At);
-        two_sum_acc(ah, al, vo * At);
-        two_sum_acc(ah, al, fv * At);
+        if constexpr (kProducts<T, EPT>) {
+          S.vterm[v] = gv * (pv * pv) * At;
+          S.vterm[(size_t)M.nv + v] = vo * At;
+        } else {
+          two_sum_acc(ph, pl, gv * (pv * pv) * At);
+          two_sum_acc(ah, al, vo * At);
+          two_sum_acc(ah, al, fv * At);
+        }
       }
     }
   }
   (void)O;
-  if (diag) {
+  if (!kProducts<T, EPT> && diag) {
     const int r[2] = {R_PE, R_AV};
     if constexpr (kF64<T>) {
       const double vv[2] = {pe, av};
@@ -736,11 +757,11 @@ __global__ void __launch_bounds__(kMaxBlock) k_vertex(DevMesh M, ModelOpt O, Sta
 }
 
 // pv on cells: scalar_v2c_interp_operator as a gather (operators_mod.F90:125-141)
-template <class T>
+template <class T, int EPT>
 __global__ void __launch_bounds__(kMaxBlock) k_v2c(DevMesh M, const T* pv_v0, T* pv_c0, long long msv, long long msc) {
   const T* pv_v = pv_v0 + blockIdx.y * msv;
   T* pv_c = pv_c0 + blockIdx.y * msc;
-  TMC_FOR_EPT(c, M.nc) {
+  TMC_FOR_N(EPT, c, M.nc) {
     const T A = T(M.areaCell[c]);
     T s = T(0);
     for (int k = M.v2c_start[c]; k < M.v2c_start[c + 1]; ++k) s = s + pv_v[M.v2c_vertex[k]] * T(M.v2c_kite[k]) / A;
@@ -751,31 +772,31 @@ __global__ void __launch_bounds__(kMaxBlock) k_v2c(DevMesh M, const T* pv_v0, T*
 // ---------------------------------------------------------------------------
 // edge_pv: PV on edges (calc_pv_on_edge, operators_mod.F90:273-412)
 // ---------------------------------------------------------------------------
-template <class T, bool kB>
+template <class T, bool kB, int EPT>
 __global__ void __launch_bounds__(kMaxBlock) k_edge_pv(DevMesh M, ModelOpt O, StageIO<T> S0) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const bool need_v = (O.pv_scheme >= 2) || (O.pv_scheme == 1 && O.apvm_weight != 0.0);
   if (!need_v) {
-    // centred pv (APVM weight 0): all loads of the thread's kEPT edges first
-    const int e0 = blockIdx.x * (kEPT * blockDim.x) + threadIdx.x;
-    int v1[kEPT], v2[kEPT];
-    T pe[kEPT];
+    // centred pv (APVM weight 0): all loads of the thread's EPT edges first
+    const int e0 = blockIdx.x * (EPT * blockDim.x) + threadIdx.x;
+    int v1[EPT], v2[EPT];
+    T pe[EPT];
 #pragma unroll
-    for (int j = 0; j < kEPT; ++j) {
+    for (int j = 0; j < EPT; ++j) {
       const int e = e0 + j * blockDim.x;
       v1[j] = e < M.ne ? M.verticesOnEdge[e] : 0;
       v2[j] = e < M.ne ? M.verticesOnEdge[M.ne + e] : 0;
     }
 #pragma unroll
-    for (int j = 0; j < kEPT; ++j) pe[j] = halve(S.pv_v[v1[j]] + S.pv_v[v2[j]]);
+    for (int j = 0; j < EPT; ++j) pe[j] = halve(S.pv_v[v1[j]] + S.pv_v[v2[j]]);
 #pragma unroll
-    for (int j = 0; j < kEPT; ++j) {
+    for (int j = 0; j < EPT; ++j) {
       const int e = e0 + j * blockDim.x;
       if (e < M.ne) S.pv_e[e] = pe[j];
     }
     return;
   }
-  TMC_FOR_EPT(e, M.ne) {
+  TMC_FOR_N(EPT, e, M.ne) {
     const int v1 = M.verticesOnEdge[e], v2 = M.verticesOnEdge[M.ne + e];
     const T p1 = S.pv_v[v1], p2 = S.pv_v[v2];
     T pe = halve(p1 + p2);
@@ -1054,28 +1075,42 @@ __global__ void __launch_bounds__(kMaxBlock) k_combine(DevMesh M, int ntr, int s
   block_store<double, 4>(ip, P, r, (int)blockIdx.x - b0);
 }
 
-// Launch KERNEL<T, kB> over (GRIDX, members): the member-batched variant
-// (kB = true, FP32 only) when the stage has several ensemble members, else the
-// single-member code, which addresses its arrays straight from the kernel
-// parameters.
-#define TMC_LAUNCH(KERNEL, GRIDX, ...)                                     \
-  do {                                                                     \
-    if constexpr (!kF64<T>) {                                              \
-      if (S.members > 1) {                                                 \
-        KERNEL<T, true><<<dim3(GRIDX, nmem(S)), bs, 0, st>>>(__VA_ARGS__); \
-        break;                                                             \
-      }                                                                    \
-    }                                                                      \
-    KERNEL<T, false><<<dim3(GRIDX, 1), bs, 0, st>>>(__VA_ARGS__);          \
+// Launch KERNEL<T, kB, EPT> over n elements of every member: the
+// member-batched variant (kB = true, FP32 only) when the stage has several
+// ensemble members, else the single-member code, which addresses its arrays
+// straight from the kernel parameters, with b.ept elements per thread.
+#define TMC_LAUNCH(KERNEL, n, ...)                                                              \
+  do {                                                                                          \
+    if constexpr (!kF64<T>) {                                                                   \
+      if (S.members > 1) {                                                                      \
+        KERNEL<T, true, kEPT><<<dim3(grid_for(n, b.bs), nmem(S)), b.bs, 0, st>>>(__VA_ARGS__); \
+        break;                                                                                  \
+      }                                                                                         \
+    }                                                                                           \
+    if (b.ept == 1)                                                                             \
+      KERNEL<T, false, 1><<<grid_for(n, b), b.bs, 0, st>>>(__VA_ARGS__);                        \
+    else                                                                                        \
+      KERNEL<T, false, kEPT><<<grid_for(n, b), b.bs, 0, st>>>(__VA_ARGS__);                     \
+  } while (0)
+// the same for kernels of kEPT elements per thread only
+#define TMC_LAUNCH_4(KERNEL, n, ...)                                                       \
+  do {                                                                                     \
+    if constexpr (!kF64<T>) {                                                              \
+      if (S.members > 1) {                                                                 \
+        KERNEL<T, true><<<dim3(grid_for(n, bs), nmem(S)), bs, 0, st>>>(__VA_ARGS__);      \
+        break;                                                                             \
+      }                                                                                    \
+    }                                                                                      \
+    KERNEL<T, false><<<grid_for(n, bs), bs, 0, st>>>(__VA_ARGS__);                         \
   } while (0)
 
 template <class T>
 void launch_cons_apvm(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Partials P, double* diag_out, int bs,
                       cudaStream_t st) {
-  TMC_LAUNCH(k_cons_tvf, grid_for(M.ne, bs), M, S);
-  TMC_LAUNCH(k_cons_vertex, grid_for(M.nv, bs), M, S, P);
+  TMC_LAUNCH_4(k_cons_tvf, M.ne, M, S);
+  TMC_LAUNCH_4(k_cons_vertex, M.nv, M, S, P);
   launch_cons_eps(P, grid_for(M.nv, bs), O.dt, diag_out, st, (int)nmem(S));
-  TMC_LAUNCH(k_cons_apply, grid_for(M.ne, bs), M, O, S, diag_out + 10);
+  TMC_LAUNCH_4(k_cons_apply, M.ne, M, O, S, diag_out + 10);
 }
 
 template <class T>
@@ -1094,14 +1129,14 @@ void launch_combine(const DevMesh& M, int ntr, int scheme, const CombineArgs<T>&
 // ---------------------------------------------------------------------------
 // edge_flux: q.F_perp, gradient of E, iap_u tendency, RK update, inner products
 // ---------------------------------------------------------------------------
-template <class T, bool kB>
+template <class T, bool kB, int EPT>
 __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S0, RKStage rk,
                                                const Partials& P0) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
   T rip = T(0), r44 = T(0);  // FP32 path: FP32 products and per-thread sums, FP64 across warps
   const int mode = rk.mode;
-  TMC_FOR_EPT(e, M.ne) {
+  TMC_FOR_N(EPT, e, M.ne) {
     // Loads that depend on no other load come first, before any store: a load
     // issued after a store through a pointer the compiler must assume aliases
     // would wait a full memory round trip.
@@ -1214,7 +1249,10 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
         break;
       case 2:
       case 3: {
-        rip = fma_acc(tp * it, ae, rip);
+        if constexpr (kProducts<T, EPT>)
+          S.ipe[(size_t)(mode - 2) * M.ne + e] = tp * it;
+        else
+          rip = fma_acc(tp * it, ae, rip);
         if constexpr (kF64<T>)
           S.iap_acc[e] = __fma_rn(2.0, it, accv);  // 2 t is exact
         else
@@ -1224,14 +1262,20 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
         break;
       }
       case 4: {
-        rip = fma_acc(tp * it, ae, rip);
+        if constexpr (kProducts<T, EPT>)
+          S.ipe[(size_t)(mode - 2) * M.ne + e] = tp * it;
+        else
+          rip = fma_acc(tp * it, ae, rip);
         T tn;
         if constexpr (kF64<T>)
           tn = f64::div_r(accv + it, 6.0, 1.0 / 6.0);
         else
           tn = (accv + it) * (1.0f / 6.0f);
         S.iap_acc[e] = tn;
-        r44 = fma_acc(tn * tn, ae, r44);
+        if constexpr (kProducts<T, EPT>)
+          S.ipe[(size_t)3 * M.ne + e] = tn * tn;
+        else
+          r44 = fma_acc(tn * tn, ae, r44);
         tb[e] = it;
         break;
       }
@@ -1244,6 +1288,7 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
       S.iap_next[e] = inext;
     }
   }
+  if constexpr (kProducts<T, EPT>) return;
   if (rk.mode >= 2) {
     const T v[2] = {rip, r44};
     const int r[2] = {R_IP_E + 2 * (rk.mode - 2), R_44_E};
@@ -1253,46 +1298,46 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
 
 // the single-model kernel, and the ensemble kernel (member = blockIdx.y) with
 // its register budget capped so that member pointers do not halve occupancy
-template <class T>
+template <class T, int EPT>
 __global__ void __launch_bounds__(kMaxBlock) k_edge_flux(DevMesh M, ModelOpt O, StageIO<T> S0, RKStage rk, Partials P0) {
-  edge_flux_body<T, false>(M, O, S0, rk, P0);
+  edge_flux_body<T, false, EPT>(M, O, S0, rk, P0);
 }
 template <class T>
 __global__ void __launch_bounds__(kMemberBlock, TMC_FLUX_MIN_BLOCKS) k_edge_flux_members(DevMesh M, ModelOpt O, StageIO<T> S0, RKStage rk,
                                                                     Partials P0) {
-  edge_flux_body<T, true>(M, O, S0, rk, P0);
+  edge_flux_body<T, true, kEPT>(M, O, S0, rk, P0);
 }
 
 // new = old + (beta dt) t_new (update_state, tmcore_swm_mod.F90:203-213)
 // Cells: gd and tracer mass of state(old) in place, and their FP32 shadows.
-template <class T, bool kB>
+template <class T, bool kB, int EPT>
 __global__ void __launch_bounds__(kMaxBlock) k_final_cells(DevMesh M, ModelOpt O, StageIO<T> S0, const double* diag0) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const double* diag = kB ? diag0 + (size_t)blockIdx.y * kDiagStride : diag0;
   const double bdt = diag[9];
-  // all loads of the thread's kEPT cells before any store (a load after a
+  // all loads of the thread's EPT cells before any store (a load after a
   // store through a possibly aliasing pointer waits a full round trip)
-  const int i0 = blockIdx.x * (kEPT * blockDim.x) + threadIdx.x;
+  const int i0 = blockIdx.x * (EPT * blockDim.x) + threadIdx.x;
   double* gd = const_cast<double*>(S.gd_old);
-  double g[kEPT];
+  double g[EPT];
 #pragma unroll
-  for (int j = 0; j < kEPT; ++j) {
+  for (int j = 0; j < EPT; ++j) {
     const int i = i0 + j * blockDim.x;
     g[j] = i < M.nc ? gd[i] + bdt * S.gd_acc[i] : 0.0;
   }
 #pragma unroll
-  for (int j = 0; j < kEPT; ++j) {
+  for (int j = 0; j < EPT; ++j) {
     const int i = i0 + j * blockDim.x;
     if (i >= M.nc) continue;
     gd[i] = g[j];
     if constexpr (!kF64<T>) const_cast<float*>(S.gdf_in)[i] = (float)g[j];
   }
   T* qq = const_cast<T*>(S.q_old);
-  double rg[kEPT];  // FP64: 1 / gd
+  double rg[EPT];  // FP64: 1 / gd
   for (int q = 0; q < O.n_tracers; ++q) {
-    T qn[kEPT];
+    T qn[EPT];
 #pragma unroll
-    for (int j = 0; j < kEPT; ++j) {
+    for (int j = 0; j < EPT; ++j) {
       const int i = i0 + j * blockDim.x;
       const size_t qi = (size_t)q * M.nc + i;
       qn[j] = i < M.nc ? qq[qi] + T(bdt) * S.q_acc[qi] : T(0);
@@ -1300,9 +1345,9 @@ __global__ void __launch_bounds__(kMaxBlock) k_final_cells(DevMesh M, ModelOpt O
     if constexpr (kF64<T>)
       if (q == 0)
 #pragma unroll
-        for (int j = 0; j < kEPT; ++j) rg[j] = f64::recip(g[j]);
+        for (int j = 0; j < EPT; ++j) rg[j] = f64::recip(g[j]);
 #pragma unroll
-    for (int j = 0; j < kEPT; ++j) {
+    for (int j = 0; j < EPT; ++j) {
       const int i = i0 + j * blockDim.x;
       if (i >= M.nc) continue;
       const size_t qi = (size_t)q * M.nc + i;
@@ -1319,7 +1364,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_final_cells(DevMesh M, ModelOpt O
 // step's first stage (into S.gd_e/u/F/Fq) and the edge part of the total
 // energy of the new state (tmcore_swm_mod.F90:229) for the next step's
 // invariants.
-template <class T, bool kB>
+template <class T, bool kB, int EPT>
 __global__ void __launch_bounds__(kB ? kMemberBlock : kMaxBlock, kB ? TMC_FINAL_MIN_BLOCKS : TMC_FINAL_SINGLE_MIN_BLOCKS)
     k_final_edges(DevMesh M, ModelOpt O, StageIO<T> S0, const double* diag0, Partials P0) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
@@ -1328,13 +1373,13 @@ __global__ void __launch_bounds__(kB ? kMemberBlock : kMaxBlock, kB ? TMC_FINAL_
   const double bdt = diag[9];
   double en = 0.0;
   const CellSrc<T> C{S.gd_old, S.gdf_in, S.q_old, S.qr_in, S.ratio};
-  // loads of all kEPT edges first (see k_final_cells)
-  const int e0 = blockIdx.x * (kEPT * blockDim.x) + threadIdx.x;
+  // loads of all EPT edges first (see k_final_cells)
+  const int e0 = blockIdx.x * (EPT * blockDim.x) + threadIdx.x;
   T* iap = const_cast<T*>(S.iap_old);
-  int c1[kEPT], c2[kEPT];
-  T ia[kEPT], g1[kEPT], g2[kEPT], ae[kEPT];
+  int c1[EPT], c2[EPT];
+  T ia[EPT], g1[EPT], g2[EPT], ae[EPT];
 #pragma unroll
-  for (int j = 0; j < kEPT; ++j) {
+  for (int j = 0; j < EPT; ++j) {
     const int e = e0 + j * blockDim.x;
     const bool in = e < M.ne;
     c1[j] = in ? M.cellsOnEdge[e] : 0;
@@ -1343,7 +1388,7 @@ __global__ void __launch_bounds__(kB ? kMemberBlock : kMaxBlock, kB ? TMC_FINAL_
     ae[j] = in ? met<T>(M.areaEdge, M.areaEdge_f, e) : T(0);  // for the energy, loaded before any store
   }
 #pragma unroll
-  for (int j = 0; j < kEPT; ++j) {
+  for (int j = 0; j < EPT; ++j) {
     if constexpr (kF64<T>) {
       g1[j] = S.gd_old[c1[j]];
       g2[j] = S.gd_old[c2[j]];
@@ -1354,7 +1399,7 @@ __global__ void __launch_bounds__(kB ? kMemberBlock : kMaxBlock, kB ? TMC_FINAL_
   }
   float eh = 0.f, el = 0.f;  // FP32 path: the thread's few terms, compensated
 #pragma unroll
-  for (int j = 0; j < kEPT; ++j) {
+  for (int j = 0; j < EPT; ++j) {
     const int e = e0 + j * blockDim.x;
     if (e >= M.ne) continue;
     iap[e] = ia[j];
@@ -1365,6 +1410,7 @@ __global__ void __launch_bounds__(kB ? kMemberBlock : kMaxBlock, kB ? TMC_FINAL_
     else
       two_sum_acc(eh, el, ia[j] * ia[j] * ae[j]);
   }
+  if constexpr (kProducts<T, EPT>) return;
   const int r[1] = {R_EN_E};
   if constexpr (kF64<T>) {
     const double v[1] = {en};
@@ -1398,9 +1444,9 @@ inline int nblk(int n, int bs) { return (n + bs - 1) / bs; }
 
 
 template <class T>
-void launch_edge_prep(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Partials P, bool diag, int bs,
+void launch_edge_prep(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Partials P, bool diag, Blk b,
                       cudaStream_t st) {
-  TMC_LAUNCH(k_edge_prep, grid_for(M.ne, bs), M, O, S, P, diag ? 1 : 0);
+  TMC_LAUNCH(k_edge_prep, M.ne, M, O, S, P, diag ? 1 : 0);
 }
 // The second-order tracer terms of the FP32 cell pass (the mass-weighted
 // form d(gd q)/dt = div_operator(F q_edge), q_edge the mean of the two
@@ -1446,7 +1492,7 @@ __device__ __forceinline__ void tracer_update_f(const StageIO<float>& S, size_t 
 // (indices and the cell's own values, then the gathers of the edges' u, F,
 // dvEdge, areaEdge and of the neighbours' tracer mixing ratios), so one cell
 // costs two memory round trips.  Same arithmetic as the FP32 branch of k_cell.
-template <int NTR, bool kB>
+template <int NTR, bool kB, int EPT>
 __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<float>& S0, RKStage rk,
                                                const Partials& P0, int diag) {
   const StageIO<float> S = kB ? S0.at(blockIdx.y) : S0;
@@ -1456,7 +1502,7 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
   double mass = 0.0;
   float eh = 0.f, el = 0.f;
   const int mode = rk.mode;
-  TMC_FOR_EPT(c, M.nc) {
+  TMC_FOR_N(EPT, c, M.nc) {
     int ei[kME], ci[kME];
     float ns[kME];
 #pragma unroll
@@ -1520,17 +1566,25 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
         break;
       case 2:
       case 3:
-        rip += tprev * tT * Af;
+        if constexpr (kProducts<float, EPT>)
+          S.ipc[(size_t)(mode - 2) * M.nc + c] = tprev * tT;
+        else
+          rip += tprev * tT * Af;
         S.gd_acc[c] = gacc + 2.0 * t;
         S.tendf[c] = tT;
         gnext = gold + rk.a_dt * t;
         break;
       default: {
-        rip += tprev * tT * Af;
         const double tn = (gacc + t) * (1.0 / 6.0);
         S.gd_acc[c] = tn;
         const float tnf = (float)tn;
-        r44 += tnf * tnf * Af;
+        if constexpr (kProducts<float, EPT>) {
+          S.ipc[(size_t)2 * M.nc + c] = tprev * tT;
+          S.ipc[(size_t)3 * M.nc + c] = tnf * tnf;
+        } else {
+          rip += tprev * tT * Af;
+          r44 += tnf * tnf * Af;
+        }
         S.tendf[c] = tT;
       }
     }
@@ -1540,7 +1594,7 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
       S.gdf_next[c] = gnf;
     }
     tracer_update_f<NTR, NQ>(S, M.nc, c, mode, (float)rk.a_dt, tq, qo, qa, gnf);
-    if (diag) {
+    if (!kProducts<float, EPT> && diag) {
       // total mass from the FP64 gd; the cell part of the total energy
       // (gd^2 + 2 gd ghs) areaCell (tmcore_swm_mod.F90:215-231) from FP32
       // terms with a compensated sum (an FP64 term would cost four FP64
@@ -1549,31 +1603,31 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
       two_sum_acc(eh, el, gdf * (gdf + 2.f * ghf) * Afd);
     }
   }
-  if (mode >= 2) {
+  if (!kProducts<float, EPT> && mode >= 2) {
     const float v[2] = {rip, r44};
     const int r[2] = {R_IP_C + 2 * (mode - 2), R_44_C};
     block_store<float, 2>(v, P, r);
   }
-  if (diag) {
+  if (!kProducts<float, EPT> && diag) {
     const double v[2] = {mass, (double)eh + (double)el};
     const int r[2] = {R_MASS, R_EN_C};
     block_store<double, 2>(v, P, r);
   }
 }
 
-template <int NTR>
+template <int NTR, int EPT>
 __global__ void __launch_bounds__(kCellBlock, TMC_CELL_SINGLE_MIN_BLOCKS) k_cell_fast(DevMesh M, StageIO<float> S0, RKStage rk, Partials P0,
                                                          int diag) {
-  cell_fast_body<NTR, false>(M, S0, rk, P0, diag);
+  cell_fast_body<NTR, false, EPT>(M, S0, rk, P0, diag);
 }
 // The tracer terms of the FP32 cell pass alone, for a stage whose cell pass
 // ran tracer-free (k_cell_fast<0>): the same loads and the same arithmetic
 // (tracer_tend_f, tracer_update_f) as k_cell_fast<NTR>, with the stage's next
 // gd in FP32 read back from S.gdf_next.  Single member.
-template <int NTR>
+template <int NTR, int EPT>
 __global__ void __launch_bounds__(kCellBlock) k_tracers_fast(DevMesh M, StageIO<float> S, RKStage rk) {
   const int mode = rk.mode;
-  TMC_FOR_EPT(c, M.nc) {
+  TMC_FOR_N(EPT, c, M.nc) {
     int ei[kME], ci[kME];
     float ns[kME];
 #pragma unroll
@@ -1611,98 +1665,96 @@ __global__ void __launch_bounds__(kCellBlock) k_tracers_fast(DevMesh M, StageIO<
 template <int NTR>
 __global__ void __launch_bounds__(kMemberBlock, NTR == 0 ? TMC_CELL_MIN_BLOCKS : 3) k_cell_fast_members(DevMesh M, StageIO<float> S0, RKStage rk,
                                                                     Partials P0, int diag) {
-  cell_fast_body<NTR, true>(M, S0, rk, P0, diag);
+  cell_fast_body<NTR, true, kEPT>(M, S0, rk, P0, diag);
 }
 
 template <class T>
-void launch_cell(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Partials P, bool diag, int bs,
+void launch_cell(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Partials P, bool diag, Blk b,
                  cudaStream_t st) {
   if constexpr (!kF64<T>) {
-    const bool fast = rk.mode >= 1 && rk.mode <= 4 && (O.n_tracers == 0 || O.tr_order == 2);
+    const bool fast = rk.mode >= 1 && rk.mode <= 4 && launch_cell_is_fast(O);
+    const int dg = diag ? 1 : 0;
+    auto run = [&](auto ntr) {
+      constexpr int N = decltype(ntr)::value;
+      if (S.members > 1)
+        k_cell_fast_members<N><<<dim3(grid_for(M.nc, b.bs), nmem(S)), b.bs, 0, st>>>(M, S, rk, P, dg);
+      else if (b.ept == 1)
+        k_cell_fast<N, 1><<<grid_for(M.nc, b), b.bs, 0, st>>>(M, S, rk, P, dg);
+      else
+        k_cell_fast<N, kEPT><<<grid_for(M.nc, b), b.bs, 0, st>>>(M, S, rk, P, dg);
+    };
     if (fast) {
-      const int g = grid_for(M.nc, bs), dg = diag ? 1 : 0;
       switch (O.n_tracers) {
-        case 0:
-          if (S.members > 1)
-            k_cell_fast_members<0><<<dim3(g, nmem(S)), bs, 0, st>>>(M, S, rk, P, dg);
-          else
-            k_cell_fast<0><<<g, bs, 0, st>>>(M, S, rk, P, dg);
-          return;
-        case 1:
-          if (S.members > 1)
-            k_cell_fast_members<1><<<dim3(g, nmem(S)), bs, 0, st>>>(M, S, rk, P, dg);
-          else
-            k_cell_fast<1><<<g, bs, 0, st>>>(M, S, rk, P, dg);
-          return;
-        case 2:
-          if (S.members > 1)
-            k_cell_fast_members<2><<<dim3(g, nmem(S)), bs, 0, st>>>(M, S, rk, P, dg);
-          else
-            k_cell_fast<2><<<g, bs, 0, st>>>(M, S, rk, P, dg);
-          return;
-        case 4:
-          if (S.members > 1)
-            k_cell_fast_members<4><<<dim3(g, nmem(S)), bs, 0, st>>>(M, S, rk, P, dg);
-          else
-            k_cell_fast<4><<<g, bs, 0, st>>>(M, S, rk, P, dg);
-          return;
+        case 0: run(std::integral_constant<int, 0>()); return;
+        case 1: run(std::integral_constant<int, 1>()); return;
+        case 2: run(std::integral_constant<int, 2>()); return;
+        case 4: run(std::integral_constant<int, 4>()); return;
         default: break;
       }
     }
   }
-  TMC_LAUNCH(k_cell, grid_for(M.nc, bs), M, O, S, rk, P, diag ? 1 : 0);
+  TMC_LAUNCH(k_cell, M.nc, M, O, S, rk, P, diag ? 1 : 0);
 }
 template <class T>
-void launch_tracers_fast(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, int bs,
+void launch_tracers_fast(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Blk b,
                          cudaStream_t st) {
   if constexpr (!kF64<T>) {
-    const int g = grid_for(M.nc, bs);
+    auto run = [&](auto ntr) {
+      constexpr int N = decltype(ntr)::value;
+      if (b.ept == 1)
+        k_tracers_fast<N, 1><<<grid_for(M.nc, b), b.bs, 0, st>>>(M, S, rk);
+      else
+        k_tracers_fast<N, kEPT><<<grid_for(M.nc, b), b.bs, 0, st>>>(M, S, rk);
+    };
     switch (O.n_tracers) {
-      case 1: k_tracers_fast<1><<<g, bs, 0, st>>>(M, S, rk); return;
-      case 2: k_tracers_fast<2><<<g, bs, 0, st>>>(M, S, rk); return;
-      case 4: k_tracers_fast<4><<<g, bs, 0, st>>>(M, S, rk); return;
+      case 1: run(std::integral_constant<int, 1>()); return;
+      case 2: run(std::integral_constant<int, 2>()); return;
+      case 4: run(std::integral_constant<int, 4>()); return;
       default: return;
     }
   }
 }
 template <class T>
-void launch_vertex(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Partials P, bool diag, int bs,
+void launch_vertex(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Partials P, bool diag, Blk b,
                    cudaStream_t st) {
-  TMC_LAUNCH(k_vertex, grid_for(M.nv, bs), M, O, S, P, diag ? 1 : 0);
+  TMC_LAUNCH(k_vertex, M.nv, M, O, S, P, diag ? 1 : 0);
 }
 template <class T>
-void launch_edge_pv(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, int bs, cudaStream_t st) {
+void launch_edge_pv(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Blk b, cudaStream_t st) {
   if ((O.pv_scheme == 1 && O.apvm_weight != 0.0) || O.pv_scheme == 2 || O.need_pv_c)
-    k_v2c<T><<<dim3(grid_for(M.nc, bs), nmem(S)), bs, 0, st>>>(M, S.pv_v, S.pv_c, S.msv, S.msc);
+    k_v2c<T, kEPT><<<dim3(grid_for(M.nc, b.bs), nmem(S)), b.bs, 0, st>>>(M, S.pv_v, S.pv_c, S.msv, S.msc);
   if constexpr (!kF64<T>) {
     if (O.pv_scheme == 3 && (O.interp_pv_order == 3 || O.interp_pv_order == 4) && M.vert2_iw) {
-      const int b = bs < 256 ? bs : 256;  // compiled for at most 256 threads per block
-      const dim3 g(nblk(M.ne, b), nmem(S));
+      const int bs = b.bs < 256 ? b.bs : 256;  // compiled for at most 256 threads per block
+      const dim3 g(nblk(M.ne, bs), nmem(S));
       if (S.members > 1)
-        k_edge_pv_up32<true><<<g, b, 0, st>>>(M, O, S);
+        k_edge_pv_up32<true><<<g, bs, 0, st>>>(M, O, S);
       else
-        k_edge_pv_up32<false><<<g, b, 0, st>>>(M, O, S);
+        k_edge_pv_up32<false><<<g, bs, 0, st>>>(M, O, S);
       return;
     }
   }
-  TMC_LAUNCH(k_edge_pv, grid_for(M.ne, bs), M, O, S);
+  TMC_LAUNCH(k_edge_pv, M.ne, M, O, S);
 }
 template <class T>
-void launch_edge_flux(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Partials P, int bs,
+void launch_edge_flux(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Partials P, Blk b,
                       cudaStream_t st) {
   if constexpr (!kF64<T>) {
     if (S.members > 1) {
-      k_edge_flux_members<T><<<dim3(grid_for(M.ne, bs), nmem(S)), bs, 0, st>>>(M, O, S, rk, P);
+      k_edge_flux_members<T><<<dim3(grid_for(M.ne, b.bs), nmem(S)), b.bs, 0, st>>>(M, O, S, rk, P);
       return;
     }
   }
-  k_edge_flux<T><<<grid_for(M.ne, bs), bs, 0, st>>>(M, O, S, rk, P);
+  if (b.ept == 1)
+    k_edge_flux<T, 1><<<grid_for(M.ne, b), b.bs, 0, st>>>(M, O, S, rk, P);
+  else
+    k_edge_flux<T, kEPT><<<grid_for(M.ne, b), b.bs, 0, st>>>(M, O, S, rk, P);
 }
 template <class T>
 void launch_final_update(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, const double* diag, Partials P,
-                         int bs, cudaStream_t st) {
-  TMC_LAUNCH(k_final_cells, grid_for(M.nc, bs), M, O, S, diag);
-  TMC_LAUNCH(k_final_edges, grid_for(M.ne, bs), M, O, S, diag, P);
+                         Blk b, cudaStream_t st) {
+  TMC_LAUNCH(k_final_cells, M.nc, M, O, S, diag);
+  TMC_LAUNCH(k_final_edges, M.ne, M, O, S, diag, P);
 }
 template <class T>
 void launch_gather(int n, const double* src, const int32_t* n2o, T* dst, cudaStream_t st) {
@@ -1758,19 +1810,19 @@ void launch_to_f64(size_t n, const T* src, double* dst, cudaStream_t st) {
   template void launch_gather<T>(int, const double*, const int32_t*, T*, cudaStream_t);                          \
   template void launch_scatter<T>(int, const T*, const int32_t*, double*, cudaStream_t);                         \
   template void launch_iap_from_u<T>(int, const double*, const double*, T*, cudaStream_t);                       \
-  template void launch_edge_prep<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, Partials, bool, int,     \
+  template void launch_edge_prep<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, Partials, bool, Blk,     \
                                     cudaStream_t);                                                                \
-  template void launch_cell<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, Partials, bool, int, \
+  template void launch_cell<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, Partials, bool, Blk, \
                                cudaStream_t);                                                                     \
-  template void launch_tracers_fast<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, int,           \
+  template void launch_tracers_fast<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, Blk,           \
                                        cudaStream_t);                                                             \
-  template void launch_vertex<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, Partials, bool, int,        \
+  template void launch_vertex<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, Partials, bool, Blk,        \
                                  cudaStream_t);                                                                   \
-  template void launch_edge_pv<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, int, cudaStream_t);        \
-  template void launch_edge_flux<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, Partials, int,  \
+  template void launch_edge_pv<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, Blk, cudaStream_t);        \
+  template void launch_edge_flux<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, Partials, Blk,  \
                                     cudaStream_t);                                                                \
   template void launch_final_update<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, const double*,         \
-                                       Partials, int, cudaStream_t);                                             \
+                                       Partials, Blk, cudaStream_t);                                             \
   template void launch_cons_apvm<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, Partials, double*, int,   \
                                     cudaStream_t);                                                                \
   template void launch_update<T>(const DevMesh&, int, const UpdateArgs<T>&, int, cudaStream_t);                 \
