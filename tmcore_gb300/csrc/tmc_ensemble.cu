@@ -16,6 +16,7 @@
 #include <cstring>
 
 #include "tmc_ensemble.cuh"
+#include "tmc_fp64.cuh"
 
 // Minimum resident blocks per SM the heavy passes are compiled for (0: none
 // given).  Any minimum changes the compiler's register heuristics: on 512
@@ -77,16 +78,13 @@ __device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float p) {
   lo = __fadd_rn(lo, err);
 }
 
-struct DD {
-  double hi, lo;
-};
-__device__ __forceinline__ DD dd_add(DD a, DD b) {
-  const double s = __dadd_rn(a.hi, b.hi);
-  const double bb = __dsub_rn(s, a.hi);
-  double e = __dadd_rn(__dsub_rn(a.hi, __dsub_rn(s, bb)), __dsub_rn(b.hi, bb));
-  e = __dadd_rn(e, __dadd_rn(a.lo, b.lo));
-  const double hi = __dadd_rn(s, e);
-  return {hi, __dsub_rn(e, __dsub_rn(hi, s))};
+// FP32 -> FP64 by moving the fields (the conversion instruction runs on the
+// 2-lane FP64 pipe); zeros, subnormals, infinities and NaN convert
+__device__ __forceinline__ double widen(float x) {
+  const unsigned b = __float_as_uint(x), e = (b >> 23) & 0xff;
+  if (e - 1u < 254u)
+    return __hiloint2double((int)((b & 0x80000000u) | ((e + 896u) << 20) | ((b >> 3) & 0xfffffu)), (int)(b << 29));
+  return (double)x;
 }
 
 // Double-float (FF) arithmetic for gd: a value h + l with |l| <= ulp(h) / 2.
@@ -921,9 +919,8 @@ __global__ void __launch_bounds__(kMaxBS) k_ens_edges(DevMesh Mh, Dims D, IO S, 
 // ---------------------------------------------------------------------------
 // reduction of the per-thread partials: block = (region, group of 32
 // members), warp w sums slots w, w + W, ... for its 32 members (FP32 TwoSum
-// for the step products, FP64 for the invariants), warp 0 combines the warps
-// in double-double and stores the region sum after the member's kDiagLen
-// outputs.
+// for the step products, FP64 for the invariants), the warps' sums of each
+// member are added and stored after the member's kDiagLen outputs.
 // ---------------------------------------------------------------------------
 struct RegionList {
   int n;
@@ -933,17 +930,21 @@ struct RegionList {
 
 // One block per (region, group of 32 members), 32 warps: warp w takes slots
 // w, w + 32, ... in rounds of four with four independent accumulators (all
-// four loads in flight), which it combines in a fixed order; the warps'
-// sums are then combined in warp order.  Deterministic for a given slot
-// count.  (With 8 warps and one accumulator the 7,680 slots of a level-7
-// edge region took about 0.3 ms, a quarter of a 16-member step.)
+// four loads in flight), which it adds in a fixed order; then warp m adds the
+// warps' sums of member m, as exact integers (f64::warp_sum).  Deterministic
+// for a given slot count.  The block is bound by FP64 instructions (64 cycles
+// each, warp-wide): combining the accumulators and the warps in double-double
+// took 36.9 us for 64 level-6 members, plain FP64 sums of four and the integer
+// sum across warps take 14.5 us.  (With 8 warps and one accumulator the 7,680
+// slots of a level-7 edge region took about 0.3 ms, a quarter of a 16-member
+// step.)
 constexpr int kRedThreads = 1024;
 __device__ __forceinline__ void ens_reduce(const Partials& P, int r, int count, double* diag_out) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  constexpr int nw = kRedThreads / 32;
   const int m = blockIdx.y * 32 + lane;
-  const bool in = m < P.M;
-  DD acc{0.0, 0.0};
-  if (in) {
+  double acc = 0.0;
+  if (m < P.M) {
     if (r <= R_44_E) {
       float fh[4] = {0.f, 0.f, 0.f, 0.f}, fl[4] = {0.f, 0.f, 0.f, 0.f};
       int s = w;
@@ -957,8 +958,8 @@ __device__ __forceinline__ void ens_reduce(const Partials& P, int r, int count, 
 #pragma unroll
       for (int q = 0; q < 3; ++q)  // the last at most 3 slots of this warp
         if (s + q * nw < count) two_sum_acc(fh[q], fl[q], P.f(r, s + q * nw)[m]);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc = dd_add(acc, DD{(double)fh[q], (double)fl[q]});
+      acc = ((widen(fh[0]) + widen(fh[1])) + (widen(fh[2]) + widen(fh[3]))) +
+            ((widen(fl[0]) + widen(fl[1])) + (widen(fl[2]) + widen(fl[3])));
     } else {
       double dh[4] = {0.0, 0.0, 0.0, 0.0};
       int s = w;
@@ -972,53 +973,57 @@ __device__ __forceinline__ void ens_reduce(const Partials& P, int r, int count, 
 #pragma unroll
       for (int q = 0; q < 3; ++q)
         if (s + q * nw < count) dh[q] += P.d(r, s + q * nw)[m];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc = dd_add(acc, DD{dh[q], 0.0});
+      acc = (dh[0] + dh[1]) + (dh[2] + dh[3]);
     }
   }
-  __shared__ double sh[kRedThreads / 32][32], sl[kRedThreads / 32][32];
-  sh[w][lane] = acc.hi;
-  sl[w][lane] = acc.lo;
+  static_assert(nw == 32, "warp m sums member m over the warps");
+  __shared__ double sh[nw][33];
+  sh[w][lane] = acc;
   __syncthreads();
-  if (w != 0 || !in) return;
-  DD tot{0.0, 0.0};
-  for (int k = 0; k < nw; ++k) tot = dd_add(tot, DD{sh[k][lane], sl[k][lane]});
-  diag_out[(size_t)m * kDiagStride + kDiagLen + r] = tot.hi + tot.lo;
+  const double tot = f64::value(f64::warp_sum(sh[lane][w]));  // lane = warp, w = member
+  const int mm = blockIdx.y * 32 + w;
+  if (lane == 0 && mm < P.M) diag_out[(size_t)mm * kDiagStride + kDiagLen + r] = tot;
 }
 __global__ void __launch_bounds__(kRedThreads) k_ens_reduce(Partials P, RegionList RL, double* diag_out) {
   ens_reduce(P, RL.r[blockIdx.x], RL.count[blockIdx.x], diag_out);
 }
 
 // beta (time_scheme_mod.F90:144-150) and the invariants (tmcore_swm_mod.F90:215-255)
-// of every member from its region sums
+// of member m from its region sums, by four lanes (k = 0..3, lanes of one
+// warp): lane k forms R[k], so that the dependent FP64 quotients run side by
+// side and a warp holds eight members (one thread per member in blocks of
+// 256: 6.3 us; eight members per block of a warp: 4.2 us)
+constexpr int kBetaMembers = 8;
 __device__ __forceinline__ void ens_beta(int M, int step, int diag, int conserve, double totalArea,
-                                         double sumAreaTriangle, double dt, double* diag_out, int m) {
-  if (m >= M) return;
-  double* out = diag_out + (size_t)m * kDiagStride;
+                                         double sumAreaTriangle, double dt, double* diag_out, int m, int k) {
+  double* out = diag_out + (size_t)min(m, M - 1) * kDiagStride;
   const double* rv = out + kDiagLen;
   if (step) {
+    const double Rk = (rv[k < 3 ? R_IP_E + 2 * k : R_44_E] + rv[k < 3 ? R_IP_C + 2 * k : R_44_C]) / totalArea;
     double R[4];
-    for (int k = 0; k < 3; ++k) R[k] = (rv[R_IP_E + 2 * k] + rv[R_IP_C + 2 * k]) / totalArea;
-    R[3] = (rv[R_44_E] + rv[R_44_C]) / totalArea;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) R[q] = __shfl_sync(0xffffffffu, Rk, (threadIdx.x & 28) + q);
     // beta = 1 for a member whose tendency is zero everywhere (k_finalize)
     const double beta = conserve && R[3] != 0.0 ? (R[0] + R[1] + R[2]) / (3.0 * R[3]) : 1.0;
-    out[4] = beta;
-    out[5] = R[0];
-    out[6] = R[1];
-    out[7] = R[2];
-    out[8] = R[3];
-    out[9] = beta * dt;
+    if (m < M) {
+      out[5 + k] = Rk;
+      if (k == 0) {
+        out[4] = beta;
+        out[9] = beta * dt;
+      }
+    }
   }
-  if (diag) {
+  if (diag && m < M && k == 0) {
     out[0] = rv[R_MASS];
     out[1] = rv[R_EN_E] + rv[R_EN_C];
     out[2] = rv[R_PE];
     out[3] = rv[R_AV] / sumAreaTriangle;
   }
 }
-__global__ void k_ens_beta(int M, int step, int diag, int conserve, double totalArea, double sumAreaTriangle,
-                           double dt, double* diag_out) {
-  ens_beta(M, step, diag, conserve, totalArea, sumAreaTriangle, dt, diag_out, blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(32) k_ens_beta(int M, int step, int diag, int conserve, double totalArea,
+                                                 double sumAreaTriangle, double dt, double* diag_out) {
+  ens_beta(M, step, diag, conserve, totalArea, sumAreaTriangle, dt, diag_out,
+           blockIdx.x * kBetaMembers + (threadIdx.x >> 2), threadIdx.x & 3);
 }
 
 // pv on cells for the learned closure: scalar_v2c_interp_operator as a
@@ -1181,10 +1186,10 @@ __global__ void __launch_bounds__(kRedThreads) k_jobs_reduce(const __grid_consta
   ens_reduce(J.P, R.r[i], count, J.diag);
 }
 // beta of every member of every job (blockIdx.y = job)
-__global__ void k_jobs_beta(const __grid_constant__ JobTable T) {
+__global__ void __launch_bounds__(32) k_jobs_beta(const __grid_constant__ JobTable T) {
   const Job& J = T.job[blockIdx.y];
   ens_beta(J.D.M, 1, 0, J.conserve, J.totalArea, J.sumAreaTriangle, J.dt, J.diag,
-           blockIdx.x * blockDim.x + threadIdx.x);
+           blockIdx.x * kBetaMembers + (threadIdx.x >> 2), threadIdx.x & 3);
 }
 
 }  // namespace
@@ -1293,7 +1298,7 @@ void launch_finalize(const Dims& D, const Partials& P, bool step, bool diag, boo
   }
   if (RL.n == 0) return;
   k_ens_reduce<<<dim3(RL.n, D.G), kRedThreads, 0, st>>>(P, RL, diag_out);
-  k_ens_beta<<<nb(D.M), 256, 0, st>>>(D.M, step ? 1 : 0, diag ? 1 : 0, conserve ? 1 : 0, totalArea,
+  k_ens_beta<<<(D.M + kBetaMembers - 1) / kBetaMembers, 32, 0, st>>>(D.M, step ? 1 : 0, diag ? 1 : 0, conserve ? 1 : 0, totalArea,
                                       sumAreaTriangle, dt, diag_out);
 }
 
@@ -1403,7 +1408,7 @@ void launch_jobs_step(const JobTable& T, int nj, const int* bsp, bool upwind, cu
   R.r[R.n] = R_44_C, R.kind[R.n++] = J_CELLS;
   R.r[R.n] = R_44_E, R.kind[R.n++] = J_EDGES;
   k_jobs_reduce<<<dim3((unsigned)(nj * R.n), (unsigned)D.G), kRedThreads, 0, st>>>(T, R);
-  k_jobs_beta<<<dim3(nb(D.M), (unsigned)nj), 256, 0, st>>>(T);
+  k_jobs_beta<<<dim3((unsigned)((D.M + kBetaMembers - 1) / kBetaMembers), (unsigned)nj), 32, 0, st>>>(T);
   const StageTable S0 = stage_table(T, nj, 0);
   if (D.V == 2) {
     k_jobs_final_cells<2><<<gc, th[4], 0, st>>>(S0, nj);
