@@ -210,6 +210,8 @@ struct Engine : EngineBase {
   T* Fq[2] = {};
   double *sq[2] = {}, *hu[2] = {}, *ke[2] = {}, *ud[2] = {};  // FP64 path (StageIO)
   double* ratio = nullptr;
+  float* uf[2] = {};
+  T* dfit = nullptr;  // upwind pv (StageIO)
   double *gd_acc = nullptr, *gd_tend = nullptr, *ghs = nullptr;
   T* q_acc = nullptr;
   T *iap_acc = nullptr, *iap_tend = nullptr, *E = nullptr;
@@ -276,6 +278,11 @@ struct Engine : EngineBase {
         if (!sq[i] || !hu[i] || !ke[i] || !ud[i]) return TMC_E_CUDA;
       }
       if (!(ratio = h->dalloc<double>(nq))) return TMC_E_CUDA;
+    }
+    if (h->M.vfit_n) {
+      if (!(dfit = h->dalloc<T>(2 * ne))) return TMC_E_CUDA;
+      for (int i = 0; std::is_same<T, double>::value && i < 2; ++i)
+        if (!(uf[i] = h->dalloc<float>(ne))) return TMC_E_CUDA;
     }
     if (h->O.pv_scheme == 2) {
       dpv = h->dalloc<T>(ne);
@@ -349,6 +356,9 @@ struct Engine : EngineBase {
     s.hu_nx = hu[1 - set];
     s.ke_nx = ke[1 - set];
     s.ud_nx = ud[1 - set];
+    s.uf = uf[set];
+    s.uf_nx = uf[1 - set];
+    s.dfit = dfit;
     s.ratio = ratio;
     s.ipc = h->ipc;
     s.ipe = h->ipe;
@@ -380,7 +390,7 @@ struct Engine : EngineBase {
 
   int launches_per_stage_passes() const {
     const bool v2c = (h->O.pv_scheme == 1 && h->O.apvm_weight != 0.0) || h->O.pv_scheme == 2;
-    return 4 + (v2c ? 1 : 0) + (h->O.pv_scheme == 2 ? 4 : 0);
+    return 4 + (v2c ? 1 : 0) + (h->O.pv_scheme == 2 ? 4 : 0) + (h->M.vfit_n ? 1 : 0);
   }
   int launches_per_step() const override {
     if (!h->generic) return 4 * launches_per_stage_passes() + 3;
@@ -1114,7 +1124,7 @@ void choose_launch_shapes(tmc_handle* h, bool default_blocks) {
   int line[P_COUNT];
   line[P_CELL] = f64 ? big : small;
   line[P_VERTEX] = f64 ? big : small;
-  line[P_PV] = f64 && h->O.pv_scheme == 3 ? big : small;
+  line[P_PV] = h->M.vfit_n ? big : small;  // (k_vert_fit, k_edge_up: always one, the line sets their blocks)
   line[P_FLUX] = line[P_FINAL] = f64 ? big : small;
   for (int k = 0; k < P_COUNT; ++k) {
     if (n[k] >= line[k]) continue;
@@ -1403,18 +1413,45 @@ int tmc_create(const tmc_mesh_desc* mesh, const tmc_params* params, tmc_handle**
   M.cell4 = upload_stencil(h.get(), hm.cell4);
   M.vert2 = upload_stencil(h.get(), hm.vert2);
   M.vert4 = upload_stencil(h.get(), hm.vert4);
-  if (p.precision == TMC_FP32 && p.pv_scheme == 3 && (p.interp_pv_order == 3 || p.interp_pv_order == 4) &&
-      hm.vert2.width > 0 && hm.vert2.width <= kUpW32) {
-    // the packed FP32 form of the vertex fit stencils (k_edge_pv_up32)
-    std::vector<int2> iw(hm.vert2.idx.size());
-    for (size_t k = 0; k < iw.size(); ++k) {
-      const float wf = (float)hm.vert2.w[k];
-      int wb;
-      std::memcpy(&wb, &wf, sizeof(wb));
-      iw[k] = make_int2(hm.vert2.idx[k], wb);
+  if (p.pv_scheme == 3 && (p.interp_pv_order == 3 || p.interp_pv_order == 4) && hm.vert2.width > 0 &&
+      p.member_layout == 0) {
+    // the vertex fit stencils by vertex: an edge's side has the points of its
+    // vertex, in the vertex's order, and weights of its own
+    const int W = hm.vert2.width, nv = hm.nv;
+    const size_t ne = hm.ne;
+    std::vector<uint8_t> n(nv);
+    std::vector<int32_t> idx((size_t)W * nv, 0);
+    std::vector<double> w((size_t)W * 3 * nv, 0.0);
+#pragma omp parallel for schedule(static)
+    for (int v = 0; v < nv; ++v)
+      for (int k = 0; k < 3; ++k) {
+        const size_t e = hm.edgesOnVertex[(size_t)k * nv + v];
+        const size_t sd = hm.tSignEdge[(size_t)k * nv + v] > 0 ? 0 : 1;
+        n[v] = hm.vert2.count[sd * ne + e];
+        for (int j = 0; j < n[v]; ++j) {
+          const size_t q = ((size_t)j * 2 + sd) * ne + e;
+          idx[(size_t)j * nv + v] = hm.vert2.idx[q];
+          w[((size_t)j * 3 + k) * nv + v] = hm.vert2.w[q];
+        }
+      }
+    M.vfit_n = h->upload(n);
+    if (p.precision == TMC_FP32) {
+      std::vector<float4> rec((size_t)W * nv);
+#pragma omp parallel for schedule(static)
+      for (int j = 0; j < W; ++j)
+        for (int v = 0; v < nv; ++v) {
+          const double* wv = &w[(size_t)j * 3 * nv + v];
+          float ib;
+          std::memcpy(&ib, &idx[(size_t)j * nv + v], sizeof(ib));
+          rec[(size_t)j * nv + v] = make_float4((float)wv[0], (float)wv[nv], (float)wv[2 * (size_t)nv], ib);
+        }
+      M.vfit_rec = h->upload(rec);
+    } else {
+      M.vfit_idx = h->upload(idx);
+      M.vfit_w = h->upload(w);
+      M.weightsOnEdge_f = h->upload(std::vector<float>(hm.weightsOnEdge.begin(), hm.weightsOnEdge.end()));
     }
-    M.vert2_iw = h->upload(iw);
-    if (!M.vert2_iw) {
+    if (!M.vfit_n || (!M.vfit_rec && (!M.vfit_idx || !M.vfit_w)) || !M.weightsOnEdge_f) {
       h->err = "device allocation failed";
       cudaGetLastError();
       *out = h.release();

@@ -34,7 +34,6 @@
 namespace tmc {
 
 constexpr int kEPT = 4;  // elements per thread (one on small meshes, see Blk)
-constexpr int kUpW32 = 16;  // widest vertex fit stencil of the packed FP32 upwind pv kernel
 
 struct DStencil {
   int width;
@@ -68,12 +67,15 @@ struct DevMesh {
   const int32_t* v2c_vertex;
   const double* v2c_kite;
   DStencil cell2, cell3, cell4, vert2, vert4;  // cell3: deriv3OnCell on the fit3 (= fit4) stencils
-  // FP32 path with upwind pv of order 3 or 4 (pv_scheme 3): vert2 packed as
-  // (stencil vertex, FP32 weight bits) entries [width][2][ne], width at most
-  // kUpW32 (null otherwise: the generic stencil loop runs)
-  const int2* vert2_iw;
+  // upwind pv of order 3 or 4 (pv_scheme 3): the vertex fit stencils by vertex,
+  // point j of vertex v and its weights for the vertex's three edges (null
+  // otherwise: the generic stencil loop runs)
+  const uint8_t* vfit_n;    // [nv] points
+  const int32_t* vfit_idx;  // [width][nv] and
+  const double* vfit_w;     // [width][3][nv]: FP64 path
+  const float4* vfit_rec;   // [width][nv] three weights, point (bits): FP32 path
   // FP32 path: FP32-rounded copies of the metrics used in FP32 arithmetic
-  // (null in FP64 mode)
+  // (null in FP64 mode, but for weightsOnEdge_f with vfit_n)
   const float* weightsOnEdge_f;
   const float* dcEdge_f;
   const float* dvEdge_f;
@@ -192,6 +194,7 @@ struct StageIO {
   // tracers' mixing ratios [ntr][nc] of the next stage's state
   double *sq, *hu, *ke, *ud;
   double *sq_nx, *hu_nx, *ke_nx, *ud_nx;
+  float *uf, *uf_nx;  // with vfit_n: u in FP32
   double* ratio;
   // FP32 path, one element per thread: factors of the CRK4 inner products
   // [4][nc] and [4][ne] (t1 t2, t2 t3, t3 t4, t_new t_new), and [2][nv] the
@@ -210,6 +213,7 @@ struct StageIO {
   T* gd_v;
   T* pv_c;
   T* pv_e;
+  T* dfit;  // [2][ne] second derivatives of pv along the edge at its vertices (k_vert_fit)
   const double* ghs;
   // conservative APVM (pv_scheme 2): correction direction and the two
   // tangent fluxes of pv_edge and of the correction
@@ -262,6 +266,7 @@ struct StageIO {
     s.gd_v = off(gd_v, v);
     s.pv_c = off(pv_c, c);
     s.pv_e = off(pv_e, e);
+    s.dfit = off(dfit, 2 * e);
     s.ghs = off(ghs, c);
     s.dpv = off(dpv, e);
     s.pvf = off(pvf, e);

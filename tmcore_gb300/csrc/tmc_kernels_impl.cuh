@@ -107,6 +107,13 @@ constexpr bool kProducts = !kF64<T> && EPT == 1;
 
 // metric in the arithmetic type: FP64 array in FP64 mode, FP32 copy otherwise
 template <class T>
+__device__ __forceinline__ const T* met_p(const double* d, const float* f) {
+  if constexpr (kF64<T>)
+    return d;
+  else
+    return f;
+}
+template <class T>
 __device__ __forceinline__ T met(const double* d, const float* f, size_t i) {
   if constexpr (kF64<T>)
     return d[i];
@@ -280,14 +287,15 @@ template <class T>
 struct EdgeSet {
   T *gd_e, *u, *F, *Fq;
   double *sq, *hu, *ke, *ud;  // FP64 path
+  float* uf;                  // FP64 path with upwind pv: u in FP32
 };
 template <class T>
 __device__ __forceinline__ EdgeSet<T> edge_set(const StageIO<T>& S) {
-  return {S.gd_e, S.u, S.F, S.Fq, S.sq, S.hu, S.ke, S.ud};
+  return {S.gd_e, S.u, S.F, S.Fq, S.sq, S.hu, S.ke, S.ud, S.uf};
 }
 template <class T>
 __device__ __forceinline__ EdgeSet<T> next_edge_set(const StageIO<T>& S) {
-  return {S.gd_e_nx, S.u_nx, S.F_nx, S.Fq_nx, S.sq_nx, S.hu_nx, S.ke_nx, S.ud_nx};
+  return {S.gd_e_nx, S.u_nx, S.F_nx, S.Fq_nx, S.sq_nx, S.hu_nx, S.ke_nx, S.ud_nx, S.uf_nx};
 }
 
 // Edge preparation of one edge (operators_mod.F90:93-104 c2e, :423-472 upwind
@@ -328,6 +336,7 @@ __device__ __forceinline__ void prep_edge(const DevMesh& M, const ModelOpt& O, i
     X.hu[e] = f64::div_r(f64::half(uu), sq.s, sq.r);
     X.ke[e] = uu * uu * ae;
     X.ud[e] = uu * dc;
+    if (X.uf) X.uf[e] = (float)uu;
     for (int k = 0; k < O.n_tracers; ++k) {
       double qe;
       if (C.ratio) {
@@ -832,71 +841,114 @@ __global__ void __launch_bounds__(kMaxBlock) k_edge_pv(DevMesh M, ModelOpt O, St
   }
 }
 
-// FP32 upwind pv on edges (pv_scheme 3, interp_pv_order 3 or 4;
-// operators_mod.F90:359-412, the tangential velocity :223-237): one edge per
-// thread.  The two-sided vertex fit stencils come as packed (index, FP32
-// weight) entries, one 8-byte load each, and every load of the edge is issued
-// up front: the tangential-velocity gathers over a fixed 10 slots (padded
-// slots are the edge itself with weight 0) and the stencil points up to the
-// width with the side's count as a predicate, so an edge's ~35 gathers are in
-// flight together instead of a count-dependent chain.  Sums in stencil order.
-// Resident 256-thread blocks per SM the kernel is compiled for.  It is
-// latency bound (two dependent loads per stencil point): at level 8 the pass
-// takes 0.295 ms with 2 (128 registers), 0.183 ms with 3 (80) and 0.171 ms
-// with 4 (64 registers, about 100 bytes spilled to L1).
-#ifndef TMC_UP32_MINB
-#define TMC_UP32_MINB 4
-#endif
-template <bool kB>
-__global__ void __launch_bounds__(256, TMC_UP32_MINB) k_edge_pv_up32(DevMesh M, ModelOpt O, StageIO<float> S0) {
-  const StageIO<float> S = kB ? S0.at(blockIdx.y) : S0;
+// Upwind pv on edges (pv_scheme 3, interp_pv_order 3 or 4;
+// operators_mod.F90:359-412) in two passes.  The three edges of a vertex share
+// the vertex's fit points and differ in their weights only, so k_vert_fit
+// gathers the points once per vertex and sums the three second derivatives,
+// each into its edge's side; k_edge_up adds the two sides.  Per edge that is 8
+// gathers, 8 point indices and 12 differences in place of 24 each, on which
+// the pass per edge was latency bound.  Us per step, pass per edge -> these:
+// level 6 FP32 87 -> 72, FP64 305 -> 275; level 8 FP32 1115 -> 727 (the two
+// passes 174 -> 88), FP64 3622 -> 3117.  Sums in stencil order.
+// A point's index and its three weights are one 16-byte record in FP32 (as
+// separate loads, 12 points at a time: 128 registers and 112 us for
+// k_vert_fit alone at level 8).  Points in flight x resident blocks, level 8,
+// both passes: 6 x 4 87.8 us, 4 x 6 87.3, 12 x 3 91.5; FP64 2 to 6 alike.
+template <class T, bool kB>
+__global__ void __launch_bounds__(256, kF64<T> ? 1 : 4) k_vert_fit(DevMesh M, StageIO<T> S0) {
+  constexpr int kU = kF64<T> ? 4 : 6;  // points whose loads are in flight together
+  const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
+  const int v = blockIdx.x * blockDim.x + threadIdx.x, nv = M.nv;
+  if (v >= nv) return;
+  const int n = __ldg(M.vfit_n + v);
+  const T fc = __ldg(S.pv_v + v);
+  T acc[3] = {T(0), T(0), T(0)};
+  for (int j0 = 0; j0 < n; j0 += kU) {
+    int ix[kU];
+    T w[3][kU], f[kU];
+#pragma unroll
+    for (int j = 0; j < kU; ++j) {
+      const int q = min(j0 + j, n - 1);
+      if constexpr (kF64<T>) {
+        ix[j] = __ldg(M.vfit_idx + (size_t)q * nv + v);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) w[k][j] = __ldg(M.vfit_w + ((size_t)q * 3 + k) * nv + v);
+      } else {
+        const float4 r = __ldg(M.vfit_rec + (size_t)q * nv + v);
+        w[0][j] = r.x;
+        w[1][j] = r.y;
+        w[2][j] = r.z;
+        ix[j] = __float_as_int(r.w);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kU; ++j) f[j] = __ldg(S.pv_v + ix[j]);
+#pragma unroll
+    for (int j = 0; j < kU; ++j)
+      if (j0 + j < n) {
+        const T d = f[j] - fc;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) acc[k] = acc[k] + w[k][j] * d;
+      }
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int e = __ldg(M.edgesOnVertex + (size_t)k * nv + v);
+    const bool first = __ldg(M.tSign + (size_t)k * nv + v) > 0;  // v is the edge's first vertex
+    S.dfit[(first ? (size_t)0 : (size_t)M.ne) + e] = acc[k];
+  }
+}
+
+// The sign of the tangential velocity (:223-237) picks the upwind side.  FP64:
+// it is decided by an FP32 sum wherever that exceeds the sum's error bound (12
+// terms of 2^-24 of the magnitudes; the test asks for 32), else by the FP64
+// sum in the reference order: 20 FP64 instructions per edge less.
+template <class T>
+__device__ __forceinline__ T upwind_sign(const DevMesh& M, const StageIO<T>& S, int e) {
+  const int ne = M.ne;
+  if constexpr (kF64<T>) {
+    const int n = M.nEdgesOnEdge[e];
+    float s = 0.f, a = 0.f;
+#pragma unroll 5
+    for (int i = 0; i < n; ++i) {
+      const float t = __fmul_rn(__ldg(S.uf + __ldg(M.edgesOnEdge + (size_t)i * ne + e)),
+                                __ldg(M.weightsOnEdge_f + (size_t)i * ne + e));
+      s = __fadd_rn(s, t);
+      a = __fadd_rn(a, fabsf(t));
+    }
+    if (fabsf(s) > a * 0x1p-19f && a > 1e-25f && a < 1e30f) return s < 0.f ? -1.0 : 1.0;
+    double ve = 0.0;
+    for (int i = 0; i < n; ++i) {
+      const size_t k = (size_t)i * ne + e;
+      ve = ve + S.u[M.edgesOnEdge[k]] * M.weightsOnEdge[k];
+    }
+    return sgn1(ve);
+  } else {
+    int eo[kME2];
+    float wo[kME2], uo[kME2], ve = 0.f;
+#pragma unroll
+    for (int i = 0; i < kME2; ++i) {
+      eo[i] = __ldg(M.edgesOnEdge + (size_t)i * ne + e);  // padded slots: the edge itself, weight 0
+      wo[i] = __ldg(M.weightsOnEdge_f + (size_t)i * ne + e);
+    }
+#pragma unroll
+    for (int i = 0; i < kME2; ++i) uo[i] = __ldg(S.u + eo[i]);
+#pragma unroll
+    for (int i = 0; i < kME2; ++i) ve = ve + uo[i] * wo[i];
+    return sgn1(ve);
+  }
+}
+template <class T, bool kB>
+__global__ void __launch_bounds__(256) k_edge_up(DevMesh M, ModelOpt O, StageIO<T> S0) {
+  const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= M.ne) return;
-  const int ne = M.ne, W = M.vert2.width;
-  const int v1 = __ldg(M.verticesOnEdge + e), v2 = __ldg(M.verticesOnEdge + ne + e);
-  const int n0 = __ldg(M.vert2.count + e), n1 = __ldg(M.vert2.count + ne + e);
-  int eo[kME2];
-  float wo[kME2];
-#pragma unroll
-  for (int i = 0; i < kME2; ++i) {
-    eo[i] = __ldg(M.edgesOnEdge + (size_t)i * ne + e);
-    wo[i] = __ldg(M.weightsOnEdge_f + (size_t)i * ne + e);
-  }
-  const int m0 = min(n0, W), m1 = min(n1, W);
-  int2 iw[2][kUpW32];
-#pragma unroll
-  for (int j = 0; j < kUpW32; ++j) {
-    iw[0][j] = j < m0 ? __ldg(M.vert2_iw + ((size_t)j * 2 + 0) * ne + e) : make_int2(0, 0);
-    iw[1][j] = j < m1 ? __ldg(M.vert2_iw + ((size_t)j * 2 + 1) * ne + e) : make_int2(0, 0);
-  }
-  const float p1 = __ldg(S.pv_v + v1), p2 = __ldg(S.pv_v + v2);
-  float uo[kME2];
-#pragma unroll
-  for (int i = 0; i < kME2; ++i) uo[i] = __ldg(S.u + eo[i]);
-  float f[2][kUpW32];
-#pragma unroll
-  for (int j = 0; j < kUpW32; ++j) {
-    f[0][j] = j < m0 ? __ldg(S.pv_v + iw[0][j].x) : 0.f;
-    f[1][j] = j < m1 ? __ldg(S.pv_v + iw[1][j].x) : 0.f;
-  }
-  float ve = 0.f;
-#pragma unroll
-  for (int i = 0; i < kME2; ++i) ve = ve + uo[i] * wo[i];
-  float d[2];
-#pragma unroll
-  for (int sd = 0; sd < 2; ++sd) {
-    const float fc = sd == 0 ? p1 : p2;
-    const int n = sd == 0 ? m0 : m1;
-    float acc = 0.f;
-#pragma unroll
-    for (int j = 0; j < kUpW32; ++j)
-      if (j < n) acc = acc + __int_as_float(iw[sd][j].y) * (f[sd][j] - fc);
-    d[sd] = acc;
-  }
-  const float dist = __ldg(M.dvEdge_f + e);
-  const float pe = 0.5f * (p1 + p2) -
-                   dist * dist * ((d[0] + d[1]) - sgn1(ve) * (float)O.vert_coef2 * (d[1] - d[0])) / 12.f;
-  S.pv_e[e] = pe;
+  const int v1 = __ldg(M.verticesOnEdge + e), v2 = __ldg(M.verticesOnEdge + M.ne + e);
+  const T d0 = __ldg(S.dfit + e), d1 = __ldg(S.dfit + M.ne + e);
+  const T dist = __ldg(met_p<T>(M.dvEdge, M.dvEdge_f) + e);
+  const T p1 = __ldg(S.pv_v + v1), p2 = __ldg(S.pv_v + v2);
+  const T sg = upwind_sign<T>(M, S, e);
+  S.pv_e[e] = halve(p1 + p2) - over12(dist * dist * ((d0 + d1) - sg * T(O.vert_coef2) * (d1 - d0)));
 }
 
 // ---------------------------------------------------------------------------
@@ -1723,16 +1775,19 @@ template <class T>
 void launch_edge_pv(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Blk b, cudaStream_t st) {
   if ((O.pv_scheme == 1 && O.apvm_weight != 0.0) || O.pv_scheme == 2 || O.need_pv_c)
     k_v2c<T, kEPT><<<dim3(grid_for(M.nc, b.bs), nmem(S)), b.bs, 0, st>>>(M, S.pv_v, S.pv_c, S.msv, S.msc);
-  if constexpr (!kF64<T>) {
-    if (O.pv_scheme == 3 && (O.interp_pv_order == 3 || O.interp_pv_order == 4) && M.vert2_iw) {
-      const int bs = b.bs < 256 ? b.bs : 256;  // compiled for at most 256 threads per block
-      const dim3 g(nblk(M.ne, bs), nmem(S));
-      if (S.members > 1)
-        k_edge_pv_up32<true><<<g, bs, 0, st>>>(M, O, S);
-      else
-        k_edge_pv_up32<false><<<g, bs, 0, st>>>(M, O, S);
-      return;
+  if (M.vfit_n) {
+    const int bs = b.bs < 256 ? b.bs : 256;
+    const dim3 gv(nblk(M.nv, bs), nmem(S)), ge(nblk(M.ne, bs), nmem(S));
+    if constexpr (!kF64<T>) {
+      if (S.members > 1) {
+        k_vert_fit<T, true><<<gv, bs, 0, st>>>(M, S);
+        k_edge_up<T, true><<<ge, bs, 0, st>>>(M, O, S);
+        return;
+      }
     }
+    k_vert_fit<T, false><<<gv, bs, 0, st>>>(M, S);
+    k_edge_up<T, false><<<ge, bs, 0, st>>>(M, O, S);
+    return;
   }
   TMC_LAUNCH(k_edge_pv, M.ne, M, O, S);
 }
