@@ -331,3 +331,36 @@ def test_ordering_autotuner(mesh4):
     best, timings = tune.autotune_ordering(mesh4, ics, steps=1, orders=(1,), dt=600.0, **kw)
     assert best["member_layout"] == 0
     assert [t["member_layout"] for t in timings if "error" in t] == [1] * nl
+
+
+def test_rows_beyond_4_gb_match_small_ensemble():
+    """64-bit row offsets (an edge array of 4.3 GB): members of a huge ensemble
+    evolve bit for bit as in one of 64 members, which has the same lanes, blocks
+    and partial sums and takes 32-bit offsets.  The members not set stay zero
+    (their NaN stays their own)."""
+    torch = pytest.importorskip("torch")
+    if torch.cuda.mem_get_info()[0] < 120e9:
+        pytest.skip("needs 120 GB of device memory")
+    from tmcore_gb300 import abi, cases, mesh
+    from tmcore_gb300.gpu import TMCoreGPU
+
+    m = mesh.icos_mesh(5)
+    M = 64 * 547
+    assert m.nEdges * M * 4 > 2 ** 32
+    kw = dict(dt=600.0, precision=abi.TMC_FP32, pv_scheme=1, apvm_weight=0.0, member_layout=1, diag_every=0)
+    ics = [cases.jet_bumps(m, seed=s) for s in range(3)]
+    out = []
+    for members, at in ((64, (0, 17, 63)), (M, (0, 64 * 300 + 17, M - 1))):
+        g = TMCoreGPU(m, members=members, **kw)
+        for k, ic in zip(at, ics):
+            g.select_member(k)
+            g.set_initial(*ic)
+        g.step(2)
+        res = []
+        for k in at:
+            g.select_member(k)
+            res.append(g.get_state()[:2])
+        out.append(res)
+        g.close()
+    for a, b in zip(*out):
+        assert all(np.array_equal(x, y) and np.all(np.isfinite(x)) for x, y in zip(a, b))

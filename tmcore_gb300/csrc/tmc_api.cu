@@ -794,7 +794,6 @@ struct EnsEngine : EngineBase {
   float* gd_acc = nullptr;  // FF
   double* ghs = nullptr;
   float *iap_acc = nullptr, *iap_tend = nullptr, *tendf = nullptr, *ghsf = nullptr;
-  float* gd_e[2] = {};
   float* u[2] = {};
   float* F[2] = {};
   float *E = nullptr, *pv_v = nullptr, *vor = nullptr, *gd_v = nullptr, *pv_e = nullptr;
@@ -827,7 +826,6 @@ struct EnsEngine : EngineBase {
     iap_acc = h->dalloc<float>(ne);
     iap_tend = h->dalloc<float>(ne);
     for (int i = 0; i < 2; ++i) {
-      gd_e[i] = h->dalloc<float>(ne);
       u[i] = h->dalloc<float>(ne);
       F[i] = h->dalloc<float>(ne);
     }
@@ -899,10 +897,8 @@ struct EnsEngine : EngineBase {
     s.iap_tend = iap_tend;
     s.tendf = tendf;
     s.ghsf = ghsf;
-    s.gd_e = gd_e[set];
     s.u = u[set];
     s.F = F[set];
-    s.gd_e_nx = fuse ? gd_e[1 - set] : nullptr;
     s.u_nx = fuse ? u[1 - set] : nullptr;
     s.F_nx = fuse ? F[1 - set] : nullptr;
     s.E = E;

@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <cstring>
+#include <type_traits>
 
 #include "tmc_ensemble.cuh"
 #include "tmc_fp64.cuh"
@@ -168,6 +169,15 @@ __device__ __forceinline__ void stv(double* p, size_t i, const double (&v)[V]) {
     p[i] = v[0];
 }
 
+// A row (one element's members) of an array by its byte offset.  With O =
+// uint32_t the load takes the array's base from a uniform register and the
+// offset from a 32-bit one; 64-bit row addresses cost two more integer
+// instructions per load, and the flux pass makes 35 loads per edge.
+template <int V, class O>
+__device__ __forceinline__ void ldo(const float* p, O off, float (&o)[V]) {
+  ldv<V>(reinterpret_cast<const float*>(reinterpret_cast<const char*>(p) + off), 0, o);
+}
+
 template <int V>
 __device__ __forceinline__ void ldff(const float* p, size_t i, size_t ffs, FF (&o)[V]) {
   float h[V], l[V];
@@ -211,6 +221,27 @@ inline dim3 grid_of(int n, const Dims& D, int bs, int* threads) {
   if (W > kMaxBS / 32) W = kMaxBS / 32;
   *threads = W * 32;
   return dim3((unsigned)slots_for(n), (unsigned)(D.M / (D.LPE * D.V)));
+}
+
+// 32-bit row offsets reach an array of up to 4 GB
+inline bool narrow_rows(int n, const Dims& D) { return (size_t)n * D.M * sizeof(float) < ((size_t)1 << 32); }
+// f with the stage (0: outside a step), or V and the row offset type, as constants
+template <class F>
+inline void on_stage(int stage, F&& f) {
+  switch (stage) {
+    case 0: f(std::integral_constant<int, 0>()); break;
+    case 1: f(std::integral_constant<int, 1>()); break;
+    case 2: f(std::integral_constant<int, 2>()); break;
+    case 3: f(std::integral_constant<int, 3>()); break;
+    default: f(std::integral_constant<int, 4>());
+  }
+}
+template <class F>
+inline void on_lanes(int V, bool narrow, F&& f) {
+  if (V == 2 && narrow) f(std::integral_constant<int, 2>(), uint32_t());
+  else if (V == 2) f(std::integral_constant<int, 2>(), size_t());
+  else if (narrow) f(std::integral_constant<int, 1>(), uint32_t());
+  else f(std::integral_constant<int, 1>(), size_t());
 }
 
 // Per-member partial sums of one block: the rows (warps and the element
@@ -277,20 +308,23 @@ __device__ __forceinline__ void block_partials_ff(const Lane& L, const FF (&v)[N
 
 // Edge preparation of one edge (operators_mod.F90:93-104 c2e, :168-176
 // inverse IAP; mass flux u gd_edge, tmcore_swm_mod.F90:135), the FP32
-// single-model arithmetic.
-__device__ __forceinline__ void prep1(float ia, float g1, float g2, float& ge, float& uu, float& Fv) {
-  ge = 0.5f * (g1 + g2);
+// single-model arithmetic.  gd_edge itself is not stored: the flux pass
+// averages the two cells' gd again, and the cell pass forms the mass flux from
+// u and the neighbours' gd (a third as many values as the edges' fluxes).  512
+// level-6 members, us per pass: flux 696 -> 662, cell 273 -> 268, final 326 ->
+// 297.
+__device__ __forceinline__ void prep1(float ia, float g1, float g2, float& uu, float& Fv) {
+  const float ge = 0.5f * (g1 + g2);
   const float sq = sqrtf(ge);
   uu = ia / sq;
   Fv = uu * ge;
 }
 template <int V>
-__device__ __forceinline__ void prep(const float (&ia)[V], const float (&g1)[V], const float (&g2)[V], float* gd_e,
-                                     float* u, float* F, size_t em) {
-  float ge[V], uu[V], Fv[V];
+__device__ __forceinline__ void prep(const float (&ia)[V], const float (&g1)[V], const float (&g2)[V], float* u,
+                                     float* F, size_t em) {
+  float uu[V], Fv[V];
 #pragma unroll
-  for (int c = 0; c < V; ++c) prep1(ia[c], g1[c], g2[c], ge[c], uu[c], Fv[c]);
-  stv<V>(gd_e, em, ge);
+  for (int c = 0; c < V; ++c) prep1(ia[c], g1[c], g2[c], uu[c], Fv[c]);
   stv<V>(u, em, uu);
   stv<V>(F, em, Fv);
 }
@@ -300,10 +334,11 @@ __device__ __forceinline__ void prep(const float (&ia)[V], const float (&g1)[V],
 // E = ke + gd + ghs, RK update of gd (div_operator operators_mod.F90:40-55,
 // calc_kinetic_energy :206-221, calc_gd_tend_on_cell tmcore_swm_mod.F90:127-139)
 // ---------------------------------------------------------------------------
-template <int V>
-__device__ __forceinline__ void ens_cell(const DevMesh& Mh, const Dims& D, const IO& S, const RKStage& rk,
+template <int V, class O, int mode>
+__device__ __forceinline__ void ens_cell(const DevMesh& Mh, const Dims& D, const IO& S, double a_dt,
                                          const Partials& P, int diag, int bx) {
-  __shared__ int s_e[kME][kEnsEPB];
+  __shared__ O s_e[kME][kEnsEPB];
+  __shared__ O s_nb[kME][kEnsEPB];
   __shared__ float s_ns[kME][kEnsEPB];
   __shared__ float s_dv[kME][kEnsEPB];
   __shared__ float s_ae[kME][kEnsEPB];
@@ -312,11 +347,13 @@ __device__ __forceinline__ void ens_cell(const DevMesh& Mh, const Dims& D, const
   __shared__ float s_invAf[kEnsEPB];
   __shared__ float s_Af[kEnsEPB];
   const int nc = Mh.nc, c0 = bx * kEnsEPB, nel = min(kEnsEPB, nc - c0);
+  const O row = (O)D.M * (O)sizeof(float);
   for (int t = threadIdx.x; t < kME * kEnsEPB; t += blockDim.x) {
     const int i = t / kEnsEPB, j = t - i * kEnsEPB;
     if (j < nel) {
       const size_t k = (size_t)i * nc + c0 + j;
-      s_e[i][j] = Mh.edgesOnCell[k];
+      s_e[i][j] = (O)Mh.edgesOnCell[k] * row;
+      s_nb[i][j] = (O)Mh.cellsOnCell[k] * row;
       s_ns[i][j] = (float)Mh.nSign[k];
       s_dv[i][j] = S.cdv[k];  // dvEdge and areaEdge of the cell's edges, gathered at set-up
       s_ae[i][j] = S.cae[k];
@@ -331,8 +368,8 @@ __device__ __forceinline__ void ens_cell(const DevMesh& Mh, const Dims& D, const
   __syncthreads();
   const Lane L = lane_of<V>(D);
   const size_t Mm = L.M, ffs = S.ffs;
-  const int mode = rk.mode;
-  const FF adt = ff_from(rk.a_dt), sixth = ff_from(1.0 / 6.0);
+  const O m0 = (O)L.m0 * (O)sizeof(float);
+  const FF adt = ff_from(a_dt), sixth = ff_from(1.0 / 6.0);
   float rip[V], r44[V], eh[V], el[V];
   FF mass[V];
 #pragma unroll
@@ -342,20 +379,20 @@ __device__ __forceinline__ void ens_cell(const DevMesh& Mh, const Dims& D, const
     FF gold[V], gacc[V];
     float tprev[V], gdf[V], ghf[V], gdl[V];
     if (mode >= 1 && mode <= 3) ldff<V>(S.gd_old, cm, ffs, gold);
-    if (mode >= 2) {
-      ldff<V>(S.gd_acc, cm, ffs, gacc);
-      ldv<V>(S.tendf, cm, tprev);
-    }
+    if (mode >= 2) ldff<V>(S.gd_acc, cm, ffs, gacc);
+    if (mode >= 3) ldv<V>(S.tendf, cm, tprev);
     ldv<V>(S.gd_in, cm, gdf);
     ldv<V>(S.ghsf, cm, ghf);
     if (diag) ldv<V>(S.gd_in + ffs, cm, gdl);
-    float uu[kME][V], Fv[kME][V];
+    float uu[kME][V], gn[kME][V];
 #pragma unroll
     for (int i = 0; i < kME; ++i) {
-      const size_t k = (size_t)s_e[i][j] * Mm + L.m0;
-      ldv<V>(S.u, k, uu[i]);
-      ldv<V>(S.F, k, Fv[i]);
+      ldo<V>(S.u, (O)(s_e[i][j] + m0), uu[i]);
+      ldo<V>(S.gd_in, (O)(s_nb[i][j] + m0), gn[i]);
     }
+    if (mode == 2)  // the accumulator after stage 1 is its tendency
+#pragma unroll
+      for (int c = 0; c < V; ++c) tprev[c] = gacc[c].h;
     FF acc_o[V], gnext[V];
     float Eo[V], tT[V];
 #pragma unroll
@@ -364,7 +401,8 @@ __device__ __forceinline__ void ens_cell(const DevMesh& Mh, const Dims& D, const
 #pragma unroll
       for (int i = 0; i < kME; ++i) {
         const float ns = s_ns[i][j];
-        two_sum_acc(hi, lo, __fmul_rn(__fmul_rn(ns, Fv[i][c]), s_dv[i][j]));
+        const float Fv = __fmul_rn(uu[i][c], __fmul_rn(0.5f, __fadd_rn(gdf[c], gn[i][c])));  // prep1
+        two_sum_acc(hi, lo, __fmul_rn(__fmul_rn(ns, Fv), s_dv[i][j]));
         k += fabsf(ns) * uu[i][c] * uu[i][c] * s_ae[i][j];
       }
       // gd tendency t = -(flux divergence) / areaCell
@@ -426,9 +464,9 @@ __device__ __forceinline__ void ens_cell(const DevMesh& Mh, const Dims& D, const
     block_partials_ff<2, V>(L, v, dst);
   }
 }
-template <int V>
-__global__ void TMC_ENS_LB(TMC_ENS_CELL_MINB) k_ens_cell(DevMesh Mh, Dims D, IO S, RKStage rk, Partials P, int diag) {
-  ens_cell<V>(Mh, D, S, rk, P, diag, blockIdx.x);
+template <int V, class O, int mode>
+__global__ void TMC_ENS_LB(TMC_ENS_CELL_MINB) k_ens_cell(DevMesh Mh, Dims D, IO S, double a_dt, Partials P, int diag) {
+  ens_cell<V, O, mode>(Mh, D, S, a_dt, P, diag, blockIdx.x);
 }
 
 // invariants of a state only (the diagnostic pass): mass and cell energy
@@ -694,78 +732,89 @@ __global__ void __launch_bounds__(kMaxBS) k_ens_edge_pv_up(DevMesh Mh, Dims D, I
 // and the CRK4 inner products (time_scheme_mod.F90:109-154); stages 1-3 also
 // prepare the next stage's gd_edge, u and F from its gd and iap_u.
 // ---------------------------------------------------------------------------
-template <int V>
-__device__ __forceinline__ void ens_edge_flux(const DevMesh& Mh, const Dims& D, const IO& S, const RKStage& rk,
+// The pass is bound by neither memory (DRAM 36%, L2 20%, L1 44% busy) but by
+// the overlap of its load and compute phases at 16 warps per SM, so what counts
+// is that a warp's loads leave in one go: with the stage a runtime value the
+// loads that depend on it sat behind branches (512 level-6 members 743 us per
+// launch, 16 level-7 members 134.8), as a constant they do not (696 and 114.6,
+// with 32-bit row offsets and without the tendency's store and load where the
+// accumulator holds it; 3 resident blocks, 80 registers, 801).
+template <int V, class O, int mode>
+__device__ __forceinline__ void ens_edge_flux(const DevMesh& Mh, const Dims& D, const IO& S, double a_dt,
                                               const Partials& P, int bx) {
-  __shared__ int s_ep[kME2][kEnsEPB];
-  __shared__ float s_w[kME2][kEnsEPB];
-  __shared__ int s_c[2][kEnsEPB];
-  __shared__ float s_dc[kEnsEPB];
-  __shared__ float s_ae[kEnsEPB];
+  // an edge's stencil: per neighbour {row byte offset, weight}, the cells'
+  // row offsets, dcEdge and areaEdge
+  struct Nb {
+    O off;
+    float w;
+  };
+  __shared__ Nb s_n[kME2][kEnsEPB];
+  __shared__ O s_c[2][kEnsEPB];
+  __shared__ float2 s_m[kEnsEPB];
   const int ne = Mh.ne, e0 = bx * kEnsEPB, nel = min(kEnsEPB, ne - e0);
+  const O row = (O)D.M * (O)sizeof(float);
   for (int t = threadIdx.x; t < kME2 * kEnsEPB; t += blockDim.x) {
     const int i = t / kEnsEPB, j = t - i * kEnsEPB;
     if (j < nel) {
       const size_t k = (size_t)i * ne + e0 + j;
-      s_ep[i][j] = Mh.edgesOnEdge[k];  // padded entries: the edge itself, weight 0
-      s_w[i][j] = Mh.weightsOnEdge_f[k];
+      s_n[i][j] = Nb{(O)Mh.edgesOnEdge[k] * row, Mh.weightsOnEdge_f[k]};  // padded entries: the edge itself, weight 0
     }
   }
   for (int t = threadIdx.x; t < 2 * kEnsEPB; t += blockDim.x) {
     const int i = t / kEnsEPB, j = t - i * kEnsEPB;
-    if (j < nel) s_c[i][j] = Mh.cellsOnEdge[(size_t)i * ne + e0 + j];
+    if (j < nel) s_c[i][j] = (O)Mh.cellsOnEdge[(size_t)i * ne + e0 + j] * row;
   }
-  for (int j = threadIdx.x; j < nel; j += blockDim.x) {
-    s_dc[j] = Mh.dcEdge_f[e0 + j];
-    s_ae[j] = Mh.areaEdge_f[e0 + j];
-  }
+  for (int j = threadIdx.x; j < nel; j += blockDim.x)
+    s_m[j] = make_float2(Mh.dcEdge_f[e0 + j], Mh.areaEdge_f[e0 + j]);
   __syncthreads();
   const Lane L = lane_of<V>(D);
-  const size_t Mm = L.M;
-  const int mode = rk.mode;
-  const bool fuse = S.u_nx != nullptr;
-  const float adt = (float)rk.a_dt;
+  static_assert(mode >= 0 && mode <= 4, "stage");
+  constexpr bool fuse = mode >= 1 && mode <= 3;  // stages 1-3 prepare the next stage's edge set
+  const float adt = (float)a_dt;
+  const O m0 = (O)L.m0 * (O)sizeof(float);
   float rip[V], r44[V];
 #pragma unroll
   for (int c = 0; c < V; ++c) rip[c] = r44[c] = 0.f;
   for (int j = L.j0; j < nel; j += L.js) {
-    const size_t em = (size_t)(e0 + j) * Mm + L.m0;
-    const size_t c1m = (size_t)s_c[0][j] * Mm + L.m0, c2m = (size_t)s_c[1][j] * Mm + L.m0;
-    float pe[V], uu[V], ge[V], tp[V], accv[V], oldv[V], gn1[V], gn2[V], E1[V], E2[V], t1[V], t2[V];
-    ldv<V>(S.pv_e, em, pe);
-    ldv<V>(S.u, em, uu);
-    ldv<V>(S.gd_e, em, ge);
+    const O eo = (O)(e0 + j) * row + m0, c1o = s_c[0][j] + m0, c2o = s_c[1][j] + m0;
+    float pe[V], uu[V], gi1[V], gi2[V], tp[V], accv[V], oldv[V], gn1[V], gn2[V], E1[V], E2[V], t1[V], t2[V];
+    ldo<V>(S.pv_e, eo, pe);
+    ldo<V>(S.u, eo, uu);
+    ldo<V>(S.gd_in, c1o, gi1);
+    ldo<V>(S.gd_in, c2o, gi2);
     if (mode >= 2) {
-      ldv<V>(S.iap_tend, em, tp);
-      ldv<V>(S.iap_acc, em, accv);
+      if (mode >= 3) ldo<V>(S.iap_tend, eo, tp);
+      ldo<V>(S.iap_acc, eo, accv);
     }
-    if (mode >= 1 && mode <= 3) ldv<V>(S.iap_old, em, oldv);
     if (fuse) {
-      ldv<V>(S.gd_next, c1m, gn1);  // h halves: the FP32 gd of the next stage
-      ldv<V>(S.gd_next, c2m, gn2);
+      ldo<V>(S.iap_old, eo, oldv);
+      ldo<V>(S.gd_next, c1o, gn1);  // h halves: the FP32 gd of the next stage
+      ldo<V>(S.gd_next, c2o, gn2);
     }
-    ldv<V>(S.E, c1m, E1);
-    ldv<V>(S.E, c2m, E2);
-    ldv<V>(S.tendf, c1m, t1);
-    ldv<V>(S.tendf, c2m, t2);
-    float Fv[kME2][V], pp[kME2][V];
+    ldo<V>(S.E, c1o, E1);
+    ldo<V>(S.E, c2o, E2);
+    ldo<V>(S.tendf, c1o, t1);
+    ldo<V>(S.tendf, c2o, t2);
+    float w[kME2], Fv[kME2][V], pp[kME2][V];
 #pragma unroll
     for (int i = 0; i < kME2; ++i) {
-      const size_t k = (size_t)s_ep[i][j] * Mm + L.m0;
-      ldv<V>(S.F, k, Fv[i]);
-      ldv<V>(S.pv_e, k, pp[i]);
+      const Nb q = s_n[i][j];
+      w[i] = q.w;
+      ldo<V>(S.F, (O)(q.off + m0), Fv[i]);
+      ldo<V>(S.pv_e, (O)(q.off + m0), pp[i]);
     }
-    const float dc = s_dc[j], ae = s_ae[j];
+    const float dc = s_m[j].x, ae = s_m[j].y;
+    const size_t em = (size_t)eo / sizeof(float);
     float acc_o[V], it_o[V], inext[V];
 #pragma unroll
     for (int c = 0; c < V; ++c) {
       float s = 0.f;
 #pragma unroll
-      for (int i = 0; i < kME2; ++i) s += s_w[i][j] * Fv[i][c] * (0.5f * (pe[c] + pp[i][c]));
+      for (int i = 0; i < kME2; ++i) s += w[i] * Fv[i][c] * (0.5f * (pe[c] + pp[i][c]));
       const float dEdx = (E2[c] - E1[c]) / dc;
       const float tge = 0.5f * (t1[c] + t2[c]);
       const float ut = s - dEdx;
-      const float sq = sqrtf(ge[c]);
+      const float sq = sqrtf(0.5f * (gi1[c] + gi2[c]));  // gd_edge of prep1
       const float it = sq * ut + 0.5f * uu[c] / sq * tge;
       it_o[c] = it;
       inext[c] = 0.f;
@@ -776,7 +825,8 @@ __device__ __forceinline__ void ens_edge_flux(const DevMesh& Mh, const Dims& D, 
           break;
         case 2:
         case 3:
-          rip[c] = rip[c] + tp[c] * it * ae;
+          // the accumulator after stage 1 is its tendency
+          rip[c] = rip[c] + (mode == 2 ? accv[c] : tp[c]) * it * ae;
           acc_o[c] = accv[c] + 2.f * it;
           inext[c] = oldv[c] + adt * it;
           break;
@@ -789,11 +839,9 @@ __device__ __forceinline__ void ens_edge_flux(const DevMesh& Mh, const Dims& D, 
       }
     }
     stv<V>(S.iap_acc, em, acc_o);
-    stv<V>(S.iap_tend, em, it_o);
+    if (mode == 2 || mode == 3) stv<V>(S.iap_tend, em, it_o);  // the next stage's t_prev
     if (fuse)
-      prep<V>(inext, gn1, gn2, S.gd_e_nx, S.u_nx, S.F_nx, em);
-    else if (mode <= 3)
-      stv<V>(S.iap_next, em, inext);
+      prep<V>(inext, gn1, gn2, S.u_nx, S.F_nx, em);
   }
   if (mode >= 2) {
     float v[2][V];
@@ -803,12 +851,11 @@ __device__ __forceinline__ void ens_edge_flux(const DevMesh& Mh, const Dims& D, 
     block_partials_f<2, V>(L, v, dst);
   }
 }
-template <int V>
+template <int V, class O, int mode>
 __global__ void __launch_bounds__(256, V == 1 ? TMC_ENS_MINB_V1 : TMC_ENS_FLUX_MINB)
-    k_ens_edge_flux(DevMesh Mh, Dims D, IO S, RKStage rk, Partials P) {
-  ens_edge_flux<V>(Mh, D, S, rk, P, blockIdx.x);
+    k_ens_edge_flux(DevMesh Mh, Dims D, IO S, double a_dt, Partials P) {
+  ens_edge_flux<V, O, mode>(Mh, D, S, a_dt, P, blockIdx.x);
 }
-
 // ---------------------------------------------------------------------------
 // final update new = old + (beta dt) t_new (update_state, tmcore_swm_mod.F90:203-213),
 // in place in state(old), with beta per member
@@ -895,8 +942,7 @@ __device__ __forceinline__ void ens_edges(const DevMesh& Mh, const Dims& D, cons
         for (int c = 0; c < V; ++c) ia[q][c] = ia[q][c] + bdt[c] * ac[q][c];
         stv<V>(iap, em, ia[q]);
       }
-      prep<V>(ia[q], g1[q], g2[q], const_cast<float*>(S.gd_e), const_cast<float*>(S.u), const_cast<float*>(S.F),
-              em);
+      prep<V>(ia[q], g1[q], g2[q], const_cast<float*>(S.u), const_cast<float*>(S.F), em);
       if (want_energy)
 #pragma unroll
         for (int c = 0; c < V; ++c) two_sum_acc(eh[c], el[c], ia[q][c] * ia[q][c] * s_ae[j]);
@@ -1125,12 +1171,12 @@ __device__ __forceinline__ void on_job(const StageTable& T, int j, F&& f) {
   }
 }
 
-template <int V>
-__global__ void TMC_ENS_LB(TMC_ENS_CELL_MINB) k_jobs_cell(const __grid_constant__ StageTable T, int nj, int stage) {
+template <int V, class O, int stage>
+__global__ void TMC_ENS_LB(TMC_ENS_CELL_MINB) k_jobs_cell(const __grid_constant__ StageTable T, int nj) {
   int j;
   const int bx = job_of(T.off, J_CELLS, nj, &j);
   on_job(T, j, [&](const JobStage& J) {
-    ens_cell<V>(J.Mh, J.D, J.io, RKStage{stage, stage_adt(stage, J.dt)}, J.P, 0, bx);
+    ens_cell<V, O, stage>(J.Mh, J.D, J.io, stage_adt(stage, J.dt), J.P, 0, bx);
   });
 }
 template <int V>
@@ -1151,13 +1197,12 @@ __global__ void __launch_bounds__(kMaxBS) k_jobs_edge_pv_up(const __grid_constan
   const int bx = job_of(T.off, J_EDGES_UP, nj, &j);
   on_job(T, j, [&](const JobStage& J) { ens_edge_pv_up<V>(J.Mh, J.D, J.io, J.up, bx); });
 }
-template <int V>
-__global__ void TMC_ENS_LB(TMC_ENS_FLUX_MINB) k_jobs_edge_flux(const __grid_constant__ StageTable T, int nj,
-                                                               int stage) {
+template <int V, class O, int stage>
+__global__ void TMC_ENS_LB(TMC_ENS_FLUX_MINB) k_jobs_edge_flux(const __grid_constant__ StageTable T, int nj) {
   int j;
   const int bx = job_of(T.off, J_EDGES, nj, &j);
   on_job(T, j, [&](const JobStage& J) {
-    ens_edge_flux<V>(J.Mh, J.D, J.io, RKStage{stage, stage_adt(stage, J.dt)}, J.P, bx);
+    ens_edge_flux<V, O, stage>(J.Mh, J.D, J.io, stage_adt(stage, J.dt), J.P, bx);
   });
 }
 template <int V>
@@ -1199,10 +1244,11 @@ void launch_cell(const DevMesh& Mh, const Dims& D, const IO& S, RKStage rk, cons
                  cudaStream_t st) {
   int th;
   const dim3 g = grid_of(Mh.nc, D, bs, &th);
-  if (D.V == 2)
-    k_ens_cell<2><<<g, th, 0, st>>>(Mh, D, S, rk, P, diag ? 1 : 0);
-  else
-    k_ens_cell<1><<<g, th, 0, st>>>(Mh, D, S, rk, P, diag ? 1 : 0);
+  on_lanes(D.V, narrow_rows(Mh.ne, D), [&](auto V, auto off) {
+    on_stage(rk.mode, [&](auto mode) {
+      k_ens_cell<V.value, decltype(off), mode.value><<<g, th, 0, st>>>(Mh, D, S, rk.a_dt, P, diag ? 1 : 0);
+    });
+  });
 }
 void launch_cell_diag(const DevMesh& Mh, const Dims& D, const IO& S, const Partials& P, int bs, cudaStream_t st) {
   int th;
@@ -1245,10 +1291,11 @@ void launch_edge_flux(const DevMesh& Mh, const Dims& D, const IO& S, RKStage rk,
                       cudaStream_t st) {
   int th;
   const dim3 g = grid_of(Mh.ne, D, bs, &th);
-  if (D.V == 2)
-    k_ens_edge_flux<2><<<g, th, 0, st>>>(Mh, D, S, rk, P);
-  else
-    k_ens_edge_flux<1><<<g, th, 0, st>>>(Mh, D, S, rk, P);
+  on_lanes(D.V, narrow_rows(Mh.ne, D), [&](auto V, auto off) {
+    on_stage(rk.mode, [&](auto mode) {
+      k_ens_edge_flux<V.value, decltype(off), mode.value><<<g, th, 0, st>>>(Mh, D, S, rk.a_dt, P);
+    });
+  });
 }
 void launch_final(const DevMesh& Mh, const Dims& D, const IO& S, const double* diag, const Partials& P, int bs,
                   cudaStream_t st) {
@@ -1367,6 +1414,8 @@ void launch_jobs_step(const JobTable& T, int nj, const int* bsp, bool upwind, cu
       gv((unsigned)T.off[J_VERTS][nj], gy), gu((unsigned)T.off[J_EDGES_UP][nj], gy);
   const bool up4 = upwind && D.LPE == 32 && D.M % 128 == 0 && TMC_ENS_UP_V == 4;
   const bool branch = side && fork && join;
+  bool narrow = true;
+  for (int j = 0; j < nj; ++j) narrow = narrow && narrow_rows(T.job[j].Mh.ne, T.job[j].D);
   const cudaStream_t sv = branch ? side : st;
   for (int k = 1; k <= 4; ++k) {
     const StageTable S = stage_table(T, nj, k);
@@ -1374,13 +1423,15 @@ void launch_jobs_step(const JobTable& T, int nj, const int* bsp, bool upwind, cu
       cudaEventRecord(fork, st);
       cudaStreamWaitEvent(side, fork, 0);
     }
-    if (D.V == 2) {
-      k_jobs_cell<2><<<gc, th[0], 0, st>>>(S, nj, k);
+    on_lanes(D.V, narrow, [&](auto V, auto off) {
+      on_stage(k, [&](auto stage) {
+        k_jobs_cell<V.value, decltype(off), stage.value><<<gc, th[0], 0, st>>>(S, nj);
+      });
+    });
+    if (D.V == 2)
       k_jobs_vertex<2><<<gv, th[1], 0, sv>>>(S, nj);
-    } else {
-      k_jobs_cell<1><<<gc, th[0], 0, st>>>(S, nj, k);
+    else
       k_jobs_vertex<1><<<gv, th[1], 0, sv>>>(S, nj);
-    }
     if (up4)
       k_jobs_edge_pv_up<4><<<dim3(gu.x, (unsigned)(D.M / 128)), th[2], 0, sv>>>(S, nj);
     else if (upwind && D.V == 2)
@@ -1395,10 +1446,11 @@ void launch_jobs_step(const JobTable& T, int nj, const int* bsp, bool upwind, cu
       cudaEventRecord(join, side);
       cudaStreamWaitEvent(st, join, 0);
     }
-    if (D.V == 2)
-      k_jobs_edge_flux<2><<<ge, th[3], 0, st>>>(S, nj, k);
-    else
-      k_jobs_edge_flux<1><<<ge, th[3], 0, st>>>(S, nj, k);
+    on_lanes(D.V, narrow, [&](auto V, auto off) {
+      on_stage(k, [&](auto stage) {
+        k_jobs_edge_flux<V.value, decltype(off), stage.value><<<ge, th[3], 0, st>>>(S, nj);
+      });
+    });
   }
   StepRegions R{};
   for (int k = 0; k < 3; ++k) {

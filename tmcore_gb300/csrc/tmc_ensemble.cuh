@@ -97,11 +97,9 @@ struct IO {
   float* iap_tend;
   float* tendf;
   const float* ghsf;
-  const float* gd_e;
   const float* u;
   const float* F;
-  float* gd_e_nx;  // the next stage's edge set (stages 1-3), null: not fused
-  float* u_nx;
+  float* u_nx;  // the next stage's edge set (stages 1-3)
   float* F_nx;
   float* E;
   float* pv_v;
@@ -146,7 +144,7 @@ void launch_edge_flux(const DevMesh& Mh, const Dims& D, const IO& S, RKStage rk,
 // of the next step's first stage and the edge energy of the new state
 void launch_final(const DevMesh& Mh, const Dims& D, const IO& S, const double* diag, const Partials& P, int bs,
                   cudaStream_t st);
-// edge preparation of slot S.gd_in / S.iap_in into S.gd_e/u/F (+ edge energy)
+// edge preparation of slot S.gd_in / S.iap_in into S.u/F (+ edge energy)
 void launch_edge_prep(const DevMesh& Mh, const Dims& D, const IO& S, const Partials& P, bool diag, int bs,
                       cudaStream_t st);
 // mass and the cell part of the energy of S.gd_in (the diagnostic pass)

@@ -166,7 +166,6 @@ struct EnsClosureSrc {
     const float pc1 = pv_c[c1 * W + m], pc2 = pv_c[c2 * W + m];
     x[0] = S.u[i];
     x[1] = ve;
-    x[2] = S.gd_e[i];
     x[3] = S.pv_e[i];
     x[4] = pv1;
     x[5] = pv2;
@@ -174,6 +173,7 @@ struct EnsClosureSrc {
     x[7] = pc2;
     x[8] = S.gd_in[c1 * W + m];  // h halves: the FP32 gd
     x[9] = S.gd_in[c2 * W + m];
+    x[2] = 0.5f * (x[8] + x[9]);  // gd_edge
     x[10] = S.E[c1 * W + m];
     x[11] = S.E[c2 * W + m];
     x[12] = S.ghsf[c1 * W + m];
