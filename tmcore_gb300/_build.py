@@ -59,6 +59,7 @@ GPU_SOURCES = [
     ("tmc_api.cu", "nvcc", []),
     ("tmc_kernels_f64.cu", "nvcc", ["-fmad=false"]),
     ("tmc_kernels_f32.cu", "nvcc", []),
+    ("tmc_kernels_f32_cell.cu", "nvcc", []),
     ("tmc_noalloc.cu", "nvcc", []),
     ("tmc_ensemble.cu", "nvcc", []),
     ("tmc_mlp.cu", "nvcc", []),

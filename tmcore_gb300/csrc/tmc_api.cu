@@ -251,7 +251,9 @@ struct Engine : EngineBase {
     iap_acc = h->dalloc<T>(ne);
     iap_tend = h->dalloc<T>(ne);
     for (int i = 0; i < 2; ++i) {
-      gd_e[i] = h->dalloc<T>(ne);
+      // second-order FP32 models average gd_edge where they use it
+      const bool plain = h->O.adv_order == 2 && h->O.pv_scheme != 2 && !h->O.flux4;
+      if (std::is_same<T, double>::value || !plain) gd_e[i] = h->dalloc<T>(ne);
       u[i] = h->dalloc<T>(ne);
       F[i] = h->dalloc<T>(ne);
       Fq[i] = h->dalloc<T>(nfq);
@@ -1101,7 +1103,8 @@ void set_counts(tmc_handle* h) {
 // Measured per step, four -> one: level 5 FP64 227 -> 89 us, FP32 74 -> 47;
 // level 6 FP64 with upwind pv 475 -> 300, FP32 103 -> 84.  The lines, us per
 // pass, four / one:
-//   FP64 flux      491k edges 115.6 / 96.2, 1.97M 342.9 / 344.7 (final, upwind pv alike)
+//   FP64 flux      491k edges 115.6 / 96.2, 1.97M 342.9 / 344.7
+//   FP64 final     491k 47.3 / 41.2, 1.97M 128.4 / 127.4, with four tracers 229.6 / 218.6
 //   FP64 cell      655k cells, four tracers 182.5 / 139.4
 //   FP64 vertex    328k 28.9 / 25.4, 1.31M 71.0 / 73.6
 //   FP32 flux      123k edges 10.5 / 8.8, 491k 18.8 / 21.5 (final alike)
@@ -1121,7 +1124,8 @@ void choose_launch_shapes(tmc_handle* h, bool default_blocks) {
   line[P_CELL] = f64 ? big : small;
   line[P_VERTEX] = f64 ? big : small;
   line[P_PV] = h->M.vfit_n ? big : small;  // (k_vert_fit, k_edge_up: always one, the line sets their blocks)
-  line[P_FLUX] = line[P_FINAL] = f64 ? big : small;
+  line[P_FLUX] = f64 ? big : small;
+  line[P_FINAL] = f64 ? 0x7fffffff : small;
   for (int k = 0; k < P_COUNT; ++k) {
     if (n[k] >= line[k]) continue;
     h->ept[k] = 1;

@@ -186,7 +186,7 @@ struct StageIO {
   float* tendf;        // gd tendency of the stage (read as t_prev before overwrite)
   const float* ghsf;
   // intermediates
-  T* gd_e;
+  T* gd_e;  // FP32: null in second-order models (edge_flux_body)
   T* u;
   T* F;   // u * gd_e (FP64 path: times dvEdge)
   T* Fq;  // [ntr][ne] (FP64 path: every order, times dvEdge)

@@ -9,6 +9,7 @@
 namespace tmc {
 
 TMC_INSTANTIATE(double)
+TMC_INSTANTIATE_CELL(double)
 
 struct FinalizeArgs {
   int counts[R_COUNT];

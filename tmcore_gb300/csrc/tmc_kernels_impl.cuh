@@ -364,7 +364,7 @@ __device__ __forceinline__ void prep_edge(const DevMesh& M, const ModelOpt& O, i
     const T sq = sqrt(ge);
     const T uu = ia / sq;
     const T Fv = uu * ge;
-    X.gd_e[e] = ge;
+    if (X.gd_e) X.gd_e[e] = ge;
     X.u[e] = uu;
     X.F[e] = Fv;
     // second-order tracers are fluxed by k_cell directly (no per-edge flux stored)
@@ -1181,13 +1181,23 @@ void launch_combine(const DevMesh& M, int ntr, int scheme, const CombineArgs<T>&
 // ---------------------------------------------------------------------------
 // edge_flux: q.F_perp, gradient of E, iap_u tendency, RK update, inner products
 // ---------------------------------------------------------------------------
-template <class T, bool kB, int EPT>
+// kMode: the stage of a second-order model (adv_order 2, no
+// flux_4th_order_correct) as a constant, or kGeneral for the others with the
+// stage at run time.  As a constant it takes the branches out from between a
+// thread's loads; FP32 also averages gd_edge again instead of loading it (the
+// edge preparation does not store it), and the tendencies of stages 1 and 4
+// are not stored: stage 1's is the accumulator, stage 4's is not read.  Level
+// 9, four tracers, us per pass: flux 201.7 -> 189.9, cell 134.7 -> 124.5
+// (cell_fast_body), final 107.7 -> 98.5.
+constexpr int kGeneral = -1;
+template <class T, bool kB, int EPT, int kMode>
 __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S0, RKStage rk,
                                                const Partials& P0) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
   T rip = T(0), r44 = T(0);  // FP32 path: FP32 products and per-thread sums, FP64 across warps
-  const int mode = rk.mode;
+  constexpr bool kPlain = kMode != kGeneral;
+  const int mode = kPlain ? kMode : rk.mode;
   TMC_FOR_N(EPT, e, M.ne) {
     // Loads that depend on no other load come first, before any store: a load
     // issued after a store through a pointer the compiler must assume aliases
@@ -1198,17 +1208,21 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
     if constexpr (kF64<T>) {
       sq = S.sq[e];
       hu = S.hu[e];
-      if (O.adv_order >= 3) uu = S.u[e];
+      if (!kPlain && O.adv_order >= 3) uu = S.u[e];
     } else {
       uu = S.u[e];
-      ge = S.gd_e[e];
+      if constexpr (kPlain)
+        ge = 0.5f * (S.gdf_in[c1] + S.gdf_in[c2]);
+      else
+        ge = S.gd_e[e];
     }
-    const T tp = (mode >= 2) ? S.iap_tend[e] : T(0);
+    const T tp0 = (mode >= (kPlain ? 3 : 2)) ? S.iap_tend[e] : T(0);
     const T accv = (mode >= 2) ? S.iap_acc[e] : T(0);
     const T oldv = (mode >= 1 && mode <= 3) ? S.iap_old[e] : T(0);
     const T ae = (mode >= 2) ? met<T>(M.areaEdge, M.areaEdge_f, e) : T(0);
+    const T tp = (kPlain && mode == 2) ? accv : tp0;
     // the next stage's gd on the two cells (written by this stage's k_cell)
-    const bool fuse = (S.u_nx != nullptr);
+    const bool fuse = kPlain ? (mode >= 1 && mode <= 3) : (S.u_nx != nullptr);
     T gn1 = T(0), gn2 = T(0);
     if (fuse) {
       if constexpr (kF64<T>) {
@@ -1256,7 +1270,7 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
       dEdx = (E2 - E1) / dc;
       tge = 0.5f * (t1 + t2);
     }
-    if (O.flux4) {
+    if (!kPlain && O.flux4) {
       // flux_4th_order_correct (tmcore_swm_mod.F90:183-195): third derivatives
       // of E on the two cells' fit3 stencils
       const T* Ev = S.E;
@@ -1266,7 +1280,7 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
       dEdx = dEdx - (d2 - d1) * dc / T(24);
     }
     const T ut = s - dEdx;
-    if (O.adv_order >= 3) {
+    if (!kPlain && O.adv_order >= 3) {
       // the upwind side is the sign of the stage's iap_u (tmcore_swm_mod.F90:107-108);
       // u = iap_u / sqrt(gd_edge) carries the same sign bit, and unlike iap_u it
       // is always stored (the fused stages keep the next iap_u in registers)
@@ -1296,7 +1310,7 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
         break;
       case 1:
         S.iap_acc[e] = it;
-        tb[e] = it;
+        if (!kPlain) tb[e] = it;
         inext = oldv + T(rk.a_dt) * it;
         break;
       case 2:
@@ -1328,7 +1342,7 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
           S.ipe[(size_t)3 * M.ne + e] = tn * tn;
         else
           r44 = fma_acc(tn * tn, ae, r44);
-        tb[e] = it;
+        if (!kPlain) tb[e] = it;
         break;
       }
     }
@@ -1341,23 +1355,38 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
     }
   }
   if constexpr (kProducts<T, EPT>) return;
-  if (rk.mode >= 2) {
+  if (mode >= 2) {
     const T v[2] = {rip, r44};
-    const int r[2] = {R_IP_E + 2 * (rk.mode - 2), R_44_E};
+    const int r[2] = {R_IP_E + 2 * (mode - 2), R_44_E};
     block_store<T, 2>(v, P, r);
   }
 }
 
 // the single-model kernel, and the ensemble kernel (member = blockIdx.y) with
 // its register budget capped so that member pointers do not halve occupancy
-template <class T, int EPT>
-__global__ void __launch_bounds__(kMaxBlock) k_edge_flux(DevMesh M, ModelOpt O, StageIO<T> S0, RKStage rk, Partials P0) {
-  edge_flux_body<T, false, EPT>(M, O, S0, rk, P0);
+// (two blocks of 512, 64 registers: left to itself the compiler takes 40 for
+// the FP32 stages, which holds their loads back, and up to 104 for the FP64
+// stages, which leaves the FP64 pipe too few warps: level 8 402 -> 419 us)
+template <class T, int EPT, int kMode>
+__global__ void __launch_bounds__(kMaxBlock, 2) k_edge_flux(DevMesh M, ModelOpt O, StageIO<T> S0, RKStage rk, Partials P0) {
+  edge_flux_body<T, false, EPT, kMode>(M, O, S0, rk, P0);
 }
-template <class T>
+template <class T, int kMode>
 __global__ void __launch_bounds__(kMemberBlock, TMC_FLUX_MIN_BLOCKS) k_edge_flux_members(DevMesh M, ModelOpt O, StageIO<T> S0, RKStage rk,
                                                                     Partials P0) {
-  edge_flux_body<T, true, kEPT>(M, O, S0, rk, P0);
+  edge_flux_body<T, true, kEPT, kMode>(M, O, S0, rk, P0);
+}
+// f with the stage as a constant, or kGeneral
+template <class F>
+inline void on_mode(bool plain, int mode, F&& f) {
+  switch (plain ? mode : kGeneral) {
+    case 0: f(std::integral_constant<int, 0>()); break;
+    case 1: f(std::integral_constant<int, 1>()); break;
+    case 2: f(std::integral_constant<int, 2>()); break;
+    case 3: f(std::integral_constant<int, 3>()); break;
+    case 4: f(std::integral_constant<int, 4>()); break;
+    default: f(std::integral_constant<int, kGeneral>());
+  }
 }
 
 // new = old + (beta dt) t_new (update_state, tmcore_swm_mod.F90:203-213)
@@ -1512,7 +1541,7 @@ __device__ __forceinline__ void tracer_tend_f(const float (&ns)[kME], const floa
     float sq = 0.f;
 #pragma unroll
     for (int i = 0; i < kME; ++i) sq += ns[i] * Fv[i] * (0.5f * (qs[j] + qn[j][i])) * dv[i];
-    tq[j] = -sq * invAf;
+    tq[j] = __fmul_rn(-sq, invAf);  // a tendency, not a term of an FMA
   }
 }
 // ... and its RK update (mode as RKStage; gnf the stage's next gd in FP32).
@@ -1544,7 +1573,10 @@ __device__ __forceinline__ void tracer_update_f(const StageIO<float>& S, size_t 
 // (indices and the cell's own values, then the gathers of the edges' u, F,
 // dvEdge, areaEdge and of the neighbours' tracer mixing ratios), so one cell
 // costs two memory round trips.  Same arithmetic as the FP32 branch of k_cell.
-template <int NTR, bool kB, int EPT>
+// kMode as in edge_flux_body; with tracers the constant stages form the mass
+// flux from u and the two cells' gd (whose index the tracers need anyway)
+// instead of gathering it.
+template <int NTR, bool kB, int EPT, int kMode>
 __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<float>& S0, RKStage rk,
                                                const Partials& P0, int diag) {
   const StageIO<float> S = kB ? S0.at(blockIdx.y) : S0;
@@ -1553,7 +1585,8 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
   float rip = 0.f, r44 = 0.f;
   double mass = 0.0;
   float eh = 0.f, el = 0.f;
-  const int mode = rk.mode;
+  constexpr bool kPlain = kMode != kGeneral;
+  const int mode = kPlain ? kMode : rk.mode;
   TMC_FOR_N(EPT, c, M.nc) {
     int ei[kME], ci[kME];
     float ns[kME];
@@ -1565,7 +1598,7 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
     }
     const double gold = (mode <= 3) ? S.gd_old[c] : 0.0;
     const double gacc = (mode >= 2) ? S.gd_acc[c] : 0.0;
-    const float tprev = (mode >= 2) ? S.tendf[c] : 0.f;
+    const float tprev = (kPlain && mode == 2) ? (float)gacc : (mode >= 2) ? S.tendf[c] : 0.f;
     const float gdf = S.gdf_in[c], ghf = S.ghsf[c];
     const double invA = M.invAreaCell[c];
     const float invAf = M.invAreaCell_f[c];
@@ -1589,7 +1622,7 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
 #pragma unroll
     for (int i = 0; i < kME; ++i) {
       uu[i] = S.u[ei[i]];
-      Fv[i] = S.F[ei[i]];
+      Fv[i] = kPlain && NTR > 0 ? S.gdf_in[ci[i]] : S.F[ei[i]];
       dv[i] = M.dvEdge_f[ei[i]];
       ae[i] = M.areaEdge_f[ei[i]];
     }
@@ -1597,6 +1630,9 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
     for (int j = 0; j < NTR; ++j)
 #pragma unroll
       for (int i = 0; i < kME; ++i) qn[j][i] = S.qr_in[(size_t)j * M.nc + ci[i]];
+    if constexpr (kPlain && NTR > 0)  // u gd_edge, the operations of prep_edge
+#pragma unroll
+      for (int i = 0; i < kME; ++i) Fv[i] = __fmul_rn(uu[i], __fmul_rn(0.5f, __fadd_rn(gdf, Fv[i])));
     // divergence of the mass flux (two-sum), kinetic energy, E
     float hi = 0.f, lo = 0.f, k = 0.f;
 #pragma unroll
@@ -1604,7 +1640,7 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
       two_sum_acc(hi, lo, __fmul_rn(__fmul_rn(ns[i], Fv[i]), dv[i]));
       k += fabsf(ns[i]) * uu[i] * uu[i] * ae[i];
     }
-    const double t = -((double)hi + (double)lo) * invA;
+    const double t = __dmul_rn(-((double)hi + (double)lo), invA);
     const float tT = (float)t;
     S.E[c] = k * 0.25f * invAf + gdf + ghf;
     float tq[NQ];
@@ -1667,10 +1703,10 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
   }
 }
 
-template <int NTR, int EPT>
+template <int NTR, int EPT, int kMode>
 __global__ void __launch_bounds__(kCellBlock, TMC_CELL_SINGLE_MIN_BLOCKS) k_cell_fast(DevMesh M, StageIO<float> S0, RKStage rk, Partials P0,
                                                          int diag) {
-  cell_fast_body<NTR, false, EPT>(M, S0, rk, P0, diag);
+  cell_fast_body<NTR, false, EPT, kMode>(M, S0, rk, P0, diag);
 }
 // The tracer terms of the FP32 cell pass alone, for a stage whose cell pass
 // ran tracer-free (k_cell_fast<0>): the same loads and the same arithmetic
@@ -1714,10 +1750,10 @@ __global__ void __launch_bounds__(kCellBlock) k_tracers_fast(DevMesh M, StageIO<
   }
 }
 
-template <int NTR>
+template <int NTR, int kMode>
 __global__ void __launch_bounds__(kMemberBlock, NTR == 0 ? TMC_CELL_MIN_BLOCKS : 3) k_cell_fast_members(DevMesh M, StageIO<float> S0, RKStage rk,
                                                                     Partials P0, int diag) {
-  cell_fast_body<NTR, true, kEPT>(M, S0, rk, P0, diag);
+  cell_fast_body<NTR, true, kEPT, kMode>(M, S0, rk, P0, diag);
 }
 
 template <class T>
@@ -1728,12 +1764,17 @@ void launch_cell(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKSta
     const int dg = diag ? 1 : 0;
     auto run = [&](auto ntr) {
       constexpr int N = decltype(ntr)::value;
-      if (S.members > 1)
-        k_cell_fast_members<N><<<dim3(grid_for(M.nc, b.bs), nmem(S)), b.bs, 0, st>>>(M, S, rk, P, dg);
-      else if (b.ept == 1)
-        k_cell_fast<N, 1><<<grid_for(M.nc, b), b.bs, 0, st>>>(M, S, rk, P, dg);
-      else
-        k_cell_fast<N, kEPT><<<grid_for(M.nc, b), b.bs, 0, st>>>(M, S, rk, P, dg);
+      on_mode(!S.gd_e, rk.mode, [&](auto m) {
+        constexpr int kMode = decltype(m)::value;
+        if constexpr (kMode != 0) {
+          if (S.members > 1)
+            k_cell_fast_members<N, kMode><<<dim3(grid_for(M.nc, b.bs), nmem(S)), b.bs, 0, st>>>(M, S, rk, P, dg);
+          else if (b.ept == 1)
+            k_cell_fast<N, 1, kMode><<<grid_for(M.nc, b), b.bs, 0, st>>>(M, S, rk, P, dg);
+          else
+            k_cell_fast<N, kEPT, kMode><<<grid_for(M.nc, b), b.bs, 0, st>>>(M, S, rk, P, dg);
+        }
+      });
     };
     if (fast) {
       switch (O.n_tracers) {
@@ -1794,16 +1835,21 @@ void launch_edge_pv(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Bl
 template <class T>
 void launch_edge_flux(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Partials P, Blk b,
                       cudaStream_t st) {
-  if constexpr (!kF64<T>) {
-    if (S.members > 1) {
-      k_edge_flux_members<T><<<dim3(grid_for(M.ne, b.bs), nmem(S)), b.bs, 0, st>>>(M, O, S, rk, P);
-      return;
+  // FP32 models that are not second order, and the conservative APVM, store gd_edge
+  const bool plain = kF64<T> ? O.adv_order == 2 && !O.flux4 : !S.gd_e;
+  on_mode(plain, rk.mode, [&](auto m) {
+    constexpr int kMode = decltype(m)::value;
+    if constexpr (!kF64<T>) {
+      if (S.members > 1) {
+        k_edge_flux_members<T, kMode><<<dim3(grid_for(M.ne, b.bs), nmem(S)), b.bs, 0, st>>>(M, O, S, rk, P);
+        return;
+      }
     }
-  }
-  if (b.ept == 1)
-    k_edge_flux<T, 1><<<grid_for(M.ne, b), b.bs, 0, st>>>(M, O, S, rk, P);
-  else
-    k_edge_flux<T, kEPT><<<grid_for(M.ne, b), b.bs, 0, st>>>(M, O, S, rk, P);
+    if (b.ept == 1)
+      k_edge_flux<T, 1, kMode><<<grid_for(M.ne, b), b.bs, 0, st>>>(M, O, S, rk, P);
+    else
+      k_edge_flux<T, kEPT, kMode><<<grid_for(M.ne, b), b.bs, 0, st>>>(M, O, S, rk, P);
+  });
 }
 template <class T>
 void launch_final_update(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, const double* diag, Partials P,
@@ -1861,16 +1907,19 @@ void launch_to_f64(size_t n, const T* src, double* dst, cudaStream_t st) {
   k_to_f64<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, src, dst);
 }
 
+// the cell passes (their many stage and tracer variants compile beside the rest)
+#define TMC_INSTANTIATE_CELL(T) \
+  template void launch_cell<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, Partials, bool, Blk, \
+                               cudaStream_t);                                                                     \
+  template void launch_tracers_fast<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, Blk,           \
+                                       cudaStream_t);
+
 #define TMC_INSTANTIATE(T)                                                                                        \
   template void launch_gather<T>(int, const double*, const int32_t*, T*, cudaStream_t);                          \
   template void launch_scatter<T>(int, const T*, const int32_t*, double*, cudaStream_t);                         \
   template void launch_iap_from_u<T>(int, const double*, const double*, T*, cudaStream_t);                       \
   template void launch_edge_prep<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, Partials, bool, Blk,     \
                                     cudaStream_t);                                                                \
-  template void launch_cell<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, Partials, bool, Blk, \
-                               cudaStream_t);                                                                     \
-  template void launch_tracers_fast<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, Blk,           \
-                                       cudaStream_t);                                                             \
   template void launch_vertex<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, Partials, bool, Blk,        \
                                  cudaStream_t);                                                                   \
   template void launch_edge_pv<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, Blk, cudaStream_t);        \

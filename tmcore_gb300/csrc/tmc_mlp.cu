@@ -67,7 +67,6 @@ __device__ __forceinline__ void closure_features(const DevMesh& M, const StageIO
   const float pc1 = S.pv_c[oc + c1], pc2 = S.pv_c[oc + c2];
   x[0] = u[e];
   x[1] = ve;
-  x[2] = S.gd_e[oe + e];
   x[3] = S.pv_e[oe + e];
   x[4] = pv1;
   x[5] = pv2;
@@ -75,6 +74,7 @@ __device__ __forceinline__ void closure_features(const DevMesh& M, const StageIO
   x[7] = pc2;
   x[8] = S.gdf_in[oc + c1];
   x[9] = S.gdf_in[oc + c2];
+  x[2] = S.gd_e ? S.gd_e[oe + e] : 0.5f * (x[8] + x[9]);
   x[10] = S.E[oc + c1];
   x[11] = S.E[oc + c2];
   x[12] = S.ghsf[oc + c1];
