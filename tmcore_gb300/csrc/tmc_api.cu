@@ -128,7 +128,20 @@ struct tmc_handle {
   // factors of the inner products and vertex terms of the invariants (FP32,
   // passes of one element per thread)
   float *ipc = nullptr, *ipe = nullptr, *vterm = nullptr;
-  Blk blk(int pass) const { return Blk(bsp[pass], ept[pass]); }
+  Blk blk(int pass, bool pdl = false) const { return Blk(bsp[pass], ept[pass], pdl && ept[pass] == 1); }
+  // a small FP32 model (every pass one element per thread) runs its stages as
+  // one chain of dependent launches on st, the cell and vertex passes in one
+  // of them, instead of on two streams (launch_stage): a stage of it is three
+  // or four launches of 3-7 us, each about 1 us later than its predecessor's
+  // end on two streams.  Us per step, two streams / chain: FP32 level 5 47 /
+  // 35, level 6 with four tracers 61 / 54, with upwind pv 72 / 67.  FP64
+  // passes fill the FP64 pipe, which two streams share better (level 6 178 /
+  // 205).
+  bool chain() const {
+    for (int k = 0; k < 5; ++k)
+      if (ept[k] != 1) return false;
+    return p.precision == TMC_FP32 && !generic && members == 1 && O.pv_scheme != 2 && bsp[0] == bsp[1];
+  }
   // learned PV-on-edge closure (FP32 path): network, per-member switch, wait status
   const tmc_mlp* closure = nullptr;
   tmc::mlp::Net closure_net{};
@@ -415,7 +428,7 @@ struct Engine : EngineBase {
   }
 
   // beta (step) and the invariants (diag) of the fused program's passes
-  void launch_sums(bool step, bool diag) {
+  void launch_sums(bool step, bool diag, bool pdl = false) {
     const DevMesh& M = h->M;
     Products X{};
     if constexpr (std::is_same<T, float>::value) {
@@ -424,7 +437,7 @@ struct Engine : EngineBase {
                    !step || !launch_cell_is_fast(h->O), !step};
     }
     launch_finalize(h->P, h->counts, h->hm.totalArea, h->hm.sumAreaTriangle, h->O.dt, step, diag,
-                    h->p.conserve_energy != 0 && step, h->d_diag, h->st, 2, h->members, X.c ? &X : nullptr);
+                    h->p.conserve_energy != 0 && step, h->d_diag, h->st, 2, h->members, X.c ? &X : nullptr, pdl);
   }
 
   // one CRK4 step (time_scheme_mod.F90:109-154); state(old) updated in place.
@@ -438,9 +451,10 @@ struct Engine : EngineBase {
     const ModelOpt& O = h->O;
     const double dt = O.dt;
     for (int k = first_stage; k <= 4; ++k) launch_stage(k, diag && k == 1, false, flux_ev, ev_pos);
-    launch_sums(true, diag);
+    const bool chain = !flux_ev && h->chain();
+    launch_sums(true, diag, chain);
     if (flux_ev && h->timed_pass == P_FINAL) cudaEventRecord((*flux_ev)[(*ev_pos)++], h->st);
-    launch_final_update<T>(M, O, io(0), h->d_diag, h->P, h->blk(P_FINAL), h->st);
+    launch_final_update<T>(M, O, io(0), h->d_diag, h->P, h->blk(P_FINAL, chain), h->st);
     if (flux_ev && h->timed_pass == P_FINAL) cudaEventRecord((*flux_ev)[(*ev_pos)++], h->st);
   }
 
@@ -458,6 +472,13 @@ struct Engine : EngineBase {
     auto mark = [&](int pass) {
       if (flux_ev && h->timed_pass == pass) cudaEventRecord((*flux_ev)[(*ev_pos)++], h->st);
     };
+    if (!flux_ev && !no_tracers && h->chain()) {
+      launch_cell_vertex<T>(M, O, s, rk, h->P, dg, h->blk(P_CELL, true), h->st);
+      launch_edge_pv<T>(M, O, s, h->blk(P_PV, !O.need_pv_c), h->st);
+      launch_closure_pass(s, k);
+      launch_edge_flux<T>(M, O, s, rk, h->P, h->blk(P_FLUX, !h->closure), h->st);
+      return;
+    }
     // concurrent cell and vertex / pv-on-edge branches, except while passes
     // are timed one by one and for the conservative APVM (its global sums)
     const bool branch = !flux_ev && O.pv_scheme != 2;

@@ -283,10 +283,27 @@ inline unsigned nmem(const StageIO<T>& S) {
 
 // Launch shape of a pass: threads per block and elements per thread, 1 or
 // kEPT.  One on a mesh too small to fill the GPU otherwise (elements_per_thread).
+// pdl: a programmatic dependent launch, for kernels of one element per thread:
+// they may start while the stream's previous kernel runs and wait for it
+// (pdl_wait) before they read or write anything but the mesh.
 struct Blk {
   int bs, ept;
-  Blk(int b, int e = kEPT) : bs(b), ept(e) {}
+  bool pdl;
+  Blk(int b, int e = kEPT, bool p = false) : bs(b), ept(e), pdl(p) {}
 };
+template <class... K, class... A>
+inline void launch(void (*kernel)(K...), int grid, const Blk& b, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)b.bs);
+  c.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = b.pdl ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, K(args)...);
+}
 
 // ---- launchers (instantiated in tmc_kernels_f64.cu / _f32.cu) ----
 template <class T>
@@ -309,6 +326,11 @@ void launch_tracers_fast(const DevMesh& M, const ModelOpt& O, const StageIO<T>& 
 template <class T>
 void launch_vertex(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Partials P, bool diag, Blk b,
                    cudaStream_t st);
+// the cell and vertex passes of one stage in one launch (they read only the
+// stage's input, nothing the other writes); b.ept 1, the same block size for both
+template <class T>
+void launch_cell_vertex(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Partials P, bool diag,
+                        Blk b, cudaStream_t st);
 template <class T>
 void launch_edge_pv(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Blk b, cudaStream_t st);
 template <class T>
@@ -339,7 +361,7 @@ struct Products {
 };
 void launch_finalize(Partials P, const int* counts_host, double totalArea, double sumAreaTriangle, double dt,
                      bool step, bool diag, bool conserve, double* diag_out, cudaStream_t st, int scheme = 2,
-                     int members = 1, const Products* products = nullptr);
+                     int members = 1, const Products* products = nullptr, bool pdl = false);
 
 // conservative APVM (pv_scheme 2) after k_edge_pv: both tangent fluxes, their
 // curls and the three global sums, epsilon, and the correction of pv_edge

@@ -98,6 +98,8 @@ __device__ __forceinline__ void finish_step(const FinalizeArgs& a, const double*
 // step went from 118.3 to 102.8 us with the integer sums.
 __global__ void __launch_bounds__(256) k_finalize(Partials P0, FinalizeArgs a, double* out0, double* res0,
                                                   unsigned int* counter0) {
+  pdl_start();
+  pdl_wait();
   // one member per blockIdx.y: its partials, outputs, region sums and counter
   const Partials P = P0.at(blockIdx.y);
   double* out = out0 + (size_t)blockIdx.y * kDiagStride;
@@ -163,6 +165,8 @@ __device__ __forceinline__ void sum_products(const Partials& P, const float* f, 
 }
 __global__ void __launch_bounds__(256) k_finalize_products(Partials P, FinalizeArgs a, Products X, int nbc, int nbe,
                                                            int nbv, double* out, double* res, unsigned int* counter) {
+  pdl_start();
+  pdl_wait();
   const int b = blockIdx.x;
   if (b < nbc) {
     if (a.step) {
@@ -258,7 +262,7 @@ __global__ void __launch_bounds__(256) k_finalize_products(Partials P, FinalizeA
 
 void launch_finalize(Partials P, const int* counts_host, double totalArea, double sumAreaTriangle, double dt,
                      bool step, bool diag, bool conserve, double* diag_out, cudaStream_t st, int scheme,
-                     int members, const Products* products) {
+                     int members, const Products* products, bool pdl) {
   FinalizeArgs a;
   for (int r = 0; r < R_COUNT; ++r) a.counts[r] = counts_host[r];
   a.totalArea = totalArea;
@@ -282,8 +286,12 @@ void launch_finalize(Partials P, const int* counts_host, double totalArea, doubl
   if (products) {
     const int nbc = products->c ? grid_for(products->nc, 256) : 0, nbe = products->e ? grid_for(products->ne, 256) : 0;
     const int nbv = products->v && diag ? grid_for(products->nv, 256) : 0;
-    k_finalize_products<<<std::max(nbc + nbe + nbv, 1), 256, 0, st>>>(P, a, *products, nbc, nbe, nbv, diag_out, res,
-                                                                      counter);
+    launch(k_finalize_products, std::max(nbc + nbe + nbv, 1), Blk(256, 1, pdl), st, P, a, *products, nbc, nbe, nbv,
+           diag_out, res, counter);
+    return;
+  }
+  if (pdl && members <= 1) {
+    launch(k_finalize, kFinalizeRegions * a.split, Blk(256, 1, true), st, P, a, diag_out, res, counter);
     return;
   }
   k_finalize<<<dim3(kFinalizeRegions * a.split, members > 1 ? members : 1), 256, 0, st>>>(P, a, diag_out, res,

@@ -98,6 +98,25 @@ __device__ __forceinline__ void block_store(const A (&v)[N], const Partials& P, 
 template <class T>
 constexpr bool kF64 = std::is_same<T, double>::value;
 
+// Programmatic dependent launch (Blk::pdl): the kernels of one element per
+// thread of a single model let the next one start at once (pdl_start) and wait
+// for the previous one before they touch the state (pdl_wait), after the loads
+// of the mesh where those come first.  In a launch without the attribute both
+// do nothing.
+__device__ __forceinline__ void pdl_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <bool kB, int EPT>
+constexpr bool kPdl = !kB && EPT == 1;
+// the state of a dependent launch is another kernel's output until pdl_wait:
+// plain loads, where a kernel alone reads its inputs through the read-only path
+template <bool kDep, class T>
+__device__ __forceinline__ T state_load(const T* p) {
+  if constexpr (kDep)
+    return *p;
+  else
+    return __ldg(p);
+}
+
 // The FP32 passes of one element per thread store the factors of the CRK4
 // inner products and the vertex terms of the invariants, and no block sums:
 // k_finalize_products sums them, and the other invariants from the state, in
@@ -190,10 +209,10 @@ __device__ __forceinline__ void block_store_ff(const float (&hi)[N], const float
 }
 
 // block-strided loop: thread handles i = base + k*blockDim.x, k < EPT
-#define TMC_FOR_N(EPT, i, n)                                                          \
-  for (int _k = 0, i = blockIdx.x * (EPT * blockDim.x) + threadIdx.x; _k < EPT; \
-       ++_k, i += blockDim.x)                                                         \
+#define TMC_FOR_AT(bx, EPT, i, n)                                                                         \
+  for (int _k = 0, i = (bx) * (EPT * blockDim.x) + threadIdx.x; _k < EPT; ++_k, i += blockDim.x) \
     if (i < (n))
+#define TMC_FOR_N(EPT, i, n) TMC_FOR_AT((int)blockIdx.x, EPT, i, n)
 #define TMC_FOR_EPT(i, n) TMC_FOR_N(kEPT, i, n)
 
 // x / 12
@@ -392,6 +411,10 @@ template <class T, bool kB, int EPT>
 __global__ void __launch_bounds__(kMaxBlock) k_edge_prep(DevMesh M, ModelOpt O, StageIO<T> S0, Partials P0, int diag) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
+  if constexpr (kPdl<kB, EPT>) {
+    pdl_start();
+    pdl_wait();
+  }
   double en = 0.0;
   const CellSrc<T> C{S.gd_in, S.gdf_in, S.q_in, S.qr_in, nullptr};
   TMC_FOR_N(EPT, e, M.ne) {
@@ -424,13 +447,18 @@ __global__ void __launch_bounds__(kMaxBlock) k_edge_prep(DevMesh M, ModelOpt O, 
 // cell: div of mass flux, kinetic energy, E, RK update of gd and tracers
 // ---------------------------------------------------------------------------
 template <class T, bool kB, int EPT>
-__global__ void __launch_bounds__(kMaxBlock) k_cell(DevMesh M, ModelOpt O, StageIO<T> S0, RKStage rk, Partials P0,
-                                                    int diag) {
+__device__ __forceinline__ void cell_body(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S0, RKStage rk,
+                                          const Partials& P0, int diag, int b0 = 0) {
+  const int bx = (int)blockIdx.x - b0;  // this block among the cells' blocks
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
+  if constexpr (kPdl<kB, EPT>) {
+    pdl_start();
+    pdl_wait();
+  }
   T rip = T(0), r44 = T(0);
   double mass = 0.0, enc = 0.0;
-  TMC_FOR_N(EPT, c, M.nc) {
+  TMC_FOR_AT(bx, EPT, c, M.nc) {
     double t;  // gd tendency, FP64 in both modes
     double rA = 0.0;  // FP64: 1 / areaCell
     T tT, ke;
@@ -663,38 +691,51 @@ __global__ void __launch_bounds__(kMaxBlock) k_cell(DevMesh M, ModelOpt O, Stage
   if (!kProducts<T, EPT> && rk.mode >= 2) {
     const T v[2] = {rip, r44};
     const int r[2] = {R_IP_C + 2 * (rk.mode - 2), R_44_C};
-    block_store<T, 2>(v, P, r);
+    block_store<T, 2>(v, P, r, bx);
   }
   if (!kProducts<T, EPT> && diag) {
     const double v[2] = {mass, enc};
     const int r[2] = {R_MASS, R_EN_C};
-    block_store<double, 2>(v, P, r);
+    block_store<double, 2>(v, P, r, bx);
   }
+}
+template <class T, bool kB, int EPT>
+__global__ void __launch_bounds__(kMaxBlock) k_cell(DevMesh M, ModelOpt O, StageIO<T> S0, RKStage rk, Partials P0,
+                                                    int diag) {
+  cell_body<T, kB, EPT>(M, O, S0, rk, P0, diag);
 }
 
 // ---------------------------------------------------------------------------
 // vertex: gd on vertices, vorticity, potential vorticity
 // ---------------------------------------------------------------------------
 template <class T, bool kB, int EPT>
-__global__ void __launch_bounds__(kMaxBlock) k_vertex(DevMesh M, ModelOpt O, StageIO<T> S0, Partials P0, int diag) {
+__device__ __forceinline__ void vertex_body(const DevMesh& M, const StageIO<T>& S0, const Partials& P0, int diag) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
+  if constexpr (kPdl<kB, EPT>) pdl_start();
   double pe = 0.0, av = 0.0;      // FP64 path
   float ph = 0.f, pl = 0.f, ah = 0.f, al = 0.f;  // FP32 path: compensated sums
   if constexpr (kF64<T>) {
     TMC_FOR_N(EPT, v, M.nv) {
       // operators_mod.F90:106-123 (c2v), :76-91 (curl), :262-270 (pv)
-      double s = 0.0, gv = 0.0;
+      double s = 0.0, gv = 0.0, kt[3];
+      int ci[3], ei[3], ts[3];
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
-        gv = gv + S.gd_in[M.cellsOnVertex[(size_t)i * M.nv + v]] * M.kite[(size_t)i * M.nv + v];
-      const double At = M.areaTriangle[v], rAt = M.invAreaTriangle[v];
+      for (int i = 0; i < 3; ++i) {
+        ci[i] = M.cellsOnVertex[(size_t)i * M.nv + v];
+        ei[i] = M.edgesOnVertex[(size_t)i * M.nv + v];
+        ts[i] = M.tSign[(size_t)i * M.nv + v];
+        kt[i] = M.kite[(size_t)i * M.nv + v];
+      }
+      const double At = M.areaTriangle[v], rAt = M.invAreaTriangle[v], fv = M.fVertex[v];
+      if constexpr (kPdl<kB, EPT>) pdl_wait();
+#pragma unroll
+      for (int i = 0; i < 3; ++i) gv = gv + S.gd_in[ci[i]] * kt[i];
       gv = f64::div_r(gv, At, rAt);
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
-        s = s + f64::with_sign(S.ud[M.edgesOnVertex[(size_t)i * M.nv + v]], M.tSign[(size_t)i * M.nv + v]);
+      for (int i = 0; i < 3; ++i) s = s + f64::with_sign(S.ud[ei[i]], ts[i]);
       const double vo = f64::div_r(-s, At, rAt);
-      const double ab = M.fVertex[v] + vo;
+      const double ab = fv + vo;
       const double pv = f64::div_r(ab, gv, f64::recip(gv));
       S.pv_v[v] = pv;
       if (S.vor) S.vor[v] = vo;
@@ -720,16 +761,20 @@ __global__ void __launch_bounds__(kMaxBlock) k_vertex(DevMesh M, ModelOpt O, Sta
         kt[i] = __ldg(M.kite_f + (size_t)i * M.nv + v);
         ts[i] = (float)__ldg(M.tSign + (size_t)i * M.nv + v);
       }
+      // (with a dependent launch the state is another kernel's output until
+      // pdl_wait, so its loads then are plain ones)
       float g[3], uu[3], dc[3];
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        g[i] = __ldg(S.gdf_in + ci[i]);
-        uu[i] = __ldg(S.u + ei[i]);
-        dc[i] = __ldg(M.dcEdge_f + ei[i]);
-      }
+      for (int i = 0; i < 3; ++i) dc[i] = __ldg(M.dcEdge_f + ei[i]);
       const float iA = __ldg(M.invAreaTriangle_f + v);
       const float At = diag ? __ldg(M.areaTriangle_f + v) : 0.f;
       const float fv = __ldg(M.fVertex_f + v);
+      if constexpr (kPdl<kB, EPT>) pdl_wait();
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        g[i] = kPdl<kB, EPT> ? S.gdf_in[ci[i]] : __ldg(S.gdf_in + ci[i]);
+        uu[i] = kPdl<kB, EPT> ? S.u[ei[i]] : __ldg(S.u + ei[i]);
+      }
       const float gv = (g[0] * kt[0] + g[1] * kt[1] + g[2] * kt[2]) * iA;
       const float sv = ts[0] * uu[0] * dc[0] + ts[1] * uu[1] * dc[1] + ts[2] * uu[2] * dc[2];
       const float vo = -sv * iA;
@@ -752,7 +797,6 @@ __global__ void __launch_bounds__(kMaxBlock) k_vertex(DevMesh M, ModelOpt O, Sta
       }
     }
   }
-  (void)O;
   if (!kProducts<T, EPT> && diag) {
     const int r[2] = {R_PE, R_AV};
     if constexpr (kF64<T>) {
@@ -763,6 +807,20 @@ __global__ void __launch_bounds__(kMaxBlock) k_vertex(DevMesh M, ModelOpt O, Sta
       block_store_ff<2>(h, l, P, r);
     }
   }
+}
+template <class T, bool kB, int EPT>
+__global__ void __launch_bounds__(kMaxBlock) k_vertex(DevMesh M, StageIO<T> S0, Partials P0, int diag) {
+  vertex_body<T, kB, EPT>(M, S0, P0, diag);
+}
+// the cell and the vertex pass of a small model's stage in one launch: blocks
+// [0, nvb) take the vertices, the others the cells
+template <class T>
+__global__ void __launch_bounds__(kMaxBlock) k_cell_vertex(DevMesh M, ModelOpt O, StageIO<T> S, RKStage rk, Partials P,
+                                                           int diag, int nvb) {
+  if ((int)blockIdx.x < nvb)
+    vertex_body<T, false, 1>(M, S, P, diag);
+  else
+    cell_body<T, false, 1>(M, O, S, rk, P, diag, nvb);
 }
 
 // pv on cells: scalar_v2c_interp_operator as a gather (operators_mod.F90:125-141)
@@ -785,6 +843,10 @@ template <class T, bool kB, int EPT>
 __global__ void __launch_bounds__(kMaxBlock) k_edge_pv(DevMesh M, ModelOpt O, StageIO<T> S0) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const bool need_v = (O.pv_scheme >= 2) || (O.pv_scheme == 1 && O.apvm_weight != 0.0);
+  if constexpr (kPdl<kB, EPT>) {
+    pdl_start();
+    if (need_v) pdl_wait();
+  }
   if (!need_v) {
     // centred pv (APVM weight 0): all loads of the thread's EPT edges first
     const int e0 = blockIdx.x * (EPT * blockDim.x) + threadIdx.x;
@@ -796,6 +858,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_edge_pv(DevMesh M, ModelOpt O, St
       v1[j] = e < M.ne ? M.verticesOnEdge[e] : 0;
       v2[j] = e < M.ne ? M.verticesOnEdge[M.ne + e] : 0;
     }
+    if constexpr (kPdl<kB, EPT>) pdl_wait();
 #pragma unroll
     for (int j = 0; j < EPT; ++j) pe[j] = halve(S.pv_v[v1[j]] + S.pv_v[v2[j]]);
 #pragma unroll
@@ -854,15 +917,17 @@ __global__ void __launch_bounds__(kMaxBlock) k_edge_pv(DevMesh M, ModelOpt O, St
 // separate loads, 12 points at a time: 128 registers and 112 us for
 // k_vert_fit alone at level 8).  Points in flight x resident blocks, level 8,
 // both passes: 6 x 4 87.8 us, 4 x 6 87.3, 12 x 3 91.5; FP64 2 to 6 alike.
-template <class T, bool kB>
+template <class T, bool kB, bool kDep>
 __global__ void __launch_bounds__(256, kF64<T> ? 1 : 4) k_vert_fit(DevMesh M, StageIO<T> S0) {
   constexpr int kU = kF64<T> ? 4 : 6;  // points whose loads are in flight together
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const int v = blockIdx.x * blockDim.x + threadIdx.x, nv = M.nv;
+  if constexpr (kDep) pdl_start();
   if (v >= nv) return;
   const int n = __ldg(M.vfit_n + v);
-  const T fc = __ldg(S.pv_v + v);
-  T acc[3] = {T(0), T(0), T(0)};
+  if (kDep && n == 0) pdl_wait();
+  T fc = T(0), acc[3] = {T(0), T(0), T(0)};
+  if constexpr (!kDep) fc = __ldg(S.pv_v + v);
   for (int j0 = 0; j0 < n; j0 += kU) {
     int ix[kU];
     T w[3][kU], f[kU];
@@ -881,8 +946,14 @@ __global__ void __launch_bounds__(256, kF64<T> ? 1 : 4) k_vert_fit(DevMesh M, St
         ix[j] = __float_as_int(r.w);
       }
     }
+    if constexpr (kDep) {  // after the first points' records
+      if (j0 == 0) {
+        pdl_wait();
+        fc = S.pv_v[v];
+      }
+    }
 #pragma unroll
-    for (int j = 0; j < kU; ++j) f[j] = __ldg(S.pv_v + ix[j]);
+    for (int j = 0; j < kU; ++j) f[j] = state_load<kDep>(S.pv_v + ix[j]);
 #pragma unroll
     for (int j = 0; j < kU; ++j)
       if (j0 + j < n) {
@@ -903,15 +974,16 @@ __global__ void __launch_bounds__(256, kF64<T> ? 1 : 4) k_vert_fit(DevMesh M, St
 // it is decided by an FP32 sum wherever that exceeds the sum's error bound (12
 // terms of 2^-24 of the magnitudes; the test asks for 32), else by the FP64
 // sum in the reference order: 20 FP64 instructions per edge less.
-template <class T>
+template <class T, bool kDep>
 __device__ __forceinline__ T upwind_sign(const DevMesh& M, const StageIO<T>& S, int e) {
   const int ne = M.ne;
   if constexpr (kF64<T>) {
     const int n = M.nEdgesOnEdge[e];
+    if constexpr (kDep) pdl_wait();
     float s = 0.f, a = 0.f;
 #pragma unroll 5
     for (int i = 0; i < n; ++i) {
-      const float t = __fmul_rn(__ldg(S.uf + __ldg(M.edgesOnEdge + (size_t)i * ne + e)),
+      const float t = __fmul_rn(state_load<kDep>(S.uf + __ldg(M.edgesOnEdge + (size_t)i * ne + e)),
                                 __ldg(M.weightsOnEdge_f + (size_t)i * ne + e));
       s = __fadd_rn(s, t);
       a = __fadd_rn(a, fabsf(t));
@@ -931,23 +1003,25 @@ __device__ __forceinline__ T upwind_sign(const DevMesh& M, const StageIO<T>& S, 
       eo[i] = __ldg(M.edgesOnEdge + (size_t)i * ne + e);  // padded slots: the edge itself, weight 0
       wo[i] = __ldg(M.weightsOnEdge_f + (size_t)i * ne + e);
     }
+    if constexpr (kDep) pdl_wait();
 #pragma unroll
-    for (int i = 0; i < kME2; ++i) uo[i] = __ldg(S.u + eo[i]);
+    for (int i = 0; i < kME2; ++i) uo[i] = state_load<kDep>(S.u + eo[i]);
 #pragma unroll
     for (int i = 0; i < kME2; ++i) ve = ve + uo[i] * wo[i];
     return sgn1(ve);
   }
 }
-template <class T, bool kB>
+template <class T, bool kB, bool kDep>
 __global__ void __launch_bounds__(256) k_edge_up(DevMesh M, ModelOpt O, StageIO<T> S0) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if constexpr (kDep) pdl_start();
   if (e >= M.ne) return;
   const int v1 = __ldg(M.verticesOnEdge + e), v2 = __ldg(M.verticesOnEdge + M.ne + e);
-  const T d0 = __ldg(S.dfit + e), d1 = __ldg(S.dfit + M.ne + e);
   const T dist = __ldg(met_p<T>(M.dvEdge, M.dvEdge_f) + e);
-  const T p1 = __ldg(S.pv_v + v1), p2 = __ldg(S.pv_v + v2);
-  const T sg = upwind_sign<T>(M, S, e);
+  const T sg = upwind_sign<T, kDep>(M, S, e);  // (waits for the previous kernel)
+  const T d0 = state_load<kDep>(S.dfit + e), d1 = state_load<kDep>(S.dfit + M.ne + e);
+  const T p1 = state_load<kDep>(S.pv_v + v1), p2 = state_load<kDep>(S.pv_v + v2);
   S.pv_e[e] = halve(p1 + p2) - over12(dist * dist * ((d0 + d1) - sg * T(O.vert_coef2) * (d1 - d0)));
 }
 
@@ -1140,7 +1214,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_combine(DevMesh M, int ntr, int s
       }                                                                                         \
     }                                                                                           \
     if (b.ept == 1)                                                                             \
-      KERNEL<T, false, 1><<<grid_for(n, b), b.bs, 0, st>>>(__VA_ARGS__);                        \
+      launch(KERNEL<T, false, 1>, grid_for(n, b), b, st, __VA_ARGS__);                          \
     else                                                                                        \
       KERNEL<T, false, kEPT><<<grid_for(n, b), b.bs, 0, st>>>(__VA_ARGS__);                     \
   } while (0)
@@ -1195,6 +1269,7 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
                                                const Partials& P0) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
+  if constexpr (kPdl<kB, EPT>) pdl_start();
   T rip = T(0), r44 = T(0);  // FP32 path: FP32 products and per-thread sums, FP64 across warps
   constexpr bool kPlain = kMode != kGeneral;
   const int mode = kPlain ? kMode : rk.mode;
@@ -1203,6 +1278,22 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
     // issued after a store through a pointer the compiler must assume aliases
     // would wait a full memory round trip.
     const int c1 = M.cellsOnEdge[e], c2 = M.cellsOnEdge[M.ne + e];
+    const T ae = (mode >= 2) ? met<T>(M.areaEdge, M.areaEdge_f, e) : T(0);
+    int ep[kME2];
+    float w[kME2];
+    T dc;
+    if constexpr (!kF64<T>) {
+#pragma unroll
+      for (int i = 0; i < kME2; ++i) {
+        const size_t k = (size_t)i * M.ne + e;
+        ep[i] = M.edgesOnEdge[k];  // padded entries: own edge with weight 0
+        w[i] = M.weightsOnEdge_f[k];
+      }
+      dc = M.dcEdge_f[e];
+    } else {
+      dc = M.dcEdge[e];
+    }
+    if constexpr (kPdl<kB, EPT>) pdl_wait();
     const T pe = S.pv_e[e];
     T uu = T(0), ge = T(0), sq = T(0), hu = T(0);
     if constexpr (kF64<T>) {
@@ -1219,7 +1310,6 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
     const T tp0 = (mode >= (kPlain ? 3 : 2)) ? S.iap_tend[e] : T(0);
     const T accv = (mode >= 2) ? S.iap_acc[e] : T(0);
     const T oldv = (mode >= 1 && mode <= 3) ? S.iap_old[e] : T(0);
-    const T ae = (mode >= 2) ? met<T>(M.areaEdge, M.areaEdge_f, e) : T(0);
     const T tp = (kPlain && mode == 2) ? accv : tp0;
     // the next stage's gd on the two cells (written by this stage's k_cell)
     const bool fuse = kPlain ? (mode >= 1 && mode <= 3) : (S.u_nx != nullptr);
@@ -1233,7 +1323,7 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
         gn2 = S.gdf_next[c2];
       }
     }
-    T s = T(0), tge, dEdx, dc;
+    T s = T(0), tge, dEdx;
     if constexpr (kF64<T>) {
       // calc_tangent_vor_flux (operators_mod.F90:239-260), in order
       // (its factor 1/2 taken out of the sum: powers of two round alike)
@@ -1245,20 +1335,10 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
         s = s + M.weightsOnEdge[k] * S.u[ep] * S.gd_e[ep] * (pe + S.pv_e[ep]);
       }
       s = f64::half(s);
-      dc = M.dcEdge[e];
       dEdx = f64::div_r(S.E[c2] - S.E[c1], dc, M.invDcEdge[e]);
       tge = f64::half(S.gd_tend[c1] + S.gd_tend[c2]);
     } else {
-      int ep[kME2];
-      float w[kME2];
-#pragma unroll
-      for (int i = 0; i < kME2; ++i) {
-        const size_t k = (size_t)i * M.ne + e;
-        ep[i] = M.edgesOnEdge[k];  // padded entries: own edge with weight 0
-        w[i] = M.weightsOnEdge_f[k];
-      }
       const float E1 = S.E[c1], E2 = S.E[c2], t1 = S.tendf[c1], t2 = S.tendf[c2];
-      dc = M.dcEdge_f[e];
       float Fv[kME2], pp[kME2];
 #pragma unroll
       for (int i = 0; i < kME2; ++i) {
@@ -1395,6 +1475,10 @@ template <class T, bool kB, int EPT>
 __global__ void __launch_bounds__(kMaxBlock) k_final_cells(DevMesh M, ModelOpt O, StageIO<T> S0, const double* diag0) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const double* diag = kB ? diag0 + (size_t)blockIdx.y * kDiagStride : diag0;
+  if constexpr (kPdl<kB, EPT>) {
+    pdl_start();
+    pdl_wait();
+  }
   const double bdt = diag[9];
   // all loads of the thread's EPT cells before any store (a load after a
   // store through a possibly aliasing pointer waits a full round trip)
@@ -1451,6 +1535,10 @@ __global__ void __launch_bounds__(kB ? kMemberBlock : kMaxBlock, kB ? TMC_FINAL_
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
   const double* diag = kB ? diag0 + (size_t)blockIdx.y * kDiagStride : diag0;
+  if constexpr (kPdl<kB, EPT>) {
+    pdl_start();
+    pdl_wait();
+  }
   const double bdt = diag[9];
   double en = 0.0;
   const CellSrc<T> C{S.gd_old, S.gdf_in, S.q_old, S.qr_in, S.ratio};
@@ -1578,7 +1666,9 @@ __device__ __forceinline__ void tracer_update_f(const StageIO<float>& S, size_t 
 // instead of gathering it.
 template <int NTR, bool kB, int EPT, int kMode>
 __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<float>& S0, RKStage rk,
-                                               const Partials& P0, int diag) {
+                                               const Partials& P0, int diag, int b0 = 0) {
+  const int bx = (int)blockIdx.x - b0;  // this block among the cells' blocks
+  if constexpr (kPdl<kB, EPT>) pdl_start();
   const StageIO<float> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
   constexpr int NQ = NTR > 0 ? NTR : 1;
@@ -1587,7 +1677,7 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
   float eh = 0.f, el = 0.f;
   constexpr bool kPlain = kMode != kGeneral;
   const int mode = kPlain ? kMode : rk.mode;
-  TMC_FOR_N(EPT, c, M.nc) {
+  TMC_FOR_AT(bx, EPT, c, M.nc) {
     int ei[kME], ci[kME];
     float ns[kME];
 #pragma unroll
@@ -1596,13 +1686,22 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
       ns[i] = (float)M.nSign[(size_t)i * M.nc + c];
       ci[i] = NTR > 0 ? M.cellsOnCell[(size_t)i * M.nc + c] : 0;
     }
+    const double invA = M.invAreaCell[c];
+    const float invAf = M.invAreaCell_f[c];
+    const float Af = (mode >= 2) ? M.areaCell_f[c] : 0.f;
+    float uu[kME], Fv[kME], dv[kME], ae[kME], qn[NQ][kME];
+    if constexpr (kPdl<kB, EPT>) {  // the mesh's values, then the previous kernel's
+#pragma unroll
+      for (int i = 0; i < kME; ++i) {
+        dv[i] = M.dvEdge_f[ei[i]];
+        ae[i] = M.areaEdge_f[ei[i]];
+      }
+      pdl_wait();
+    }
     const double gold = (mode <= 3) ? S.gd_old[c] : 0.0;
     const double gacc = (mode >= 2) ? S.gd_acc[c] : 0.0;
     const float tprev = (kPlain && mode == 2) ? (float)gacc : (mode >= 2) ? S.tendf[c] : 0.f;
     const float gdf = S.gdf_in[c], ghf = S.ghsf[c];
-    const double invA = M.invAreaCell[c];
-    const float invAf = M.invAreaCell_f[c];
-    const float Af = (mode >= 2) ? M.areaCell_f[c] : 0.f;
     float qs[NQ], qo[NQ], qa[NQ];
 #pragma unroll
     for (int j = 0; j < NTR; ++j) {
@@ -1618,13 +1717,14 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
       Ad = M.areaCell[c];
       Afd = M.areaCell_f[c];
     }
-    float uu[kME], Fv[kME], dv[kME], ae[kME], qn[NQ][kME];
 #pragma unroll
     for (int i = 0; i < kME; ++i) {
       uu[i] = S.u[ei[i]];
       Fv[i] = kPlain && NTR > 0 ? S.gdf_in[ci[i]] : S.F[ei[i]];
-      dv[i] = M.dvEdge_f[ei[i]];
-      ae[i] = M.areaEdge_f[ei[i]];
+      if constexpr (!kPdl<kB, EPT>) {
+        dv[i] = M.dvEdge_f[ei[i]];
+        ae[i] = M.areaEdge_f[ei[i]];
+      }
     }
 #pragma unroll
     for (int j = 0; j < NTR; ++j)
@@ -1708,6 +1808,14 @@ __global__ void __launch_bounds__(kCellBlock, TMC_CELL_SINGLE_MIN_BLOCKS) k_cell
                                                          int diag) {
   cell_fast_body<NTR, false, EPT, kMode>(M, S0, rk, P0, diag);
 }
+template <int NTR, int kMode>
+__global__ void __launch_bounds__(kCellBlock, TMC_CELL_SINGLE_MIN_BLOCKS) k_cell_vertex_fast(DevMesh M, StageIO<float> S, RKStage rk,
+                                                         Partials P, int diag, int nvb) {
+  if ((int)blockIdx.x < nvb)
+    vertex_body<float, false, 1>(M, S, P, diag);
+  else
+    cell_fast_body<NTR, false, 1, kMode>(M, S, rk, P, diag, nvb);
+}
 // The tracer terms of the FP32 cell pass alone, for a stage whose cell pass
 // ran tracer-free (k_cell_fast<0>): the same loads and the same arithmetic
 // (tracer_tend_f, tracer_update_f) as k_cell_fast<NTR>, with the stage's next
@@ -1789,6 +1897,30 @@ void launch_cell(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKSta
   TMC_LAUNCH(k_cell, M.nc, M, O, S, rk, P, diag ? 1 : 0);
 }
 template <class T>
+void launch_cell_vertex(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Partials P, bool diag,
+                        Blk b, cudaStream_t st) {
+  const int nvb = grid_for(M.nv, b), g = nvb + grid_for(M.nc, b), dg = diag ? 1 : 0;
+  if constexpr (!kF64<T>) {
+    auto run = [&](auto ntr) {
+      on_mode(!S.gd_e, rk.mode, [&](auto m) {
+        constexpr int kMode = decltype(m)::value;
+        if constexpr (kMode != 0)
+          launch(k_cell_vertex_fast<decltype(ntr)::value, kMode>, g, b, st, M, S, rk, P, dg, nvb);
+      });
+    };
+    if (launch_cell_is_fast(O)) {
+      switch (O.n_tracers) {
+        case 0: run(std::integral_constant<int, 0>()); return;
+        case 1: run(std::integral_constant<int, 1>()); return;
+        case 2: run(std::integral_constant<int, 2>()); return;
+        case 4: run(std::integral_constant<int, 4>()); return;
+        default: break;
+      }
+    }
+  }
+  launch(k_cell_vertex<T>, g, b, st, M, O, S, rk, P, dg, nvb);
+}
+template <class T>
 void launch_tracers_fast(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Blk b,
                          cudaStream_t st) {
   if constexpr (!kF64<T>) {
@@ -1810,7 +1942,7 @@ void launch_tracers_fast(const DevMesh& M, const ModelOpt& O, const StageIO<T>& 
 template <class T>
 void launch_vertex(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Partials P, bool diag, Blk b,
                    cudaStream_t st) {
-  TMC_LAUNCH(k_vertex, M.nv, M, O, S, P, diag ? 1 : 0);
+  TMC_LAUNCH(k_vertex, M.nv, M, S, P, diag ? 1 : 0);
 }
 template <class T>
 void launch_edge_pv(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Blk b, cudaStream_t st) {
@@ -1821,13 +1953,20 @@ void launch_edge_pv(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Bl
     const dim3 gv(nblk(M.nv, bs), nmem(S)), ge(nblk(M.ne, bs), nmem(S));
     if constexpr (!kF64<T>) {
       if (S.members > 1) {
-        k_vert_fit<T, true><<<gv, bs, 0, st>>>(M, S);
-        k_edge_up<T, true><<<ge, bs, 0, st>>>(M, O, S);
+        k_vert_fit<T, true, false><<<gv, bs, 0, st>>>(M, S);
+        k_edge_up<T, true, false><<<ge, bs, 0, st>>>(M, O, S);
         return;
       }
     }
-    k_vert_fit<T, false><<<gv, bs, 0, st>>>(M, S);
-    k_edge_up<T, false><<<ge, bs, 0, st>>>(M, O, S);
+    if constexpr (!kF64<T>) {
+      if (b.pdl) {
+        launch(k_vert_fit<T, false, true>, gv.x, Blk(bs, 1, true), st, M, S);
+        launch(k_edge_up<T, false, true>, ge.x, Blk(bs, 1, true), st, M, O, S);
+        return;
+      }
+    }
+    k_vert_fit<T, false, false><<<gv, bs, 0, st>>>(M, S);
+    k_edge_up<T, false, false><<<ge, bs, 0, st>>>(M, O, S);
     return;
   }
   TMC_LAUNCH(k_edge_pv, M.ne, M, O, S);
@@ -1846,7 +1985,7 @@ void launch_edge_flux(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, 
       }
     }
     if (b.ept == 1)
-      k_edge_flux<T, 1, kMode><<<grid_for(M.ne, b), b.bs, 0, st>>>(M, O, S, rk, P);
+      launch(k_edge_flux<T, 1, kMode>, grid_for(M.ne, b), b, st, M, O, S, rk, P);
     else
       k_edge_flux<T, kEPT, kMode><<<grid_for(M.ne, b), b.bs, 0, st>>>(M, O, S, rk, P);
   });
@@ -1911,6 +2050,8 @@ void launch_to_f64(size_t n, const T* src, double* dst, cudaStream_t st) {
 #define TMC_INSTANTIATE_CELL(T) \
   template void launch_cell<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, Partials, bool, Blk, \
                                cudaStream_t);                                                                     \
+  template void launch_cell_vertex<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, Partials, bool, \
+                                      Blk, cudaStream_t);                                                          \
   template void launch_tracers_fast<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, Blk,           \
                                        cudaStream_t);
 
