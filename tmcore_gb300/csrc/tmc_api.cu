@@ -823,6 +823,7 @@ struct EnsEngine : EngineBase {
   float* pv_c = nullptr;  // pv on cells (the learned closure's features)
   float *invA_hl = nullptr, *A_hl = nullptr;
   float *cdv = nullptr, *cae = nullptr, *vdc = nullptr;
+  ens::EdgeRec* edge_rec = nullptr;  // the learned closure's mesh values per edge
   ens::Upwind up{};  // pv_scheme 3: the vertex fit stencils (width 0 otherwise)
   explicit EnsEngine(tmc_handle* hh) : h(hh) {}
   const ens::Upwind* upwind() const { return up.width ? &up : nullptr; }
@@ -885,6 +886,26 @@ struct EnsEngine : EngineBase {
     cdv = h->upload(v_cdv);
     cae = h->upload(v_cae);
     vdc = h->upload(v_vdc);
+    {
+      std::vector<ens::EdgeRec> rec(h->M.ne);
+      const size_t ne_ = h->M.ne;
+#pragma omp parallel for schedule(static)
+      for (int e = 0; e < h->M.ne; ++e) {
+        ens::EdgeRec& r = rec[e];
+        for (int k = 0; k < 10; ++k) {
+          r.e[k] = hm.edgesOnEdge[(size_t)k * ne_ + e];
+          r.w[k] = (float)hm.weightsOnEdge[(size_t)k * ne_ + e];
+        }
+        for (int s = 0; s < 2; ++s) {
+          r.c[s] = hm.cellsOnEdge[(size_t)s * ne_ + e];
+          r.v[s] = hm.verticesOnEdge[(size_t)s * ne_ + e];
+          r.f[s] = (float)hm.fVertex[r.v[s]];
+        }
+        r.dv = (float)hm.dvEdge[e];
+        r.dc = (float)hm.dcEdge[e];
+      }
+      if (!(edge_rec = h->upload(rec))) return TMC_E_CUDA;
+    }
     if (h->O.pv_scheme == 3) {
       // the weights in FP32, as the FP32 single-model kernel converts them
       std::vector<float> wf(hm.vert2.w.begin(), hm.vert2.w.end());
@@ -977,7 +998,7 @@ struct EnsEngine : EngineBase {
         const int mode = h->closure_every_stage ? 0 : (k == 1 ? 1 : 2);
         if (mode != 2) ens::launch_v2c(M, D, s, pv_c, h->st);
         const ClosureArgs a{&h->closure_net, h->d_member_on, h->d_closure_err, h->sms, h->d_closure_dq, mode};
-        ens::launch_closure(M, D, s, pv_c, a, h->st);
+        ens::launch_closure(M, D, s, edge_rec, pv_c, a, h->st);
       }
       mark(P_PV);
       mark(P_FLUX);
@@ -1051,7 +1072,7 @@ struct EnsEngine : EngineBase {
     ens::launch_cell(h->M, D, s, RKStage{0, 0.0}, EP, false, h->bsp[P_CELL], h->st);
     ens::launch_edge_pv(h->M, D, s, upwind(), h->bsp[P_PV], h->st);
     ens::launch_v2c(h->M, D, s, pv_c, h->st);
-    ens::launch_closure_features(h->M, D, s, pv_c, h->cur, feat, pv, h->st);
+    ens::launch_closure_features(h->M, D, s, edge_rec, pv_c, h->cur, feat, pv, h->st);
   }
 
   // history fields of the selected member: its u, gd and ghs copied out of

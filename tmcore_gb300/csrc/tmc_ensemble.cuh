@@ -216,11 +216,20 @@ void launch_jobs_step(const JobTable& T, int nj, const int* bsp, bool upwind, cu
 // 1 stage 1, output also held in a.dq; 2 add the held a.dq only)
 void launch_v2c(const DevMesh& Mh, const Dims& D, const IO& S, float* pv_c, cudaStream_t st);
 void launch_closure_hold(const DevMesh& Mh, const Dims& D, const IO& S, const float* dq, cudaStream_t st);
-void launch_closure(const DevMesh& Mh, const Dims& D, const IO& S, const float* pv_c, const ClosureArgs& a,
-                    cudaStream_t st);
+// the mesh values of one edge that the network's features read
+struct alignas(16) EdgeRec {
+  int e[10];    // edgesOnEdge
+  float w[10];  // weightsOnEdge
+  int c[2], v[2];
+  float f[2];   // Coriolis on the two vertices
+  float dv, dc;
+};
+static_assert(sizeof(EdgeRec) == 112, "seven 16-byte loads");
+void launch_closure(const DevMesh& Mh, const Dims& D, const IO& S, const EdgeRec* rec, const float* pv_c,
+                    const ClosureArgs& a, cudaStream_t st);
 // the closure's features and pv_edge of member m (internal edge order) into feat[ne][24], pv[ne]
-void launch_closure_features(const DevMesh& Mh, const Dims& D, const IO& S, const float* pv_c, int m, float* feat,
-                             float* pv, cudaStream_t st);
+void launch_closure_features(const DevMesh& Mh, const Dims& D, const IO& S, const EdgeRec* rec, const float* pv_c,
+                             int m, float* feat, float* pv, cudaStream_t st);
 
 // state transfer of member m (caller's element order <-> member-innermost);
 // _ff: an FF array (h, then l at offset n * M)

@@ -172,9 +172,11 @@ __device__ bool forward_tiles(const Net& net, Src& src, long long ntiles, uint8_
   uint8_t* sA0 = sW3 + kSmemW;  // kGroups tile operands
   uint64_t* mbar0 = reinterpret_cast<uint64_t*>(sA0 + kGroups * kSmemA);  // one mbarrier per group
   uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar0 + kGroups);
-  __shared__ float sb[3][kH];
-  __shared__ float sw4[kH];
-  __shared__ float sxm[kIn], sxi[kIn];
+  // aligned so that a thread reads four biases, output weights or scalings per
+  // shared-memory load (one by one they were 240 of a row's 2,090 instructions)
+  __shared__ __align__(16) float sb[3][kH];
+  __shared__ __align__(16) float sw4[kH];
+  __shared__ __align__(16) float sxm[kIn], sxi[kIn];
   const int t = threadIdx.x, warp = t >> 5;
   // tile group of this thread (its own tiles, operand, mbarrier, accumulator
   // columns and named barrier) and its row in the group's tiles
