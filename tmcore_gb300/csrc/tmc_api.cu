@@ -823,6 +823,7 @@ struct EnsEngine : EngineBase {
   float* pv_c = nullptr;  // pv on cells (the learned closure's features)
   float *invA_hl = nullptr, *A_hl = nullptr;
   float *cdv = nullptr, *cae = nullptr, *vdc = nullptr;
+  float* v2c_kite = nullptr;         // v2c_kite in FP32
   ens::EdgeRec* edge_rec = nullptr;  // the learned closure's mesh values per edge
   ens::Upwind up{};  // pv_scheme 3: the vertex fit stencils (width 0 otherwise)
   explicit EnsEngine(tmc_handle* hh) : h(hh) {}
@@ -905,6 +906,7 @@ struct EnsEngine : EngineBase {
         r.dc = (float)hm.dcEdge[e];
       }
       if (!(edge_rec = h->upload(rec))) return TMC_E_CUDA;
+      if (!(v2c_kite = h->upload(std::vector<float>(hm.v2c_kite.begin(), hm.v2c_kite.end())))) return TMC_E_CUDA;
     }
     if (h->O.pv_scheme == 3) {
       // the weights in FP32, as the FP32 single-model kernel converts them
@@ -996,7 +998,7 @@ struct EnsEngine : EngineBase {
         // the learned closure on this stage's pv_edge: in every stage, or in
         // stage 1 with its output held for stages 2-4
         const int mode = h->closure_every_stage ? 0 : (k == 1 ? 1 : 2);
-        if (mode != 2) ens::launch_v2c(M, D, s, pv_c, h->st);
+        if (mode != 2) ens::launch_v2c(M, D, s, v2c_kite, pv_c, h->st);
         const ClosureArgs a{&h->closure_net, h->d_member_on, h->d_closure_err, h->sms, h->d_closure_dq, mode};
         ens::launch_closure(M, D, s, edge_rec, pv_c, a, h->st);
       }
@@ -1071,7 +1073,7 @@ struct EnsEngine : EngineBase {
     const ens::IO s = io(0);
     ens::launch_cell(h->M, D, s, RKStage{0, 0.0}, EP, false, h->bsp[P_CELL], h->st);
     ens::launch_edge_pv(h->M, D, s, upwind(), h->bsp[P_PV], h->st);
-    ens::launch_v2c(h->M, D, s, pv_c, h->st);
+    ens::launch_v2c(h->M, D, s, v2c_kite, pv_c, h->st);
     ens::launch_closure_features(h->M, D, s, edge_rec, pv_c, h->cur, feat, pv, h->st);
   }
 

@@ -214,7 +214,8 @@ void launch_jobs_step(const JobTable& T, int nj, const int* bsp, bool upwind, cu
 // (the network reads it), then the network on rows [edge][member] with its
 // output added to pv_edge of members whose switch is on (a.mode 0 every stage;
 // 1 stage 1, output also held in a.dq; 2 add the held a.dq only)
-void launch_v2c(const DevMesh& Mh, const Dims& D, const IO& S, float* pv_c, cudaStream_t st);
+// (kite: v2c_kite in FP32)
+void launch_v2c(const DevMesh& Mh, const Dims& D, const IO& S, const float* kite, float* pv_c, cudaStream_t st);
 void launch_closure_hold(const DevMesh& Mh, const Dims& D, const IO& S, const float* dq, cudaStream_t st);
 // the mesh values of one edge that the network's features read
 struct alignas(16) EdgeRec {
