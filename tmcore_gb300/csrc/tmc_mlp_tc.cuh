@@ -198,10 +198,22 @@ __device__ bool forward_tiles(const Net& net, Src& src, long long ntiles, uint8_
     }
     *reinterpret_cast<__nv_bfloat16*>(sW1 + core_off(n, k, kInPad)) = w;
   }
-  for (int i = t; i < kH * kH; i += blockDim.x) {
-    const int n = i / kH, k = i % kH;
-    *reinterpret_cast<__nv_bfloat16*>(sW2 + core_off(n, k, kH)) = __hmul(net.pb[kOffW2 + i], __float2bfloat16_rn(0.5f));
-    *reinterpret_cast<__nv_bfloat16*>(sW3 + core_off(n, k, kH)) = __hmul(net.pb[kOffW3 + i], __float2bfloat16_rn(0.5f));
+  for (int i = t; i < kH * kH / 8; i += blockDim.x) {  // eight inputs: 16 bytes, one core-matrix row
+    const int n = i / (kH / 8), k = i % (kH / 8) * 8;
+    union {
+      uint4 v;
+      __nv_bfloat162 h[4];
+    } a, b;
+    a.v = *reinterpret_cast<const uint4*>(net.pb + kOffW2 + n * kH + k);
+    b.v = *reinterpret_cast<const uint4*>(net.pb + kOffW3 + n * kH + k);
+    const __nv_bfloat162 half = __float2bfloat162_rn(0.5f);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      a.h[q] = __hmul2(a.h[q], half);
+      b.h[q] = __hmul2(b.h[q], half);
+    }
+    *reinterpret_cast<uint4*>(sW2 + core_off(n, k, kH)) = a.v;
+    *reinterpret_cast<uint4*>(sW3 + core_off(n, k, kH)) = b.v;
   }
   for (int i = t; i < kH; i += blockDim.x) {
     sb[0][i] = net.p[kOffB1 + i];

@@ -163,30 +163,40 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
   uint8_t* const sDZ1 = smem + kTrDZ1;
   uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + kTrBar);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + kTrBar + 8);
-  __shared__ float sb[3][kH], sw4[kH], sxm[kIn], sxi[kIn], sred[4];
+  // (aligned: a thread's 16 consecutive biases or weights are four loads)
+  __shared__ __align__(16) float sb[3][kH], sw4[kH], sxm[kIn], sxi[kIn];
+  __shared__ float sred[4];
   __shared__ float sy[kTrCG][kTile];  // the column groups' partial sums of the output
   const int t = threadIdx.x, warp = t >> 5, quarter = warp & 3, cg = warp >> 2;
   const int r = quarter * 32 + (t & 31);  // this thread's row of the tile (TMEM lane)
   const int cc = 16 * cg;                 // its first hidden column
 
-  // weights (BF16) K-major by input; layer 1's bias as a high and a low BF16
-  // part against the two input columns of ones
-  for (int i = t; i < kH * kInPad; i += blockDim.x) {
-    const int n = i / kInPad, k = i % kInPad;
-    __nv_bfloat16 w = __float2bfloat16_rn(0.f);
+  // weights (BF16) K-major by input, eight inputs (16 bytes, one core-matrix
+  // row) at a time: one load and store per thread and matrix (element by
+  // element the staging was 20 dependent rounds of every launch); layer 1's
+  // bias as a high and a low BF16 part against the two input columns of ones
+  static_assert(kOffW2 % 8 == 0 && kOffW3 % 8 == 0 && kIn % 8 == 0, "16-byte rows of BF16 weights");
+  for (int i = t; i < kH * kInPad / 8; i += blockDim.x) {
+    const int n = i / (kInPad / 8), k = i % (kInPad / 8) * 8;
+    uint4 w = make_uint4(0u, 0u, 0u, 0u);
     if (k < kIn) {
-      w = net.pb[kOffW1 + n * kIn + k];
-    } else if (k == kIn || k == kIn + 1) {
+      w = *reinterpret_cast<const uint4*>(net.pb + kOffW1 + n * kIn + k);
+    } else {
       const float b = net.p[kOffB1 + n];
       const __nv_bfloat16 hi = __float2bfloat16_rn(b);
-      w = k == kIn ? hi : __float2bfloat16_rn(b - __bfloat162float(hi));
+      __nv_bfloat162 hl;
+      hl.x = hi;
+      hl.y = __float2bfloat16_rn(b - __bfloat162float(hi));
+      w.x = *reinterpret_cast<uint32_t*>(&hl);
     }
-    *reinterpret_cast<__nv_bfloat16*>(smem + kTrW1 + core_off(n, k, kInPad)) = w;
+    *reinterpret_cast<uint4*>(smem + kTrW1 + core_off(n, k, kInPad)) = w;
   }
-  for (int i = t; i < kH * kH; i += blockDim.x) {
-    const int n = i / kH, k = i % kH;
-    *reinterpret_cast<__nv_bfloat16*>(smem + kTrW2 + core_off(n, k, kH)) = net.pb[kOffW2 + i];
-    *reinterpret_cast<__nv_bfloat16*>(smem + kTrW3 + core_off(n, k, kH)) = net.pb[kOffW3 + i];
+  for (int i = t; i < kH * kH / 8; i += blockDim.x) {
+    const int n = i / (kH / 8), k = i % (kH / 8) * 8;
+    const uint4 w2 = *reinterpret_cast<const uint4*>(net.pb + kOffW2 + n * kH + k);
+    const uint4 w3 = *reinterpret_cast<const uint4*>(net.pb + kOffW3 + n * kH + k);
+    *reinterpret_cast<uint4*>(smem + kTrW2 + core_off(n, k, kH)) = w2;
+    *reinterpret_cast<uint4*>(smem + kTrW3 + core_off(n, k, kH)) = w3;
   }
   for (int i = t; i < kH; i += blockDim.x) {
     sb[0][i] = net.p[kOffB1 + i];
@@ -233,12 +243,15 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
   double loss = 0.0;
   bool first = true;  // no accumulation into D yet
 
-  // issue (thread 0), commit, and wait for the MMAs of one step
-  auto run = [&](auto issue) -> bool {
+  // issue (thread 0), commit, and wait for the MMAs of one step; the MMAs of
+  // `rest` follow the commit and run beside the next epilogue (the next step's
+  // commit covers them, and until then nothing writes their operands)
+  auto run = [&](auto issue, auto rest) -> bool {
     if (t == 0) {
       fence_after_sync();
       issue();
       mma_commit(mb);
+      rest();
     }
     const bool got = mbar_wait(mb, phase, net.wait_polls);
     phase ^= 1u;
@@ -288,7 +301,7 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
         const Opnd A = l == 0 ? k_major(aX, kTrN1) : l == 1 ? k_major(aH1, kTrN2) : k_major(aH2, kTrN3);
         const Opnd B = l == 0 ? k_major(aW1, kInPad) : l == 1 ? k_major(aW2, kH) : k_major(aW3, kH);
         mma_steps(zc, A, B, K, kIdF, false);
-      });
+      }, [] {});
       if (!ok) break;
       float d[16];
       tmem_ld16(tl + (uint32_t)(kTmZ1 + 64 * l + cc), d);
@@ -336,8 +349,7 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
     }
     publish();
     if (t == 0) loss += (double)(sred[0] + sred[1] + sred[2] + sred[3]) * inv_batch;
-    ok = run([&] {
-      mma_steps(tmem + kTmZ3, k_major(aDZ3, kTrWZ3), mn_major(aW3, kH), kH, kIdH, false);
+    ok = run([&] { mma_steps(tmem + kTmZ3, k_major(aDZ3, kTrWZ3), mn_major(aW3, kH), kH, kIdH, false); }, [&] {
       mma_steps(tmem + kTmD3, mn_major(aDZ3, kTrWZ3), mn_major(aH2, kTrN3), kTrK, idesc_tr(kTile, kTrN3, true, true),
                 !first);
     });
@@ -359,8 +371,7 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
       }
       publish();
       if (l == 1)
-        ok = run([&] {
-          mma_steps(tmem + kTmZ2, k_major(aDZ2, kH), mn_major(aW2, kH), kH, kIdH, false);
+        ok = run([&] { mma_steps(tmem + kTmZ2, k_major(aDZ2, kH), mn_major(aW2, kH), kH, kIdH, false); }, [&] {
           mma_steps(tmem + kTmD2, mn_major(aDZ2, kH), mn_major(aH1, kTrN2), kTrK, idesc_tr(kTile, kTrN2, true, true),
                     !first);
         });
@@ -368,7 +379,7 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
         ok = run([&] {
           mma_steps(tmem + kTmD1, mn_major(aDZ1, kH), mn_major(aX, kTrN1), kTrK, idesc_tr(kTile, kTrN1, true, true),
                     !first);
-        });
+        }, [] {});
     }
     first = false;
   }
@@ -397,9 +408,13 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
     for (int i = t; i < kParams; i += blockDim.x) g[i] = 0.f;
   }
   if (t == 0) ploss[blockIdx.x] = loss;
-  // after a timed-out wait, the MMAs of that commit may still be running:
-  // wait for them (bounded) before the columns are freed
-  if (!ok) mbar_wait(mb, phase ^ 1u, kWaitPolls);
+  // after a timed-out wait, the MMAs of that commit, and those issued after it,
+  // may still be running: wait for them (bounded) before the columns are freed
+  if (!ok) {
+    mbar_wait(mb, phase ^ 1u, kWaitPolls);
+    if (t == 0) mma_commit(mb);
+    mbar_wait(mb, phase, kWaitPolls);
+  }
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
