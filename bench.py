@@ -169,29 +169,39 @@ def measured_peaks():
 # path, FP64 otherwise); gd is FP64 in both paths.  The layouts are those of
 # tmcore_gb300/csrc (structure of arrays, int32 indices, int8 signs).
 # ---------------------------------------------------------------------------
-def flux_kernel_bytes(nc: int, ne: int, S: int, mode: int | None = None) -> float:
+def flux_kernel_bytes(nc: int, ne: int, S: int, mode: int | None = None, ntr: int = 0) -> float:
     """k_edge_flux: edgesOnEdge 40, weightsOnEdge 10 Mw, cellsOnEdge 8, dcEdge Mw;
-    pv_e, u, F (FP32) or gd_edge (FP64) and own gd_edge: 4 S; RK traffic by
-    stage (1: old r, acc/tend/next w; 2,3: areaEdge, tend r+w, acc r+w, old r,
-    next w; 4: areaEdge, tend r+w, acc r+w); per cell E (S) and the gd
-    tendency (S in the FP32 path's shadow, 8 in FP64)."""
+    pv_e, u and F (FP32) or gd_edge (FP64), which the neighbours' gathers share
+    with the edge's own; RK traffic by stage (1: old r, acc w; 2: areaEdge, acc
+    r+w, tend w, old r; 3: the same and tend r; 4: areaEdge, tend r, acc r+w);
+    per cell E and the gd tendency.  FP32: the stage's gd per cell (gd_edge is
+    averaged).  FP64: 1/dcEdge, sqrt(gd_edge) and (u/2)/sqrt(gd_edge).  Stages
+    1-3 prepare the next stage's edge set: next gd per cell; FP32 u and F out;
+    FP64 dvEdge, areaEdge (stage 1) in, seven values and the tracers' terms
+    out, the tracers' ratios per cell in."""
     Mw = S
-    rk = {1: 4 * S, 2: Mw + 6 * S, 3: Mw + 6 * S, 4: Mw + 4 * S}
+    rk = {1: 2 * S, 2: Mw + 4 * S, 3: Mw + 5 * S, 4: Mw + 3 * S}
     modes = [mode] if mode else [1, 2, 3, 4]
     tot = 0.0
     for md in modes:
-        tot += ne * (40 + 10 * Mw + 8 + Mw + 4 * S + rk[md]) + nc * (S + S)
+        tot += ne * (40 + 10 * Mw + 8 + Mw + 3 * S + rk[md]) + nc * (S + S)
+        if S == 4:
+            tot += nc * S
+        else:
+            tot += ne * 3 * S
         if md <= 3:
-            # fused preparation of the next stage: next gd gathered, gd_edge/u/F
-            # written instead of the next stage's iap_u
-            tot += nc * S + ne * 2 * S
+            tot += nc * S
+            if S == 4:
+                tot += ne * 2 * S
+            else:
+                tot += ne * (Mw * (2 if md == 1 else 1) + 7 * S + ntr * S) + nc * ntr * S
     return tot / len(modes)
 
 
 def pass_bytes(nc: int, ne: int, nv: int, S: int, ntr: int, diag: bool = True) -> dict:
     """Algorithmic bytes of each pass of one CRK4 step (4 stages of cell,
     vertex, edge_pv, edge_flux with the invariants on stage 1; stages 1-3 of
-    the flux pass also prepare the next stage's gd_edge, u, F), then the final
+    the flux pass also prepare the next stage's edge set), then the final
     update of cells and of edges (which prepares the next step's first stage),
     as mean bytes per launch."""
     Mw = S
@@ -204,31 +214,37 @@ def pass_bytes(nc: int, ne: int, nv: int, S: int, ntr: int, diag: bool = True) -
         if S == 4:
             # k_cell_fast: edgesOnCell, nSign, cellsOnCell (tracers), 1/areaCell (f64 and f32), the
             # gd and ghs shadows, E out; RK of gd: old r (stages 1-3), acc r (2-4) and w, tendency
-            # shadow r (2-4) and w, areaCell_f (2-4), next gd and its shadow w (1-3); per tracer:
+            # shadow r (3-4) and w, areaCell_f (2-4), next gd and its shadow w (1-3); per tracer:
             # ratio r, mass of old r (1-3), acc r (2-4) and w, next ratio w (1-3); invariants
             # (stage 1): gd, areaCell, areaCell_f
             base = 24 + 6 + (24 if ntr else 0) + 8 + 4 + 4 + 4 + 4
-            rk_gd = {1: 32, 2: 48, 3: 48, 4: 28}[k]
+            rk_gd = {1: 32, 2: 44, 3: 48, 4: 28}[k]
             trq = {1: 16, 2: 20, 3: 20, 4: 12}[k]
             dgb = 20
+            # per edge: u, dvEdge, areaEdge; without tracers also F (with them u times the mean gd)
+            edge = 3 * S + (0 if ntr else S)
         else:
-            # k_cell<double>: nEdgesOnCell, edgesOnCell, nSign, cellsOnCell (tracers), areaCell, gd,
-            # ghs, E out; RK of gd; per tracer: mass of the stage r (= old in stage 1), old r
-            # (2-3), acc r (2-4) and w, next w (1-3)
-            base = 1 + 24 + 6 + (24 if ntr else 0) + 8 + 3 * 8
+            # k_cell<double>: nEdgesOnCell, edgesOnCell, nSign, areaCell, 1/areaCell, gd, ghs, E out;
+            # RK of gd; per tracer: old r (1-3), acc r (2-4) and w, next mass and ratio w (1-3)
+            base = 1 + 24 + 6 + 16 + 3 * 8
             rk_gd = {1: 32, 2: 48, 3: 48, 4: 32}[k]
-            trq = {1: 24, 2: 40, 3: 40, 4: 24}[k]
-            dgb = 24
-        cell += nc * (base + rk_gd + ntr * trq + (dgb if dg else 0)) + ne * (2 * S + 2 * Mw)
-        # vertex: cellsOnVertex, edgesOnVertex, kite, tSign, 1/areaTriangle, fVertex; pv out;
-        # gd and u, dcEdge gathered
-        vert += nv * (12 + 12 + 3 * Mw + 3 + Mw + Mw + S + (16 if dg else 0)) + nc * S + ne * (S + Mw)
+            trq = {1: 32, 2: 40, 3: 40, 4: 16}[k]
+            dgb = 0
+            # per edge: the flux and kinetic-energy terms, the tracers' terms
+            edge = (2 + ntr) * S
+        cell += nc * (base + rk_gd + ntr * trq + (dgb if dg else 0)) + ne * edge
+        # vertex: cellsOnVertex, edgesOnVertex, kite, tSign, 1/areaTriangle, fVertex; pv out; gd, and u
+        # and dcEdge (FP64: areaTriangle, and the product u dcEdge) gathered
+        vert += nv * (12 + 12 + 3 * Mw + 3 + (2 if S == 4 else 3) * Mw + S + (4 if dg and S == 4 else 0))
+        vert += nc * S + ne * (S + (Mw if S == 4 else 0))
         # edge_pv: verticesOnEdge; pv_e out; pv gathered
         epv += ne * (8 + S) + nv * S
-        flux += flux_kernel_bytes(nc, ne, S, k)
-    # final cells: gd r+w, acc r, shadow w; tracers r+w, acc r, shadow w
-    # final edges: iap_u r+w, acc r, cellsOnEdge, gd gathered, gd_edge/u/F written, areaEdge (energy)
-    final = nc * (24 + sh + ntr * (3 * S + sh)) + ne * (3 * S + 8 + 3 * S + Mw) + nc * S
+        flux += flux_kernel_bytes(nc, ne, S, k, ntr)
+    # final cells: gd r+w, acc r, shadow w; tracers r+w, acc r, shadow (FP64: ratio) w
+    # final edges: iap_u r+w, acc r, cellsOnEdge, gd gathered, areaEdge (energy), u and F (FP64: dvEdge,
+    # dcEdge, the ratios gathered, seven values and the tracers' terms) written
+    out = 2 * S if S == 4 else 2 * Mw + (7 + ntr) * S
+    final = nc * (24 + sh + ntr * (3 * S + (sh or 2 * S))) + ne * (3 * S + 8 + out + Mw) + nc * S
     return {"cell": cell / 4, "vertex": vert / 4, "edge_pv": epv / 4, "edge_flux": flux / 4, "final": final}
 
 
@@ -258,7 +274,10 @@ def inner_ensemble_pass_bytes(nc: int, ne: int, nv: int, members: int) -> dict:
     """Algorithmic bytes per launch of each pass of the member-innermost
     ensemble step (every array once per pass, gathers at perfect reuse),
     averaged over the four CRK4 stages: FP32 edge and vertex fields, gd and
-    its RK accumulator double-float (8 bytes), mesh tables once per pass.
+    its RK accumulator double-float (8 bytes), mesh tables once per pass.  A
+    fixed yardstick: the passes have since stopped moving gd_e, the cell pass's
+    F and the edge tendencies of stages 1 and 4 (about 15% of these bytes), so
+    a fraction by this model compares times, not DRAM throughput.
     Per member and stage (modes 1 / 2-3 / 4):
       cell   u, F 8 Ne; gd old 8, acc 8 / 16 / 8, tend 0 / 4 / 4 in, gd h, ghs 8,
              E 4, acc 8, tend 4, next gd 8 / 8 / 0 out  (+4 Nc gd l on the diag stage)
