@@ -22,10 +22,15 @@
 //               geopotential gradient, iap_u tendency (tmcore_swm_mod.F90:155-201),
 //               the RK stage update of iap_u and the CRK4 inner products
 //               (time_scheme_mod.F90:109-154)
-// Each thread handles kEPT elements (block-strided, so loads stay coalesced).
-// Global sums (beta, invariants) are per-thread sums, a warp shuffle tree and
-// a double-double combination of the warp sums per block; k_finalize reduces
-// the per-block partials in a fixed order: deterministic and compensated.
+// A step runs four of them per stage: the final update prepares the first
+// stage's edges and the flux pass those of the next stage (prep_edge); small
+// FP32 models run cell and vertex in one launch.
+// Each thread handles kEPT elements (block-strided, so loads stay coalesced),
+// one on a small mesh (Blk).  Global sums (beta, invariants) are per-thread
+// sums and one sum per block; k_finalize adds the blocks' as integers over a
+// common scale, exactly, so in any order: deterministic.  An FP32 pass at one
+// element per thread stores its elements' terms and k_finalize_products sums
+// them in the four-element launch's order.
 #pragma once
 
 #include <cstdint>
@@ -291,11 +296,16 @@ struct Blk {
   bool pdl;
   Blk(int b, int e = kEPT, bool p = false) : bs(b), ept(e), pdl(p) {}
 };
+// the kernel's side of such a launch: let the next kernel of the stream start,
+// wait for the previous one (both do nothing without the attribute)
+__device__ __forceinline__ void pdl_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <class... K, class... A>
-inline void launch(void (*kernel)(K...), int grid, const Blk& b, cudaStream_t st, A&&... args) {
+inline void launch_smem(void (*kernel)(K...), int grid, const Blk& b, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchConfig_t c{};
   c.gridDim = dim3((unsigned)grid);
   c.blockDim = dim3((unsigned)b.bs);
+  c.dynamicSmemBytes = smem;
   c.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -303,6 +313,10 @@ inline void launch(void (*kernel)(K...), int grid, const Blk& b, cudaStream_t st
   c.attrs = at;
   c.numAttrs = b.pdl ? 1 : 0;
   cudaLaunchKernelEx(&c, kernel, K(args)...);
+}
+template <class... K, class... A>
+inline void launch(void (*kernel)(K...), int grid, const Blk& b, cudaStream_t st, A&&... args) {
+  launch_smem(kernel, grid, b, 0, st, static_cast<A&&>(args)...);
 }
 
 // ---- launchers (instantiated in tmc_kernels_f64.cu / _f32.cu) ----

@@ -103,8 +103,6 @@ constexpr bool kF64 = std::is_same<T, double>::value;
 // for the previous one before they touch the state (pdl_wait), after the loads
 // of the mesh where those come first.  In a launch without the attribute both
 // do nothing.
-__device__ __forceinline__ void pdl_start() { asm volatile("griddepcontrol.launch_dependents;"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <bool kB, int EPT>
 constexpr bool kPdl = !kB && EPT == 1;
 // the state of a dependent launch is another kernel's output until pdl_wait:

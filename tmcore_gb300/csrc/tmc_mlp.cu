@@ -513,6 +513,7 @@ struct TrainSrc {
 __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train_tc(Net net, TrainSrc src, long long ntiles, float inv_batch,
                                                              float* part, double* ploss, int* err) {
   extern __shared__ __align__(128) uint8_t smem[];
+  tmc::pdl_start();
   if (!train_tiles(net, src, ntiles, inv_batch, part, ploss, smem) && threadIdx.x == 0) atomicExch(err, 1);
 }
 
@@ -564,6 +565,8 @@ __global__ void __launch_bounds__(32 * kRedChains) k_grad_adam(const float* part
                                                                float lr, float b1c, float b2c, const int* err,
                                                                double* loss) {
   const int i = blockIdx.x * 32 + (threadIdx.x & 31);
+  tmc::pdl_wait();
+  tmc::pdl_start();
   const float gi = grad_sum(part, nblk, i);
   if (blockIdx.x == 0 && threadIdx.x < 32) {
     const double l = loss_sum(ploss, nblk);
@@ -842,8 +845,8 @@ static int launch_train_tc(tmc_mlp* n, const float* X, const float* Y, long long
                            long long batch) {
   const long long ntiles = batch / kTile;
   const int grid = (int)std::min<long long>(ntiles, (long long)n->sms);
-  k_mlp_train_tc<<<grid, kTrThreads, kSmemTrain, n->st>>>(n->net(), TrainSrc{X, Y, rows, offset, n->yscale}, ntiles,
-                                                        1.f / (float)batch, n->part, n->ploss, n->d_err);
+  tmc::launch_smem(k_mlp_train_tc, grid, tmc::Blk(kTrThreads, 1, true), kSmemTrain, n->st, n->net(),
+                   TrainSrc{X, Y, rows, offset, n->yscale}, ntiles, 1.f / (float)batch, n->part, n->ploss, n->d_err);
   return grid;
 }
 
@@ -912,8 +915,8 @@ int tmc_mlp_train(tmc_mlp* n, int32_t batch, int32_t steps, float lr, float* los
       // two launches per step: the gradient tiles, then the fixed-order sum
       // of their partials with Adam
       const int grid = launch_train_tc(n, n->dx, n->dy, n->rows, n->cursor, batch);
-      k_grad_adam<<<(kParams + 31) / 32, 32 * kRedChains, 0, n->st>>>(n->part, n->ploss, grid, n->p, n->pb, n->m,
-                                                                      n->v, lr, b1c, b2c, n->d_err, dl);
+      tmc::launch(k_grad_adam, (kParams + 31) / 32, tmc::Blk(32 * kRedChains, 1, true), n->st, n->part, n->ploss,
+                  grid, n->p, n->pb, n->m, n->v, lr, b1c, b2c, n->d_err, dl);
     } else {
       cudaMemsetAsync(dl, 0, sizeof(double), n->st);
       launch_gradient(n, n->dx, n->dy, n->rows, n->cursor, batch, dl);

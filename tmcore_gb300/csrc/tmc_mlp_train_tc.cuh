@@ -82,11 +82,12 @@ constexpr int kTmZ1 = 0, kTmZ2 = 64, kTmZ3 = 128, kTmD3 = 192, kTmD2 = 352, kTmD
 constexpr int kTmCols = 512;
 static_assert(kTmD3 + kTrN3 <= kTmD2 && kTmD2 + kTrN2 <= kTmD1 && kTmD1 + kTrN1 <= kTmCols, "TMEM columns overlap");
 
-__device__ __forceinline__ float gelu_f(float z) { return gelu_tanh(z, tanh_fast(gelu_arg(z))); }
-__device__ __forceinline__ float gelu_grad_f(float z) {
+// gelu and its derivative at z share the hyperbolic tangent
+__device__ __forceinline__ float gelu_f(float z, float& grad) {
   const float c = 0.7978845608028654f;
   const float th = tanh_fast(gelu_arg(z));
-  return 0.5f * (1.f + th) + 0.5f * z * (1.f - th * th) * c * (1.f + 3.f * 0.044715f * z * z);
+  grad = 0.5f * (1.f + th) + 0.5f * z * (1.f - th * th) * c * (1.f + 3.f * 0.044715f * z * z);
+  return gelu_tanh(z, th);
 }
 
 // one BF16 value at (row n, column k) of a K-major operand with K columns
@@ -171,6 +172,35 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
   const int r = quarter * 32 + (t & 31);  // this thread's row of the tile (TMEM lane)
   const int cc = 16 * cg;                 // its first hidden column
 
+  // Everything that no earlier kernel of the step writes comes before pdl_wait:
+  // the kernel starts beside the previous step's Adam and waits for its weights.
+  for (int i = t; i < kIn; i += blockDim.x) {
+    sxm[i] = net.xmean[i];
+    sxi[i] = net.xinv[i];
+  }
+  // the constant columns of H1 and H2: ones at 64, zeros at 65..79
+  for (int i = t; i < 16 * kTile; i += blockDim.x) {
+    const int c = kH + i / kTile, row = i % kTile;
+    const float v = c == kH ? 1.f : 0.f;
+    st_bf16(sH2, row, c, kTrN3, v);
+    st_bf16(sH1, row, c, kTrN2, v);
+  }
+  const uint32_t mb = smem_u32(mbar);
+  if (t == 0) {
+    mbar_init(mb, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
+                 "r"(kTmCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  // this thread's part of the row of the block's next tile, loaded while the
+  // current one runs
+  float xr[8], xd[4], tr = 0.f;
+  bool vr = blockIdx.x < ntiles ? src.sample((long long)blockIdx.x * kTrTile + r, cg, xr, xd, tr) : false;
+  pdl_wait();
   // weights (BF16) K-major by input, eight inputs (16 bytes, one core-matrix
   // row) at a time: one load and store per thread and matrix (element by
   // element the staging was 20 dependent rounds of every launch); layer 1's
@@ -204,29 +234,7 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
     sb[2][i] = net.p[kOffB3 + i];
     sw4[i] = __bfloat162float(net.pb[kOffW4 + i]);
   }
-  for (int i = t; i < kIn; i += blockDim.x) {
-    sxm[i] = net.xmean[i];
-    sxi[i] = net.xinv[i];
-  }
-  // the constant columns of H1 and H2: ones at 64, zeros at 65..79
-  for (int i = t; i < 16 * kTile; i += blockDim.x) {
-    const int c = kH + i / kTile, row = i % kTile;
-    const float v = c == kH ? 1.f : 0.f;
-    st_bf16(sH2, row, c, kTrN3, v);
-    st_bf16(sH1, row, c, kTrN2, v);
-  }
   const float b4 = net.p[kOffB4];
-  const uint32_t mb = smem_u32(mbar);
-  if (t == 0) {
-    mbar_init(mb, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
-                 "r"(kTmCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
   fence_async_smem();
   fence_before_sync();
   __syncthreads();
@@ -267,10 +275,6 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
     __syncthreads();
   };
 
-  // this thread's part of the row of the block's next tile, loaded while the
-  // current one runs
-  float xr[8], xd[4], tr = 0.f;
-  bool vr = blockIdx.x < ntiles ? src.sample((long long)blockIdx.x * kTrTile + r, cg, xr, xd, tr) : false;
   for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
     const float tgt = vr ? tr : 0.f;
     const float dir = vr ? head_dir4(net, xd[0], xd[1], xd[2], xd[3]) : 0.f;  // raw features
@@ -291,9 +295,12 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
       const long long nt = tile + gridDim.x;
       vr = nt < ntiles ? src.sample(nt * kTrTile + r, cg, xr, xd, tr) : false;
     }
-    // forward
-#pragma unroll 1
-    for (int l = 0; l < 3 && ok; ++l) {
+    // forward; the derivatives of the thread's 3 x 16 activations stay in
+    // registers for the backward (read back from TMEM as pre-activations, they
+    // cost a second tanh each and a TMEM round trip per layer)
+    float gp[3][16];
+#pragma unroll
+    for (int l = 0; l < 3; ++l) {
       const int K = l == 0 ? kInPad : kH;
       const uint32_t zc = tmem + (uint32_t)(kTmZ1 + 64 * l);
       // A the previous layer K-major, B the weights K-major
@@ -310,7 +317,7 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const float z = l == 0 ? d[i] : d[i] + sb[l][cc + i];
-        h[i] = __bfloat162float(__float2bfloat16_rn(gelu_f(z)));
+        h[i] = __bfloat162float(__float2bfloat16_rn(gelu_f(z, gp[l][i])));
       }
       // H1 -> sH1, H2 -> sH2 (columns 0..63), H3 -> sH2 (columns 80..143)
       uint8_t* const hb = l == 0 ? sH1 : sH2;
@@ -339,11 +346,9 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
     }
     // dZ3 = dy w4 gelu'(z3)
     {
-      float d[16], g[16];
-      tmem_ld16(tl + (uint32_t)(kTmZ3 + cc), d);
-      tmem_wait_ld();
+      float g[16];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) g[i] = dy * sw4[cc + i] * gelu_grad_f(d[i] + sb[2][cc + i]);
+      for (int i = 0; i < 16; ++i) g[i] = dy * sw4[cc + i] * gp[2][i];
       store8_bf16(sDZ3, r, cc, kTrWZ3, g);
       store8_bf16(sDZ3, r, cc + 8, kTrWZ3, g + 8);
     }
@@ -355,16 +360,15 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
     });
     if (!ok) break;
     // dZ2 = dH2 gelu'(z2), dZ1 = dH1 gelu'(z1)
-#pragma unroll 1
-    for (int l = 1; l >= 0 && ok; --l) {
-      const uint32_t dh = (uint32_t)(kTmZ1 + 64 * (l + 1)), zc = (uint32_t)(kTmZ1 + 64 * l);
+#pragma unroll
+    for (int l = 1; l >= 0; --l) {
+      const uint32_t dh = (uint32_t)(kTmZ1 + 64 * (l + 1));
       {
-        float d[16], z[16], g[16];
+        float d[16], g[16];
         tmem_ld16(tl + dh + cc, d);
-        tmem_ld16(tl + zc + cc, z);
         tmem_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) g[i] = d[i] * gelu_grad_f(l == 0 ? z[i] : z[i] + sb[l][cc + i]);
+        for (int i = 0; i < 16; ++i) g[i] = d[i] * gp[l][i];
         uint8_t* const gz = l == 1 ? sDZ2 : sDZ1;
         store8_bf16(gz, r, cc, kH, g);
         store8_bf16(gz, r, cc + 8, kH, g + 8);
@@ -380,6 +384,7 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
           mma_steps(tmem + kTmD1, mn_major(aDZ1, kH), mn_major(aX, kTrN1), kTrK, idesc_tr(kTile, kTrN1, true, true),
                     !first);
         }, [] {});
+      if (!ok) break;
     }
     first = false;
   }
