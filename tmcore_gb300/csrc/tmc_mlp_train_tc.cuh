@@ -56,7 +56,8 @@ constexpr int kTrX = kTrH1 + kTile * kTrN2 * 2;      // [128][32]: X, 1, 1, 0
 constexpr int kTrDZ3 = kTrX + kTile * kTrN1 * 2;     // [128][72]: dZ3, dy, 7 unused
 constexpr int kTrDZ2 = kTrDZ3 + kTile * kTrWZ3 * 2;  // [128][64]
 constexpr int kTrDZ1 = kTrDZ2 + kTile * kH * 2;      // [128][64]
-constexpr int kTrBar = kTrDZ1 + kTile * kH * 2;      // mbarrier (8 B) and the TMEM address (4 B)
+constexpr int kTrX2 = kTrDZ1 + kTile * kH * 2;       // the second X: tiles alternate
+constexpr int kTrBar = kTrX2 + kTile * kTrN1 * 2;    // mbarrier (8 B) and the TMEM address (4 B)
 // Furthest byte an MN-major read of the operand at `base` (width w columns,
 // MN extent e, k16 steps of 16 K-rows) reaches: with the core-matrix strides
 // as mn_major sets them (K: 16 w bytes per 8 rows; M or N: 128 bytes per 8
@@ -74,7 +75,7 @@ constexpr int kSmemTrain =
     tr_max(tr_max(tr_max(kTrBar + 16, tr_reach(kTrDZ3, kTrWZ3, 128, 8)),
                   tr_max(tr_reach(kTrDZ2, kH, 128, 8), tr_reach(kTrDZ1, kH, 128, 8))),
            tr_max(tr_max(tr_reach(kTrH2, kTrN3, kTrN3, 8), tr_reach(kTrH1, kTrN2, kTrN2, 8)),
-                  tr_max(tr_reach(kTrX, kTrN1, kTrN1, 8), tr_reach(kTrW3, kH, kH, 4))));
+                  tr_max(tr_reach(kTrX2, kTrN1, kTrN1, 8), tr_reach(kTrW3, kH, kH, 4))));
 static_assert(kSmemTrain <= 227 * 1024, "training tile does not fit in shared memory");
 // TMEM columns: the three pre-activations (then the dH), and the three
 // weight-gradient accumulators
@@ -156,7 +157,6 @@ __device__ __forceinline__ void store_dw(uint32_t tl, int m, int cg, int nin, in
 template <class Src>
 __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, float inv_batch, float* part,
                             double* ploss, uint8_t* smem) {
-  uint8_t* const sX = smem + kTrX;
   uint8_t* const sH1 = smem + kTrH1;
   uint8_t* const sH2 = smem + kTrH2;
   uint8_t* const sDZ3 = smem + kTrDZ3;
@@ -241,7 +241,7 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
   fence_after_sync();
   const uint32_t tmem = *tslot;
   const uint32_t tl = tmem + ((uint32_t)(quarter * 32) << 16);  // this warp's lane quarter
-  const uint32_t aX = smem_u32(sX), aH1 = smem_u32(sH1), aH2 = smem_u32(sH2);
+  const uint32_t aX = smem_u32(smem + kTrX), aH1 = smem_u32(sH1), aH2 = smem_u32(sH2);
   const uint32_t aDZ3 = smem_u32(sDZ3), aDZ2 = smem_u32(sDZ2), aDZ1 = smem_u32(sDZ1);
   const uint32_t aW1 = smem_u32(smem + kTrW1), aW2 = smem_u32(smem + kTrW2), aW3 = smem_u32(smem + kTrW3);
   constexpr uint32_t kIdF = idesc_tr(kTile, kH, false, false);
@@ -249,18 +249,20 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
   uint32_t phase = 0;
   bool ok = true;
   double loss = 0.0;
-  bool first = true;  // no accumulation into D yet
+  int done = 0;  // tiles of this block whose D2 and D3 products are issued
 
   // issue (thread 0), commit, and wait for the MMAs of one step; the MMAs of
   // `rest` follow the commit and run beside the next epilogue (the next step's
-  // commit covers them, and until then nothing writes their operands)
-  auto run = [&](auto issue, auto rest) -> bool {
+  // commit covers them, and until then nothing writes their operands).  Every
+  // thread does `beside` before it waits.
+  auto run = [&](auto issue, auto rest, auto beside) -> bool {
     if (t == 0) {
       fence_after_sync();
       issue();
       mma_commit(mb);
       rest();
     }
+    beside();
     const bool got = mbar_wait(mb, phase, net.wait_polls);
     phase ^= 1u;
     const bool all = __syncthreads_and(got) != 0;
@@ -275,22 +277,37 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
     __syncthreads();
   };
 
-  for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-    const float tgt = vr ? tr : 0.f;
-    const float dir = vr ? head_dir4(net, xd[0], xd[1], xd[2], xd[3]) : 0.f;  // raw features
-    {
-      // the row's 32 input columns are 24 normalised features, 2 ones and 6
-      // zeros; this thread stores columns 8 cg .. 8 cg + 7
-      float v[8];
+  // the row's 32 input columns are 24 normalised features, 2 ones and 6 zeros;
+  // this thread stores columns 8 cg .. 8 cg + 7, and keeps the target and the
+  // head's direction (from raw features)
+  float tgt = 0.f, dir = 0.f;
+  auto put_row = [&](uint8_t* sX) {
+    tgt = vr ? tr : 0.f;
+    dir = vr ? head_dir4(net, xd[0], xd[1], xd[2], xd[3]) : 0.f;
+    float v[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] = k < 2 ? 1.f : 0.f;  // column group 3
-      if (cg < 3) {
+    for (int k = 0; k < 8; ++k) v[k] = k < 2 ? 1.f : 0.f;  // column group 3
+    if (cg < 3) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = vr ? (xr[k] - sxm[8 * cg + k]) * sxi[8 * cg + k] : 0.f;
-      }
-      store8_bf16(sX, r, 8 * cg, kInPad, v);
+      for (int k = 0; k < 8; ++k) v[k] = vr ? (xr[k] - sxm[8 * cg + k]) * sxi[8 * cg + k] : 0.f;
     }
-    publish();
+    store8_bf16(sX, r, 8 * cg, kInPad, v);
+  };
+  auto nothing = [] {};
+  // the layer-1 weight-gradient product of the tile whose X is at offset b
+  auto d1 = [&](uint32_t b, bool accumulate) {
+    mma_steps(tmem + kTmD1, mn_major(aDZ1, kH), mn_major(aX + b, kTrN1), kTrK, idesc_tr(kTile, kTrN1, true, true),
+              accumulate);
+  };
+  constexpr uint32_t kXStep = kTrX2 - kTrX;
+  uint32_t xb = 0;  // offset of this tile's X buffer: 0 or kXStep
+  put_row(smem + kTrX);
+  publish();
+  // A tile waits for five products: three forward, dH2 and dH1.  The weight
+  // gradients run beside what follows them (D1 beside the next tile's first
+  // layer), and the next tile's inputs are stored beside dH2, so that a tile
+  // begins with its first product.
+  for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
     {
       const long long nt = tile + gridDim.x;
       vr = nt < ntiles ? src.sample(nt * kTrTile + r, cg, xr, xd, tr) : false;
@@ -305,10 +322,12 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
       const uint32_t zc = tmem + (uint32_t)(kTmZ1 + 64 * l);
       // A the previous layer K-major, B the weights K-major
       ok = run([&] {
-        const Opnd A = l == 0 ? k_major(aX, kTrN1) : l == 1 ? k_major(aH1, kTrN2) : k_major(aH2, kTrN3);
+        const Opnd A = l == 0 ? k_major(aX + xb, kTrN1) : l == 1 ? k_major(aH1, kTrN2) : k_major(aH2, kTrN3);
         const Opnd B = l == 0 ? k_major(aW1, kInPad) : l == 1 ? k_major(aW2, kH) : k_major(aW3, kH);
         mma_steps(zc, A, B, K, kIdF, false);
-      }, [] {});
+      }, [&] {
+        if (l == 0 && done > 0) d1(kXStep - xb, done > 1);
+      }, nothing);
       if (!ok) break;
       float d[16];
       tmem_ld16(tl + (uint32_t)(kTmZ1 + 64 * l + cc), d);
@@ -356,8 +375,8 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
     if (t == 0) loss += (double)(sred[0] + sred[1] + sred[2] + sred[3]) * inv_batch;
     ok = run([&] { mma_steps(tmem + kTmZ3, k_major(aDZ3, kTrWZ3), mn_major(aW3, kH), kH, kIdH, false); }, [&] {
       mma_steps(tmem + kTmD3, mn_major(aDZ3, kTrWZ3), mn_major(aH2, kTrN3), kTrK, idesc_tr(kTile, kTrN3, true, true),
-                !first);
-    });
+                done > 0);
+    }, [&] { put_row(smem + kTrX + (kXStep - xb)); });
     if (!ok) break;
     // dZ2 = dH2 gelu'(z2), dZ1 = dH1 gelu'(z1)
 #pragma unroll
@@ -374,23 +393,22 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
         store8_bf16(gz, r, cc + 8, kH, g + 8);
       }
       publish();
-      if (l == 1)
+      if (l == 1) {
         ok = run([&] { mma_steps(tmem + kTmZ2, k_major(aDZ2, kH), mn_major(aW2, kH), kH, kIdH, false); }, [&] {
           mma_steps(tmem + kTmD2, mn_major(aDZ2, kH), mn_major(aH1, kTrN2), kTrK, idesc_tr(kTile, kTrN2, true, true),
-                    !first);
-        });
-      else
-        ok = run([&] {
-          mma_steps(tmem + kTmD1, mn_major(aDZ1, kH), mn_major(aX, kTrN1), kTrK, idesc_tr(kTile, kTrN1, true, true),
-                    !first);
-        }, [] {});
-      if (!ok) break;
+                    done > 0);
+        }, nothing);
+        if (!ok) break;
+      }
     }
-    first = false;
+    if (!ok) break;
+    ++done;
+    xb = kXStep - xb;
   }
+  if (ok && done > 0) ok = run([&] { d1(kXStep - xb, done > 1); }, nothing, nothing);
   // the block's partial gradient (zeros when it had no tile) and loss
   float* const g = part + (size_t)blockIdx.x * kParams;
-  if (ok && !first) {
+  if (ok && done > 0) {
     store_dw(tl + kTmD3, r, cg, kH, kH, g + kOffW3, g + kOffB3);
     store_dw(tl + kTmD2, r, cg, kH, kH, g + kOffW2, g + kOffB2);
     store_dw(tl + kTmD1, r, cg, kIn, kIn, g + kOffW1, g + kOffB1);
