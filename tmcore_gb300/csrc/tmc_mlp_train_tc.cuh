@@ -38,7 +38,9 @@
 // 56.5 us with each tanh formed again in the backward from Z in TMEM and
 // launches one after another, 42.5 with the derivatives in registers and
 // dependent launches, 41.9 with D1 and the next tile's inputs beside other
-// products.
+// products, 39.9 with Adam's loads together, 38.1 without a block barrier after
+// each wait (publish carries the outcome) and the next rows' loads beside the
+// first product.
 #pragma once
 
 #include "tmc_mlp_tc.cuh"
@@ -263,7 +265,9 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
   // issue (thread 0), commit, and wait for the MMAs of one step; the MMAs of
   // `rest` follow the commit and run beside the next epilogue (the next step's
   // commit covers them, and until then nothing writes their operands).  Every
-  // thread does `beside` before it waits.
+  // thread does `beside` before it waits.  Whether the wait ended in time is the
+  // warp's own answer (a warp whose wait ran out leaves its epilogue out); the
+  // next publish makes it the block's.
   auto run = [&](auto issue, auto rest, auto beside) -> bool {
     if (t == 0) {
       fence_after_sync();
@@ -272,18 +276,17 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
       rest();
     }
     beside();
-    const bool got = mbar_wait(mb, phase, net.wait_polls);
+    const bool got = __all_sync(0xffffffffu, mbar_wait(mb, phase, net.wait_polls)) != 0;
     phase ^= 1u;
-    const bool all = __syncthreads_and(got) != 0;
     fence_after_sync();
-    return all;
+    return got;
   };
   // make this thread's shared-memory operand writes and TMEM reads visible
-  // before the next MMA
-  auto publish = [&]() {
+  // before the next MMA; true if every thread's last wait ended in time
+  auto publish = [&](bool got) -> bool {
     fence_async_smem();
     fence_before_sync();
-    __syncthreads();
+    return __syncthreads_and(got) != 0;
   };
 
   // the row's 32 input columns are 24 normalised features, 2 ones and 6 zeros;
@@ -311,16 +314,12 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
   constexpr uint32_t kXStep = kTrX2 - kTrX;
   uint32_t xb = 0;  // offset of this tile's X buffer: 0 or kXStep
   put_row(smem + kTrX);
-  publish();
+  publish(true);
   // A tile waits for five products: three forward, dH2 and dH1.  The weight
   // gradients run beside what follows them (D1 beside the next tile's first
   // layer), and the next tile's inputs are stored beside dH2, so that a tile
   // begins with its first product.
   for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-    {
-      const long long nt = tile + gridDim.x;
-      vr = nt < ntiles ? src.sample(nt * kTrTile + r, cg, xr, xd, tr) : false;
-    }
     // forward; the derivatives of the thread's 3 x 16 activations stay in
     // registers for the backward (read back from TMEM as pre-activations, they
     // cost a second tanh each and a TMEM round trip per layer)
@@ -330,35 +329,40 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
       const int K = l == 0 ? kInPad : kH;
       const uint32_t zc = tmem + (uint32_t)(kTmZ1 + 64 * l);
       // A the previous layer K-major, B the weights K-major
-      ok = run([&] {
+      const bool got = run([&] {
         const Opnd A = l == 0 ? k_major(aX + xb, kTrN1) : l == 1 ? k_major(aH1, kTrN2) : k_major(aH2, kTrN3);
         const Opnd B = l == 0 ? k_major(aW1, kInPad) : l == 1 ? k_major(aW2, kH) : k_major(aW3, kH);
         mma_steps(zc, A, B, K, kIdF, false);
       }, [&] {
         if (l == 0 && done > 0) d1(kXStep - xb, done > 1);
-      }, nothing);
+      }, [&] {
+        const long long nt = tile + gridDim.x;
+        if (l == 0) vr = nt < ntiles ? src.sample(nt * kTrTile + r, cg, xr, xd, tr) : false;
+      });
+      if (got) {
+        float d[16];
+        tmem_ld16(tl + (uint32_t)(kTmZ1 + 64 * l + cc), d);
+        tmem_wait_ld();
+        float h[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float z = l == 0 ? d[i] : d[i] + sb[l][cc + i];
+          h[i] = __bfloat162float(__float2bfloat16_rn(gelu_f(z, gp[l][i])));
+        }
+        // H1 -> sH1, H2 -> sH2 (columns 0..63), H3 -> sH2 (columns 80..143)
+        uint8_t* const hb = l == 0 ? sH1 : sH2;
+        const int hw = l == 0 ? kTrN2 : kTrN3, c0 = (l == 2 ? kTrH3Col : 0) + cc;
+        store8_bf16(hb, r, c0, hw, h);
+        store8_bf16(hb, r, c0 + 8, hw, h + 8);
+        if (l == 2) {
+          float yp = 0.f;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) yp += sw4[cc + i] * h[i];
+          sy[cg][r] = yp;
+        }
+      }
+      ok = publish(got);
       if (!ok) break;
-      float d[16];
-      tmem_ld16(tl + (uint32_t)(kTmZ1 + 64 * l + cc), d);
-      tmem_wait_ld();
-      float h[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const float z = l == 0 ? d[i] : d[i] + sb[l][cc + i];
-        h[i] = __bfloat162float(__float2bfloat16_rn(gelu_f(z, gp[l][i])));
-      }
-      // H1 -> sH1, H2 -> sH2 (columns 0..63), H3 -> sH2 (columns 80..143)
-      uint8_t* const hb = l == 0 ? sH1 : sH2;
-      const int hw = l == 0 ? kTrN2 : kTrN3, c0 = (l == 2 ? kTrH3Col : 0) + cc;
-      store8_bf16(hb, r, c0, hw, h);
-      store8_bf16(hb, r, c0 + 8, hw, h + 8);
-      if (l == 2) {
-        float yp = 0.f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) yp += sw4[cc + i] * h[i];
-        sy[cg][r] = yp;
-      }
-      publish();
     }
     if (!ok) break;
     // output head and loss (every thread of the row forms the same y)
@@ -380,18 +384,19 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
       store8_bf16(sDZ3, r, cc, kTrWZ3, g);
       store8_bf16(sDZ3, r, cc + 8, kTrWZ3, g + 8);
     }
-    publish();
-    if (t == 0) loss += (double)(sred[0] + sred[1] + sred[2] + sred[3]) * inv_batch;
-    ok = run([&] { mma_steps(tmem + kTmZ3, k_major(aDZ3, kTrWZ3), mn_major(aW3, kH), kH, kIdH, false); }, [&] {
+    publish(true);
+    bool got = run([&] { mma_steps(tmem + kTmZ3, k_major(aDZ3, kTrWZ3), mn_major(aW3, kH), kH, kIdH, false); }, [&] {
       mma_steps(tmem + kTmD3, mn_major(aDZ3, kTrWZ3), mn_major(aH2, kTrN3), kTrK, idesc_tr(kTile, kTrN3, true, true),
                 done > 0);
-    }, [&] { put_row(smem + kTrX + (kXStep - xb)); });
-    if (!ok) break;
+    }, [&] {
+      if (t == 0) loss += (double)(sred[0] + sred[1] + sred[2] + sred[3]) * inv_batch;
+      put_row(smem + kTrX + (kXStep - xb));
+    });
     // dZ2 = dH2 gelu'(z2), dZ1 = dH1 gelu'(z1)
 #pragma unroll
     for (int l = 1; l >= 0; --l) {
       const uint32_t dh = (uint32_t)(kTmZ1 + 64 * (l + 1));
-      {
+      if (got) {
         float d[16], g[16];
         tmem_ld16(tl + dh + cc, d);
         tmem_wait_ld();
@@ -401,20 +406,19 @@ __device__ bool train_tiles(const Net& net, const Src& src, long long ntiles, fl
         store8_bf16(gz, r, cc, kH, g);
         store8_bf16(gz, r, cc + 8, kH, g + 8);
       }
-      publish();
-      if (l == 1) {
-        ok = run([&] { mma_steps(tmem + kTmZ2, k_major(aDZ2, kH), mn_major(aW2, kH), kH, kIdH, false); }, [&] {
+      ok = publish(got);
+      if (!ok) break;
+      if (l == 1)
+        got = run([&] { mma_steps(tmem + kTmZ2, k_major(aDZ2, kH), mn_major(aW2, kH), kH, kIdH, false); }, [&] {
           mma_steps(tmem + kTmD2, mn_major(aDZ2, kH), mn_major(aH1, kTrN2), kTrK, idesc_tr(kTile, kTrN2, true, true),
                     done > 0);
         }, nothing);
-        if (!ok) break;
-      }
     }
     if (!ok) break;
     ++done;
     xb = kXStep - xb;
   }
-  if (ok && done > 0) ok = run([&] { d1(kXStep - xb, done > 1); }, nothing, nothing);
+  if (ok && done > 0) ok = __syncthreads_and(run([&] { d1(kXStep - xb, done > 1); }, nothing, nothing)) != 0;
   // the block's partial gradient (zeros when it had no tile) and loss
   float* const g = part + (size_t)blockIdx.x * kParams;
   if (ok && done > 0) {
