@@ -6,7 +6,8 @@
 // busy with DRAM at 11-13% of peak), so here everything that an exponent or a
 // sign bit can express is done on the integer units, and quotients by a
 // divisor whose reciprocal is at hand cost three FP64 instructions.  Results
-// are those of IEEE division, square root and multiplication bit for bit.
+// are those of IEEE division, square root and multiplication bit for bit; the
+// reasons stand at div_r and sqrt_r.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -43,30 +44,60 @@ __device__ __forceinline__ double with_sign(double x, int sign) {
   return __hiloint2double(__double2hiint(x) ^ (sign & 0x80000000), __double2loint(x));
 }
 
-// a / b rounded to nearest from r = RN(1/b): quotient estimate, its exact
-// residual by FMA, one correction (Markstein 1990; Brisebarre, Muller and
-// Raina 2004 prove the form for a divisor known in advance).  Outside the
-// range where the residual is exact (zeros, infinities, NaN, extreme
-// exponents) the plain division.
+// a / b rounded to nearest from r = RN(1/b), or from r = 0 (which makes it
+// divide): quotient estimate q, its residual by FMA, one correction (Markstein
+// 1990; Brisebarre, Muller and Raina 2004 for a divisor known in advance).
+// Why, in units in the last place of q: with the mantissas of b and r as
+// integers B and R, B R = 2^105 + h with |h| <= B/2 (h = 0 for a power of two).
+// The corrected value, before its rounding, is off a/b by |a/b - q| |h| / 2^105,
+// at most 1.5 2^-53.  a/b itself is a midpoint plus N / (2 B), N a nonzero
+// integer, so only |N| <= 2 could round the wrong way.  So near a midpoint q is
+// one of its two neighbours, |a/b - q| is a half, and the deviation at most
+// B/4 2^-105 < 1 / (2 B) stays on the quotient's side.
+// That needs r correctly rounded: with the reciprocal one unit off, 1 / (2 -
+// 2^-52) comes out one unit off.  Outside the range where the residual is
+// exact (zeros, infinities, NaN, extreme exponents) the plain division.
 __device__ __forceinline__ double div_r(double a, double b, double r) {
   const double q = __dmul_rn(a, r);
   if (mid(q)) return __fma_rn(__fma_rn(-q, b, a), r, q);
   return a / b;
 }
 
-// 1/b for div_r: Newton iterations from the 20-bit hardware estimate
+// y if it is 1/b rounded to nearest, else 0, for y within a few units of 1/b.
+// A Newton iteration ends within 2^-80 of 1/b before its rounding and so may
+// round the other way where 1/b is next to a midpoint.  With the mantissas as
+// integers the product's distance from the power of two is its low 64 bits:
+// 14 integer instructions, where a residual in FP64 would hold the pipe for 64
+// cycles.  (Where y is a power of two and b is not, the distance is 2^52 or
+// more, above B/2: the closer spacing below y needs no case.)
+__device__ __forceinline__ double nearest_or_zero(double b, double y) {
+  auto mantissa = [](double x) {
+    return (unsigned long long)(unsigned)((__double2hiint(x) & 0xfffff) | 0x100000) << 32 |
+           (unsigned)__double2loint(x);
+  };
+  const unsigned long long B = mantissa(b);
+  const long long h = (long long)(B * mantissa(y));
+  return 2 * (unsigned long long)(h < 0 ? -h : h) <= B ? y : 0.0;
+}
+
+// 1/b rounded to nearest for div_r, or 0: Newton iterations from the 20-bit
+// hardware estimate
 __device__ __forceinline__ double recip(double b) {
   if (!mid(b)) return 0.0;
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
   y = __fma_rn(__fma_rn(-b, y, 1.0), y, y);
-  return __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+  return nearest_or_zero(b, __fma_rn(__fma_rn(-b, y, 1.0), y, y));
 }
 
-// s = sqrt(a) rounded to nearest and r = 1/s (for div_r): coupled iteration
-// (Goldschmidt 1964) from the hardware's reciprocal square root estimate, g
-// -> sqrt(a), h -> 1/(2 sqrt(a)), and one residual correction of g
-// (Markstein 1990)
+// s = sqrt(a) rounded to nearest and r = 1/s rounded to nearest, or 0 (for
+// div_r): coupled iteration (Goldschmidt 1964) from the hardware's reciprocal
+// square root estimate, g -> sqrt(a), h -> 1/(2 sqrt(a)), and one residual
+// correction of g (Markstein 1990).  g and h end within 2^-52 (relative), so
+// the corrected root is within 2^-50 units in the last place of sqrt(a) before
+// its rounding.  A root that near a midpoint m (54 bits) has a 2^s = m^2 - c
+// with |c| <= 64: some 25 mantissas, for which (and for 150 more) equality
+// with the IEEE square root is tested.
 struct SqrtR {
   double s, r;
 };
@@ -84,7 +115,7 @@ __device__ __forceinline__ SqrtR sqrt_r(double a) {
   h = __fma_rn(h, e, h);
   const double s = __fma_rn(__fma_rn(-g, g, a), h, g);
   y = __hiloint2double(__double2hiint(h) + 0x00100000, __double2loint(h));
-  return {s, __fma_rn(__fma_rn(-s, y, 1.0), y, y)};
+  return {s, nearest_or_zero(s, __fma_rn(__fma_rn(-s, y, 1.0), y, y))};
 }
 
 // ---------------------------------------------------------------------------
