@@ -964,9 +964,10 @@ __global__ void __launch_bounds__(kMaxBS) k_ens_edges(DevMesh Mh, Dims D, IO S, 
 
 // ---------------------------------------------------------------------------
 // reduction of the per-thread partials: block = (region, group of 32
-// members), warp w sums slots w, w + W, ... for its 32 members (FP32 TwoSum
-// for the step products, FP64 for the invariants), the warps' sums of each
-// member are added and stored after the member's kDiagLen outputs.
+// members), warp w sums slots w, w + W, ... for its 32 members into four
+// accumulators (FP32 TwoSum for the step products, FP64 for the invariants),
+// the warps' accumulators of each member are added and the sum stored after
+// the member's kDiagLen outputs.
 // ---------------------------------------------------------------------------
 struct RegionList {
   int n;
@@ -976,57 +977,68 @@ struct RegionList {
 
 // One block per (region, group of 32 members), 32 warps: warp w takes slots
 // w, w + 32, ... in rounds of four with four independent accumulators (all
-// four loads in flight), which it adds in a fixed order; then warp m adds the
-// warps' sums of member m, as exact integers (f64::warp_sum).  Deterministic
-// for a given slot count.  The block is bound by FP64 instructions (64 cycles
-// each, warp-wide): combining the accumulators and the warps in double-double
-// took 36.9 us for 64 level-6 members, plain FP64 sums of four and the integer
-// sum across warps take 14.5 us.  (With 8 warps and one accumulator the 7,680
-// slots of a level-7 edge region took about 0.3 ms, a quarter of a 16-member
-// step.)
+// four loads in flight); then warp m adds the warps' accumulators of member m
+// as exact integers (f64::warp_sum).  Deterministic for a given slot count.  The
+// block is bound by FP64 instructions (64 cycles each, warp-wide): combining
+// the accumulators and the warps in double-double took 36.9 us for 64 level-6
+// members, the integer sum takes 14.0 us.  (With 8 warps and one accumulator the
+// 7,680 slots of a level-7 edge region took about 0.3 ms, a quarter of a
+// 16-member step.)
 constexpr int kRedThreads = 1024;
 __device__ __forceinline__ void ens_reduce(const Partials& P, int r, int count, double* diag_out) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   constexpr int nw = kRedThreads / 32;
   const int m = blockIdx.y * 32 + lane;
-  double acc = 0.0;
-  if (m < P.M) {
-    if (r <= R_44_E) {
-      float fh[4] = {0.f, 0.f, 0.f, 0.f}, fl[4] = {0.f, 0.f, 0.f, 0.f};
-      int s = w;
-      for (; s + 3 * nw < count; s += 4 * nw) {
-        float v[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = P.f(r, s + q * nw)[m];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) two_sum_acc(fh[q], fl[q], v[q]);
-      }
-#pragma unroll
-      for (int q = 0; q < 3; ++q)  // the last at most 3 slots of this warp
-        if (s + q * nw < count) two_sum_acc(fh[q], fl[q], P.f(r, s + q * nw)[m]);
-      acc = ((widen(fh[0]) + widen(fh[1])) + (widen(fh[2]) + widen(fh[3]))) +
-            ((widen(fl[0]) + widen(fl[1])) + (widen(fl[2]) + widen(fl[3])));
-    } else {
-      double dh[4] = {0.0, 0.0, 0.0, 0.0};
-      int s = w;
-      for (; s + 3 * nw < count; s += 4 * nw) {
-        double v[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = P.d(r, s + q * nw)[m];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) dh[q] += v[q];
-      }
-#pragma unroll
-      for (int q = 0; q < 3; ++q)
-        if (s + q * nw < count) dh[q] += P.d(r, s + q * nw)[m];
-      acc = (dh[0] + dh[1]) + (dh[2] + dh[3]);
-    }
-  }
   static_assert(nw == 32, "warp m sums member m over the warps");
-  __shared__ double sh[nw][33];
-  sh[w][lane] = acc;
+  // the accumulators [term][warp][member]: 8 FP32 (hi and lo of four pairs) or 4 FP64
+  __shared__ double sh[4][nw][33];
+  float* const sf = reinterpret_cast<float*>(sh);
+  auto at = [](int term, int warp, int member) { return (term * nw + warp) * 33 + member; };
+  const bool f32 = r <= R_44_E;
+  if (f32) {
+    float fh[4] = {0.f, 0.f, 0.f, 0.f}, fl[4] = {0.f, 0.f, 0.f, 0.f};
+    int s = m < P.M ? w : count;
+    for (; s + 3 * nw < count; s += 4 * nw) {
+      float v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = P.f(r, s + q * nw)[m];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) two_sum_acc(fh[q], fl[q], v[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q)  // the last at most 3 slots of this warp
+      if (s + q * nw < count) two_sum_acc(fh[q], fl[q], P.f(r, s + q * nw)[m]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sf[at(q, w, lane)] = fh[q], sf[at(4 + q, w, lane)] = fl[q];
+  } else {
+    double dh[4] = {0.0, 0.0, 0.0, 0.0};
+    int s = m < P.M ? w : count;
+    for (; s + 3 * nw < count; s += 4 * nw) {
+      double v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = P.d(r, s + q * nw)[m];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) dh[q] += v[q];
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      if (s + q * nw < count) dh[q] += P.d(r, s + q * nw)[m];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sh[q][w][lane] = dh[q];
+  }
   __syncthreads();
-  const double tot = f64::value(f64::warp_sum(sh[lane][w]));  // lane = warp, w = member
+  double tot;  // lane = warp, w = member
+  if (f32) {
+    double v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = widen(sf[at(q, lane, w)]);
+    tot = f64::value(f64::warp_sum<8>(v));
+  } else {
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = sh[q][lane][w];
+    tot = f64::value(f64::warp_sum<4>(v));
+  }
   const int mm = blockIdx.y * 32 + w;
   if (lane == 0 && mm < P.M) diag_out[(size_t)mm * kDiagStride + kDiagLen + r] = tot;
 }

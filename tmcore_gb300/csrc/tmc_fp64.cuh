@@ -120,10 +120,11 @@ __device__ __forceinline__ SqrtR sqrt_r(double a) {
 
 // ---------------------------------------------------------------------------
 // sums across lanes in integers: every term is aligned to the largest
-// exponent as a 128-bit integer (53 bits of mantissa, 64 bits below them), the
-// integers are added exactly and the sum is rounded once.  A warp sum costs
-// about a hundred integer instructions; the five additions of an FP64 shuffle
-// tree occupy the FP64 pipe for 320 cycles, a double-double tree's for 6,400.
+// exponent as a 128-bit integer (53 bits of mantissa, 64 bits below them,
+// further bits dropped), the integers are added exactly and the sum is rounded
+// once.  A warp sum costs about a hundred integer instructions and twenty for
+// each further term of a lane; the five additions of an FP64 shuffle tree
+// occupy the FP64 pipe for 320 cycles, a double-double tree's for 6,400.
 // ---------------------------------------------------------------------------
 struct Fixed {
   __int128 m;  // the sum is m 2^(e - 1139)
@@ -164,27 +165,41 @@ __device__ __forceinline__ double value(const Fixed& f) {
   return v.hi + v.lo;
 }
 
-// the sum over the warp of each lane's v, in every lane (all 32 lanes call)
-__device__ __forceinline__ Fixed warp_sum(double v) {
+// the sum over the warp of each lane's N terms, in every lane (all 32 lanes call)
+template <int N>
+__device__ __forceinline__ Fixed warp_sum(const double (&v)[N]) {
+  static_assert(N <= 64, "the lanes' sums leave room for 6 bits above 32 terms");
   const unsigned all = 0xffffffffu;
-  const int hi = __double2hiint(v);
-  const int ex = (hi >> 20) & 0x7ff;
+  int ex = 0;
+#pragma unroll
+  for (int k = 0; k < N; ++k) ex = max(ex, (__double2hiint(v[k]) >> 20) & 0x7ff);
   const int e = (int)__reduce_max_sync(all, (unsigned)ex);
   if ((unsigned)(e - 200) > 1700u) {  // zeros, extreme exponents, infinities, NaN: in FP64
+    double t = v[0];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(all, v, off);
-    return {(__int128)__double_as_longlong(v), -1};
+    for (int k = 1; k < N; ++k) t += v[k];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(all, t, off);
+    return {(__int128)__double_as_longlong(t), -1};
   }
-  long long m = (long long)(((unsigned long long)(unsigned)(hi & 0xfffff) << 32) | (unsigned)__double2loint(v));
-  if (ex) m |= 1ll << 52;
-  if (hi < 0) m = -m;
-  const int sh = e - (ex ? ex : 1);
-  const long long H = m >> (sh < 63 ? sh : 63);
-  unsigned long long L = 0;
-  if (sh >= 64)
-    L = sh < 127 ? (unsigned long long)(m >> (sh - 64)) : (unsigned long long)H;
-  else if (sh > 0)
-    L = (unsigned long long)m << (64 - sh);
+  unsigned __int128 acc = 0;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const int hi = __double2hiint(v[k]), x = (hi >> 20) & 0x7ff;
+    long long m = (long long)(((unsigned long long)(unsigned)(hi & 0xfffff) << 32) | (unsigned)__double2loint(v[k]));
+    if (x) m |= 1ll << 52;
+    if (hi < 0) m = -m;
+    const int sh = e - (x ? x : 1);
+    const long long H = m >> (sh < 63 ? sh : 63);
+    unsigned long long L = 0;
+    if (sh >= 64)
+      L = sh < 127 ? (unsigned long long)(m >> (sh - 64)) : (unsigned long long)H;
+    else if (sh > 0)
+      L = (unsigned long long)m << (64 - sh);
+    acc += (unsigned __int128)(unsigned long long)H << 64 | L;
+  }
+  const long long H = (long long)(unsigned long long)(acc >> 64);
+  const unsigned long long L = (unsigned long long)acc;
   const unsigned M26 = (1u << 26) - 1;
   const unsigned s0 = __reduce_add_sync(all, (unsigned)L & M26);
   const unsigned s1 = __reduce_add_sync(all, (unsigned)(L >> 26) & M26);
@@ -194,6 +209,10 @@ __device__ __forceinline__ Fixed warp_sum(double v) {
   const unsigned __int128 s = (unsigned __int128)s0 + ((unsigned __int128)s1 << 26) + ((unsigned __int128)s2 << 52) +
                               ((unsigned __int128)s3 << 78) + ((unsigned __int128)(__int128)s4 << 104);
   return {(__int128)s, e};
+}
+__device__ __forceinline__ Fixed warp_sum(double v) {
+  const double t[1] = {v};
+  return warp_sum<1>(t);
 }
 
 }  // namespace f64
