@@ -37,3 +37,21 @@ def test_ensemble_mass_is_exact():
     mass = g.diag_all()[:, 0]
     assert np.array_equal(mass, np.ldexp(math.fsum(gd), np.arange(16)))
     g.close()
+
+
+def test_single_model_mass_is_exact():
+    """Blocks of 1024 cells; lane l of a warp takes blocks l and l + 32.
+    Blocks 0-8 hold 2^30 each (unit 2^-22), blocks 32-39 0.47 of that unit,
+    blocks 9-24 2^-25."""
+    from tmcore_gb300.gpu import TMCoreGPU
+
+    m = _unit_areas(6)
+    block = np.arange(m.nCells) // 1024
+    gd = np.full(m.nCells, 2.0 ** -70)
+    gd[block < 9] = 2.0 ** 20
+    gd[(block >= 9) & (block < 25)] = 2.0 ** -35
+    gd[(block >= 32) & (block < 40)] = 15 * 2.0 ** -37
+    g = TMCoreGPU(m, dt=60.0, precision=1, renumber=0, radius=1.0, pv_scheme=1, apvm_weight=0.0)
+    g.set_state(gd, np.zeros(g.ne))
+    assert g.diag_all()[0, 0] == math.fsum(gd)
+    g.close()

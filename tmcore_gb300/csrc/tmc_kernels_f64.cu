@@ -139,6 +139,39 @@ __global__ void __launch_bounds__(256) k_finalize(Partials P0, FinalizeArgs a, d
   if (threadIdx.x == 0) *counter = 0u;
 }
 
+// The sum of `count` per-block pairs (their lo halves only if kLo, else zero) by
+// one warp, in every lane: K pairs per lane at a time, added exactly
+// (f64::warp_sum).  Level 6 has 41 to 120 pairs per region, level 7 up to 480;
+// meshes with more than 32 K add their rounds in double-double.
+template <int K, bool kLo>
+__device__ double region_sum(const double* reg, int count) {
+  const int lane = threadIdx.x & 31;
+  f64::HiLo sum{0.0, 0.0};
+  for (int i0 = 0; i0 < count; i0 += 32 * K) {
+    double t[kLo ? 2 * K : K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int i = i0 + 32 * k + lane;
+      if constexpr (kLo) {
+        const double2 p = i < count ? __ldcg(reinterpret_cast<const double2*>(reg) + i) : make_double2(0.0, 0.0);
+        t[k] = p.x;
+        t[K + k] = p.y;
+      } else {
+        t[k] = i < count ? __ldcg(reg + 2 * (size_t)i) : 0.0;
+      }
+    }
+    const f64::HiLo r = f64::split(f64::warp_sum(t));
+    if (i0 == 0) {
+      sum = r;
+    } else {  // TwoSum (Knuth)
+      const double h = __dadd_rn(sum.hi, r.hi), b = __dsub_rn(h, sum.hi);
+      const double e = __dadd_rn(__dsub_rn(sum.hi, __dsub_rn(h, b)), __dsub_rn(r.hi, b));
+      sum = {h, __dadd_rn(e, __dadd_rn(sum.lo, r.lo))};
+    }
+  }
+  return sum.hi + sum.lo;
+}
+
 // The same after passes of one element per thread, for small FP32 models: the
 // blocks first form the block sums those passes did not store, 256 threads of
 // four elements with the fused multiply-adds, shuffle tree and block tree of
@@ -244,15 +277,13 @@ __global__ void __launch_bounds__(256) k_finalize_products(Partials P, FinalizeA
   __shared__ double rs[kFinalizeRegions];
   const int lane = threadIdx.x & 31;
   for (int q = threadIdx.x >> 5; q < kFinalizeRegions; q += blockDim.x >> 5) {
-    const bool on = (q <= R_44_E) ? a.step : a.diag;
-    double hi = 0.0, lo = 0.0;
-    for (int i = lane; on && i < a.counts[q]; i += 32) {
-      const double2 p = __ldcg(reinterpret_cast<const double2*>(P.region(q)) + i);
-      hi = __dadd_rn(hi, p.x);
-      lo = __dadd_rn(lo, p.y);
-    }
-    const f64::HiLo h = f64::split(f64::warp_sum(hi));
-    const double s = h.hi + (h.lo + f64::value(f64::warp_sum(lo)));
+    const int n = ((q <= R_44_E) ? a.step : a.diag) ? a.counts[q] : 0;
+    const double* const reg = P.region(q);
+    double s;
+    if (q <= R_44_E)  // the products' block sums have no lo half
+      s = n <= 4 * 32 ? region_sum<4, false>(reg, n) : region_sum<16, false>(reg, n);
+    else
+      s = n <= 4 * 32 ? region_sum<4, true>(reg, n) : region_sum<16, true>(reg, n);
     if (lane == 0) rs[q] = res[q] = s;
   }
   __syncthreads();
