@@ -128,6 +128,7 @@ struct tmc_handle {
   // factors of the inner products and vertex terms of the invariants (FP32,
   // passes of one element per thread)
   float *ipc = nullptr, *ipe = nullptr, *vterm = nullptr;
+  int* en64 = nullptr;  // with ipe (StageIO)
   Blk blk(int pass, bool pdl = false) const { return Blk(bsp[pass], ept[pass], pdl && ept[pass] == 1); }
   // a small FP32 model (every pass one element per thread) runs its stages as
   // one chain of dependent launches on st, the cell and vertex passes in one
@@ -378,6 +379,7 @@ struct Engine : EngineBase {
     s.ipc = h->ipc;
     s.ipe = h->ipe;
     s.vterm = h->vterm;
+    s.en64 = h->en64;
     s.E = E;
     s.pv_v = pv_v;
     s.vor = vor;
@@ -434,7 +436,7 @@ struct Engine : EngineBase {
     if constexpr (std::is_same<T, float>::value) {
       X = Products{M.nc, M.ne, M.nv, h->ipc, h->ipe, h->vterm, M.areaCell_f, M.areaEdge_f, M.areaTriangle_f,
                    M.fVertex_f, M.areaCell, gd[0], ghs, gdf[0], ghsf, iap[0],
-                   !step || !launch_cell_is_fast(h->O), !step};
+                   !step || !launch_cell_is_fast(h->O), h->en64};
     }
     launch_finalize(h->P, h->counts, h->hm.totalArea, h->hm.sumAreaTriangle, h->O.dt, step, diag,
                     h->p.conserve_energy != 0 && step, h->d_diag, h->st, 2, h->members, X.c ? &X : nullptr, pdl);
@@ -1567,9 +1569,12 @@ int tmc_create(const tmc_mesh_desc* mesh, const tmc_params* params, tmc_handle**
   if (!h->generic && h->members == 1) choose_launch_shapes(h.get(), p.block_size == 0);
   if (p.precision == TMC_FP32 && h->members == 1) {
     if (h->ept[P_CELL] == 1) h->ipc = h->dalloc<float>((size_t)4 * hm.nc);
-    if (h->ept[P_FLUX] == 1) h->ipe = h->dalloc<float>((size_t)4 * hm.ne);
+    if (h->ept[P_FLUX] == 1) {
+      h->ipe = h->dalloc<float>((size_t)4 * hm.ne);
+      h->en64 = h->dalloc<int>(1);
+    }
     if (h->ept[P_VERTEX] == 1) h->vterm = h->dalloc<float>((size_t)2 * hm.nv);
-    if ((h->ept[P_CELL] == 1 && !h->ipc) || (h->ept[P_FLUX] == 1 && !h->ipe) ||
+    if ((h->ept[P_CELL] == 1 && !h->ipc) || (h->ept[P_FLUX] == 1 && (!h->ipe || !h->en64)) ||
         (h->ept[P_VERTEX] == 1 && !h->vterm)) {
       h->err = "device allocation failed";
       cudaGetLastError();

@@ -205,6 +205,7 @@ struct StageIO {
   // [4][nc] and [4][ne] (t1 t2, t2 t3, t3 t4, t_new t_new), and [2][nv] the
   // vertex terms of potential enstrophy and vorticity; see Products
   float *ipc, *ipe, *vterm;
+  int* en64;  // 1: state(old) comes from k_edge_prep, whose energy is an FP64 sum; 0: from a step
   // the next stage's gd_e, u, F, Fq, written by k_edge_flux (stages 1-3) and
   // k_final_edges (next step): the edge preparation of the next stage fused
   // into the pass that produces its iap_u (null: not fused)
@@ -371,7 +372,8 @@ struct Products {
   const float *areaCell_f, *areaEdge_f, *areaTriangle_f, *fVertex_f;
   const double *areaCell, *gd, *ghs;
   const float *gdf, *ghsf, *iap;
-  bool enc64, ene64;  // the cells' (edges') energy terms in FP64 (k_cell, k_edge_prep), else FP32, compensated
+  bool enc64;       // the cells' energy terms in FP64 (k_cell), else FP32, compensated
+  const int* en64;  // the edges' likewise (k_edge_prep; k_final_edges)
 };
 void launch_finalize(Partials P, const int* counts_host, double totalArea, double sumAreaTriangle, double dt,
                      bool step, bool diag, bool conserve, double* diag_out, cudaStream_t st, int scheme = 2,

@@ -232,19 +232,20 @@ __global__ void __launch_bounds__(256) k_finalize_products(Partials P, FinalizeA
       sum_products(P, X.e, X.areaEdge_f, X.ne, slot, r);
     }
     if (a.diag) {
+      const bool ene64 = *X.en64 != 0;
       double en = 0.0;
       float eh = 0.f, el = 0.f;
       for (int j = 0; j < kEPT; ++j) {
         const int i = slot * (kEPT * 256) + j * 256 + threadIdx.x;
         if (i >= X.ne) break;
         const float t = X.iap[i] * X.iap[i] * X.areaEdge_f[i];
-        if (X.ene64)
+        if (ene64)
           en += (double)t;
         else
           two_sum_acc(eh, el, t);
       }
       const int r[1] = {R_EN_E};
-      if (X.ene64) {
+      if (ene64) {
         const double v[1] = {en};
         block_store<double, 1>(v, P, r, slot);
       } else {

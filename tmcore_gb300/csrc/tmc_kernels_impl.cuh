@@ -439,6 +439,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_edge_prep(DevMesh M, ModelOpt O, 
     const int r[1] = {R_EN_E};
     block_store<double, 1>(v, P, r);
   }
+  if (kProducts<T, EPT> && diag && blockIdx.x == 0 && threadIdx.x == 0) *S.en64 = 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -1577,7 +1578,10 @@ __global__ void __launch_bounds__(kB ? kMemberBlock : kMaxBlock, kB ? TMC_FINAL_
     else
       two_sum_acc(eh, el, ia[j] * ia[j] * ae[j]);
   }
-  if constexpr (kProducts<T, EPT>) return;
+  if constexpr (kProducts<T, EPT>) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *S.en64 = 0;
+    return;
+  }
   const int r[1] = {R_EN_E};
   if constexpr (kF64<T>) {
     const double v[1] = {en};
