@@ -1,0 +1,37 @@
+"""Small FP32 models run a step as one chain of dependent launches with the
+cell and the vertex pass of a stage in one: what the timing calls report is
+that program, and no block size takes a model off it."""
+import numpy as np
+import pytest
+
+from tmcore_gb300 import abi, cases, mesh
+
+pytestmark = pytest.mark.gpu
+
+CENTRED = dict(pv_scheme=1, apvm_weight=0.0)
+UPWIND = dict(pv_scheme=3, interp_pv_order=3)
+
+
+def _model(level=4, precision=abi.TMC_FP32, **kw):
+    from tmcore_gb300.gpu import TMCoreGPU
+
+    m = mesh.icos_mesh(level)
+    g = TMCoreGPU(m, dt=60.0, precision=precision, **kw)
+    g.set_initial(*cases.jet_bumps(m, seed=1))
+    return g
+
+
+def _launches(g):
+    return g.time_steps(1, total=True, flux=False)[3]
+
+
+@pytest.mark.parametrize("kw,chained,separate", [(CENTRED, 15, 19), (UPWIND, 19, 23),
+                                                 (dict(pv_scheme=1, apvm_weight=0.5), 19, 23)])
+def test_launch_count(kw, chained, separate):
+    """Per stage cell + vertex (one launch in a chain), pv on edges (one, or
+    two with the vertex fits or with pv on cells) and flux; then the sums and
+    the two final updates."""
+    for precision, want in ((abi.TMC_FP32, chained), (abi.TMC_FP64, separate)):
+        g = _model(precision=precision, **kw)
+        assert _launches(g) == want
+        g.close()

@@ -410,7 +410,8 @@ struct Engine : EngineBase {
     return 4 + (v2c ? 1 : 0) + (h->O.pv_scheme == 2 ? 4 : 0) + (h->M.vfit_n ? 1 : 0);
   }
   int launches_per_step() const override {
-    if (!h->generic) return 4 * launches_per_stage_passes() + 3;
+    // (a chain runs the cell and the vertex pass of a stage in one launch)
+    if (!h->generic) return 4 * (launches_per_stage_passes() - (h->chain() ? 1 : 0)) + 3;
     // generic: spatial passes per evaluation (+ the edge preparation), state
     // updates (adv: + 2 wind kernels each), combination, finaliser, final update
     const int ts = h->p.time_scheme;
