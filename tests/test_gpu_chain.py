@@ -35,3 +35,11 @@ def test_launch_count(kw, chained, separate):
         g = _model(precision=precision, **kw)
         assert _launches(g) == want
         g.close()
+
+
+@pytest.mark.parametrize("block_size", [32, 224, 256, 288, 512])
+def test_block_sizes_keep_the_chain(block_size):
+    """The FP32 cell pass takes at most 256 threads per block, the others 512."""
+    g = _model(block_size=block_size, **CENTRED)
+    assert _launches(g) == 15
+    g.close()

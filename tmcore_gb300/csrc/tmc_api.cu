@@ -137,11 +137,11 @@ struct tmc_handle {
   // end on two streams.  Us per step, two streams / chain: FP32 level 5 47 /
   // 35, level 6 with four tracers 61 / 54, with upwind pv 72 / 67.  FP64
   // passes fill the FP64 pipe, which two streams share better (level 6 178 /
-  // 205).
+  // 205).  The merged launch takes the cell pass's block size.
   bool chain() const {
     for (int k = 0; k < 5; ++k)
       if (ept[k] != 1) return false;
-    return p.precision == TMC_FP32 && !generic && members == 1 && O.pv_scheme != 2 && bsp[0] == bsp[1];
+    return p.precision == TMC_FP32 && !generic && members == 1 && O.pv_scheme != 2;
   }
   // learned PV-on-edge closure (FP32 path): network, per-member switch, wait status
   const tmc_mlp* closure = nullptr;

@@ -342,7 +342,7 @@ template <class T>
 void launch_vertex(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Partials P, bool diag, Blk b,
                    cudaStream_t st);
 // the cell and vertex passes of one stage in one launch (they read only the
-// stage's input, nothing the other writes); b.ept 1, the same block size for both
+// stage's input, nothing the other writes); b.ept 1
 template <class T>
 void launch_cell_vertex(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Partials P, bool diag,
                         Blk b, cudaStream_t st);
