@@ -160,7 +160,8 @@ int tmc_autotune(tmc_handle* h, int32_t steps, int32_t block_sizes[5]);
 /* Mean device time of one launch of each pass of the fused step over
  * `steps` eager steps (CUDA events around the pass; the steps advance the
  * state): ms = {cell, vertex, edge_pv (with the closure and conservative APVM
- * kernels), edge_flux, final update}. */
+ * kernels), edge_flux, final update}.  A small FP32 model runs cell and vertex
+ * in one launch: its time is the cell's, the vertex's is 0. */
 int tmc_pass_times(tmc_handle* h, int32_t steps, double ms[5]);
 
 /* History diagnostics on the device (history_mod.F90:124-174 with

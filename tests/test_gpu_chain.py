@@ -43,3 +43,19 @@ def test_block_sizes_keep_the_chain(block_size):
     g = _model(block_size=block_size, **CENTRED)
     assert _launches(g) == 15
     g.close()
+
+
+@pytest.mark.parametrize("kw", [CENTRED, UPWIND])
+def test_pass_times_are_the_chain_s(kw):
+    """The merged launch is the cell pass's time; the timed steps give the
+    chain's states and invariants bit for bit."""
+    g, ref = _model(**kw), _model(**kw)
+    t = g.pass_times(3)
+    assert t["vertex"] == 0.0 and all(t[k] > 0.0 for k in ("cell", "edge_pv", "edge_flux", "final"))
+    ms, flux, n, _ = g.time_steps(2, total=False, flux=True)
+    assert flux > 0.0 and n == 8
+    ref.step(5 * 3 + 2)
+    for a, b in zip(g.get_state() + (g.diag(),), ref.get_state() + (ref.diag(),)):
+        assert np.array_equal(a, b)
+    g.close()
+    ref.close()

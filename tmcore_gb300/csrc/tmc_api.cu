@@ -475,11 +475,18 @@ struct Engine : EngineBase {
     auto mark = [&](int pass) {
       if (flux_ev && h->timed_pass == pass) cudaEventRecord((*flux_ev)[(*ev_pos)++], h->st);
     };
-    if (!flux_ev && !no_tracers && h->chain()) {
-      launch_cell_vertex<T>(M, O, s, rk, h->P, dg, h->blk(P_CELL, true), h->st);
-      launch_edge_pv<T>(M, O, s, h->blk(P_PV, !O.need_pv_c), h->st);
+    if (!no_tracers && h->chain()) {
+      const bool pdl = !flux_ev;  // passes timed one by one run one after another
+      mark(P_CELL);
+      launch_cell_vertex<T>(M, O, s, rk, h->P, dg, h->blk(P_CELL, pdl), h->st);
+      mark(P_CELL);
+      mark(P_PV);
+      launch_edge_pv<T>(M, O, s, h->blk(P_PV, pdl && !O.need_pv_c), h->st);
       launch_closure_pass(s, k);
-      launch_edge_flux<T>(M, O, s, rk, h->P, h->blk(P_FLUX, !h->closure), h->st);
+      mark(P_PV);
+      mark(P_FLUX);
+      launch_edge_flux<T>(M, O, s, rk, h->P, h->blk(P_FLUX, pdl && !h->closure), h->st);
+      mark(P_FLUX);
       return;
     }
     // concurrent cell and vertex / pv-on-edge branches, except while passes
