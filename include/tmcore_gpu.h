@@ -154,7 +154,9 @@ int tmc_spatial_operators(tmc_handle* h, const double* gd, const double* iap_u, 
 /* Autotuner: times `steps` eager steps of the current state for each block
  * size in {64, 128, 192, 256, 384, 512} (256 at most for ensembles), one pass
  * of the fused step at a time (edge_flux, cell, vertex, edge_pv, final), keeps
- * the fastest per pass, restores the state and re-captures the step graphs.
+ * the fastest per pass, restores the state and re-captures the step graphs.  A
+ * small FP32 model, whose passes overlap in one chain of launches, is timed by
+ * whole steps (at least 20), its cell and vertex passes as one.
  * block_sizes (may be NULL) receives {cell, vertex, edge_pv, edge_flux, final}. */
 int tmc_autotune(tmc_handle* h, int32_t steps, int32_t block_sizes[5]);
 /* Mean device time of one launch of each pass of the fused step over

@@ -2366,39 +2366,85 @@ int tmc_autotune(tmc_handle* h, int32_t steps, int32_t block_sizes[5]) {
   const int limit = h->members > 1 ? 256 : 512;
   const int order[P_COUNT] = {P_FLUX, P_CELL, P_VERTEX, P_PV, P_FINAL};
   const int saved_timed = h->timed_pass;
+  const bool chain = h->chain();
+  // time of the pass with the present block sizes, in *t: of the pass alone over
+  // `steps` steps; in a chain of dependent launches (which overlap) of whole
+  // steps as tmc_step runs them, the best of three runs.  1e300: refused
+  auto timed = [&](double* t) -> int {
+    *t = 1e300;
+    set_counts(h);
+    h->prep_valid = false;
+    int rc;
+    if (chain) {
+      const int n = std::max(steps, 20);
+      const long count = h->step_count;
+      const int diag_every = h->p.diag_every;
+      h->p.diag_every = 0;
+      h->drop_graphs();
+      rc = launch_one_step(h);
+      double best = 1e300;
+      for (int rep = 0; rep < 3 && rc == TMC_OK; ++rep) {
+        cudaEventRecord(h->ev_pool[0], h->st);
+        for (int i = 0; i < n && rc == TMC_OK; ++i) rc = launch_one_step(h);
+        cudaEventRecord(h->ev_pool[1], h->st);
+        const int rs = sync(h, "tmc_autotune");
+        if (rs) return rs;
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, h->ev_pool[0], h->ev_pool[1]);
+        best = std::min(best, (double)ms);
+      }
+      h->step_count = count;
+      h->p.diag_every = diag_every;
+      if (rc == TMC_OK && cudaGetLastError() == cudaSuccess) *t = best;
+      return sync(h, "tmc_autotune");
+    }
+    // one untimed step with this block size, then `steps` timed ones
+    ensure_prep(h);
+    h->eng->launch_step(false, nullptr, nullptr);
+    std::vector<cudaEvent_t> evs(h->ev_pool.begin(), h->ev_pool.begin() + nev);
+    size_t pos = 0;
+    for (int i = 0; i < steps; ++i) h->eng->launch_step(false, &evs, &pos);
+    if ((rc = sync(h, "tmc_autotune"))) return rc;
+    // a block size whose launches were refused (its events would time
+    // nothing) is not a candidate
+    if (cudaGetLastError() != cudaSuccess) return TMC_OK;
+    double sum = 0.0;
+    for (size_t k = 0; k + 1 < pos; k += 2) {
+      float dt = 0.f;
+      cudaEventElapsedTime(&dt, evs[k], evs[k + 1]);
+      sum += dt;
+    }
+    *t = sum;
+    return TMC_OK;
+  };
   for (int pi = 0; pi < P_COUNT; ++pi) {
     const int pass = order[pi];
+    if (chain && pass == P_VERTEX) continue;  // in the cell pass's launch
     h->timed_pass = pass;
-    double best = 1e300;
+    auto set = [&](int bs) {
+      h->bsp[pass] = bs;
+      if (chain && pass == P_CELL) h->bsp[P_VERTEX] = bs;
+    };
     int best_bs = h->bsp[pass];
+    double best = 1e300;
+    // a chain's sizes differ by little: another must win by more than 1%
+    if (chain) {
+      if ((rc = timed(&best))) break;
+      best *= 0.99;
+    }
     for (int c : cand_all) {
       if (c > limit || (pass == P_CELL && f32 && c > 256)) continue;
-      h->bsp[pass] = c;
-      set_counts(h);
-      // one untimed step with this block size, then `steps` timed ones
-      h->prep_valid = false;
-      ensure_prep(h);
-      h->eng->launch_step(false, nullptr, nullptr);
-      std::vector<cudaEvent_t> evs(h->ev_pool.begin(), h->ev_pool.begin() + nev);
-      size_t pos = 0;
-      for (int i = 0; i < steps; ++i) h->eng->launch_step(false, &evs, &pos);
-      if ((rc = sync(h, "tmc_autotune"))) break;
-      // a block size whose launches were refused (its events would time
-      // nothing) is not a candidate
-      if (cudaGetLastError() != cudaSuccess) continue;
-      double sum = 0.0;
-      for (size_t k = 0; k + 1 < pos; k += 2) {
-        float dt = 0.f;
-        cudaEventElapsedTime(&dt, evs[k], evs[k + 1]);
-        sum += dt;
-      }
-      if (sum < best) {
-        best = sum;
+      if (chain && c == best_bs) continue;
+      set(c);
+      double t;
+      if ((rc = timed(&t))) break;
+      if (t < best) {
+        best = t;
         best_bs = c;
       }
     }
     if (rc) break;
-    h->bsp[pass] = best_bs;
+    set(best_bs);
   }
   h->timed_pass = saved_timed;
   set_counts(h);
