@@ -97,7 +97,8 @@ typedef struct tmc_params {
                                      members; a lane takes two members when members is a multiple of twice
                                      that, else one.  0 = automatic: 32 lanes (16 when members is not a
                                      multiple of 32), two members per lane when members is a multiple of 64 */
-  int32_t reserved[2];
+  int32_t elements_per_thread;    /* fused single-model passes: 1 or 4; otherwise chosen by the mesh's size */
+  int32_t reserved[1];
 } tmc_params;
 
 typedef struct tmc_handle tmc_handle;

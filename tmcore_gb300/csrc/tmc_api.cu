@@ -1150,7 +1150,7 @@ void set_counts(tmc_handle* h) {
 }
 
 // Elements per thread (1 or kEPT) and default block size of each pass of the
-// fused single-model step, by element count.  Four elements per thread leave
+// fused single-model step, by element count unless the caller chose.  Four elements per thread leave
 // SMs without a block on a small mesh (level 6: 120 blocks of 256 edges x 4
 // on 152 SMs) and run a thread's elements one after another; one element per
 // thread costs a large mesh the loads in flight and the warps' start-up.
@@ -1181,7 +1181,8 @@ void choose_launch_shapes(tmc_handle* h, bool default_blocks) {
   line[P_FLUX] = f64 ? big : small;
   line[P_FINAL] = f64 ? 0x7fffffff : small;
   for (int k = 0; k < P_COUNT; ++k) {
-    if (n[k] >= line[k]) continue;
+    const int ept = h->p.elements_per_thread;
+    if (ept == kEPT || (ept != 1 && n[k] >= line[k])) continue;
     h->ept[k] = 1;
     if (default_blocks) h->bsp[k] = f64 && n[k] < 64 * 16 * h->sms ? 64 : 128;
   }

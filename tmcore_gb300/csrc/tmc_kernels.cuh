@@ -288,7 +288,7 @@ inline unsigned nmem(const StageIO<T>& S) {
 }
 
 // Launch shape of a pass: threads per block and elements per thread, 1 or
-// kEPT.  One on a mesh too small to fill the GPU otherwise (elements_per_thread).
+// kEPT.  One on a mesh too small to fill the GPU otherwise (choose_launch_shapes).
 // pdl: a programmatic dependent launch, for kernels of one element per thread:
 // they may start while the stream's previous kernel runs and wait for it
 // (pdl_wait) before they read or write anything but the mesh.
