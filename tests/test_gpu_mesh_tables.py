@@ -41,3 +41,15 @@ def test_foreign_edges(change):
     m = copy.deepcopy(mesh.icos_mesh(3))
     change(m)
     _check(m, **CENTRED)
+
+
+def _edge_missing_from_vertex(m):
+    m.vars["edgesOnVertex"][200, 1] = m.vars["edgesOnVertex"][200, 0]
+
+
+@pytest.mark.parametrize("order", [3, 4])
+def test_upwind_pv_of_an_edge_its_vertex_does_not_list(order):
+    """The vertex fits, formed by vertex, would leave the edge's side unset."""
+    m = copy.deepcopy(mesh.icos_mesh(3))
+    _edge_missing_from_vertex(m)
+    _check(m, pv_scheme=3, interp_pv_order=order)

@@ -1133,6 +1133,21 @@ int build_graph(tmc_handle* h, bool diag, cudaGraphExec_t* out, int first_stage 
   return TMC_OK;
 }
 
+// every edge's two sides belong to one vertex each that lists the edge, once
+// (k_vert_fit writes an edge's side from its vertex)
+bool vertices_cover_edges(const HostMesh& hm) {
+  std::vector<uint8_t> seen((size_t)2 * hm.ne, 0);
+  for (int k = 0; k < 3; ++k)
+    for (int v = 0; v < hm.nv; ++v) {
+      const size_t q = (size_t)k * hm.nv + v, e = hm.edgesOnVertex[q];
+      if (hm.tSignEdge[q] == 0) return false;
+      const size_t side = (hm.tSignEdge[q] > 0 ? 0 : (size_t)hm.ne) + e;
+      if (hm.verticesOnEdge[side] != v || seen[side]) return false;
+      seen[side] = 1;
+    }
+  return std::find(seen.begin(), seen.end(), 0) == seen.end();
+}
+
 // partial counts per region: the grid of the passes that write it
 void set_counts(tmc_handle* h) {
   const int bc = grid_for(h->M.nc, h->blk(P_CELL)), bf = grid_for(h->M.ne, h->blk(P_FLUX)),
@@ -1492,7 +1507,7 @@ int tmc_create(const tmc_mesh_desc* mesh, const tmc_params* params, tmc_handle**
   M.vert2 = upload_stencil(h.get(), hm.vert2);
   M.vert4 = upload_stencil(h.get(), hm.vert4);
   if (p.pv_scheme == 3 && (p.interp_pv_order == 3 || p.interp_pv_order == 4) && hm.vert2.width > 0 &&
-      p.member_layout == 0) {
+      p.member_layout == 0 && vertices_cover_edges(hm)) {
     // the vertex fit stencils by vertex: an edge's side has the points of its
     // vertex, in the vertex's order, and weights of its own
     const int W = hm.vert2.width, nv = hm.nv;

@@ -74,7 +74,8 @@ struct DevMesh {
   DStencil cell2, cell3, cell4, vert2, vert4;  // cell3: deriv3OnCell on the fit3 (= fit4) stencils
   // upwind pv of order 3 or 4 (pv_scheme 3): the vertex fit stencils by vertex,
   // point j of vertex v and its weights for the vertex's three edges (null
-  // otherwise: the generic stencil loop runs)
+  // otherwise, and where the mesh's vertices do not list every edge's two sides
+  // once: the generic stencil loop runs)
   const uint8_t* vfit_n;    // [nv] points
   const int32_t* vfit_idx;  // [width][nv] and
   const double* vfit_w;     // [width][3][nv]: FP64 path
