@@ -53,3 +53,16 @@ def test_upwind_pv_of_an_edge_its_vertex_does_not_list(order):
     m = copy.deepcopy(mesh.icos_mesh(3))
     _edge_missing_from_vertex(m)
     _check(m, pv_scheme=3, interp_pv_order=order)
+
+
+@pytest.mark.parametrize("kw", [CENTRED, dict(pv_scheme=3, interp_pv_order=3)])
+def test_wide_neighbour_tables(kw):
+    """Six entries per neighbour, with alternating signs but for the first: 60
+    of the 64 neighbours a mesh may have, and sums that cancel."""
+    m = copy.deepcopy(mesh.icos_mesh(3))
+    w = m.vars["weightsOnEdge"][:, :, None] * np.array([1.0, 0.7, -0.7, 0.3, -0.3, 0.0])
+    m.vars["weightsOnEdge"] = np.ascontiguousarray(w.reshape(m.nEdges, -1))
+    m.vars["edgesOnEdge"] = np.ascontiguousarray(np.repeat(m.vars["edgesOnEdge"], 6, axis=1))
+    m.vars["nEdgesOnEdge"] = m.vars["nEdgesOnEdge"] * 6
+    m.dims = dict(m.dims, maxEdges2=6 * m.dims["maxEdges2"])
+    _check(m, **kw)

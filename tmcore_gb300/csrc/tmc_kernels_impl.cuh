@@ -970,9 +970,10 @@ __global__ void __launch_bounds__(256, kF64<T> ? 1 : 4) k_vert_fit(DevMesh M, St
 }
 
 // The sign of the tangential velocity (:223-237) picks the upwind side.  FP64:
-// it is decided by an FP32 sum wherever that exceeds the sum's error bound (12
-// terms of 2^-24 of the magnitudes; the test asks for 32), else by the FP64
-// sum in the reference order: 20 FP64 instructions per edge less.
+// it is decided by an FP32 sum wherever that exceeds the sum's error bound (n + 2
+// roundings of 2^-24 of the magnitudes for n neighbours, of which a mesh has at
+// most 64; the test asks for 128), else by the FP64 sum in the reference order:
+// 20 FP64 instructions per edge less.
 template <class T, bool kDep>
 __device__ __forceinline__ T upwind_sign(const DevMesh& M, const StageIO<T>& S, int e) {
   const int ne = M.ne;
@@ -987,7 +988,7 @@ __device__ __forceinline__ T upwind_sign(const DevMesh& M, const StageIO<T>& S, 
       s = __fadd_rn(s, t);
       a = __fadd_rn(a, fabsf(t));
     }
-    if (fabsf(s) > a * 0x1p-19f && a > 1e-25f && a < 1e30f) return s < 0.f ? -1.0 : 1.0;
+    if (fabsf(s) > a * 0x1p-17f && a > 1e-25f && a < 1e30f) return s < 0.f ? -1.0 : 1.0;
     double ve = 0.0;
     for (int i = 0; i < n; ++i) {
       const size_t k = (size_t)i * ne + e;
