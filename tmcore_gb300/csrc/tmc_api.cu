@@ -475,19 +475,21 @@ struct Engine : EngineBase {
     auto mark = [&](int pass) {
       if (flux_ev && h->timed_pass == pass) cudaEventRecord((*flux_ev)[(*ev_pos)++], h->st);
     };
-    if (!no_tracers && h->chain()) {
-      const bool pdl = !flux_ev;  // passes timed one by one run one after another
-      mark(P_CELL);
-      launch_cell_vertex<T>(M, O, s, rk, h->P, dg, h->blk(P_CELL, pdl), h->st);
-      mark(P_CELL);
-      mark(P_PV);
-      launch_edge_pv<T>(M, O, s, h->blk(P_PV, pdl && !O.need_pv_c), h->st);
-      launch_closure_pass(s, k);
-      mark(P_PV);
-      mark(P_FLUX);
-      launch_edge_flux<T>(M, O, s, rk, h->P, h->blk(P_FLUX, pdl && !h->closure), h->st);
-      mark(P_FLUX);
-      return;
+    if constexpr (std::is_same<T, float>::value) {
+      if (!no_tracers && h->chain()) {
+        const bool pdl = !flux_ev;  // passes timed one by one run one after another
+        mark(P_CELL);
+        launch_cell_vertex(M, O, s, rk, h->P, dg, h->blk(P_CELL, pdl), h->st);
+        mark(P_CELL);
+        mark(P_PV);
+        launch_edge_pv<T>(M, O, s, h->blk(P_PV, pdl && !O.need_pv_c), h->st);
+        launch_closure_pass(s, k);
+        mark(P_PV);
+        mark(P_FLUX);
+        launch_edge_flux<T>(M, O, s, rk, h->P, h->blk(P_FLUX, pdl && !h->closure), h->st);
+        mark(P_FLUX);
+        return;
+      }
     }
     // concurrent cell and vertex / pv-on-edge branches, except while passes
     // are timed one by one and for the conservative APVM (its global sums)
@@ -948,7 +950,6 @@ struct EnsEngine : EngineBase {
     s.gd_acc = gd_acc;
     s.iap_in = iap0;
     s.iap_old = iap0;
-    s.iap_next = nullptr;
     s.iap_acc = iap_acc;
     s.iap_tend = iap_tend;
     s.tendf = tendf;

@@ -92,7 +92,6 @@ struct IO {
   float* gd_acc;
   const float* iap_in;
   const float* iap_old;
-  float* iap_next;
   float* iap_acc;
   float* iap_tend;
   float* tendf;

@@ -290,7 +290,7 @@ inline unsigned nmem(const StageIO<T>& S) {
 
 // Launch shape of a pass: threads per block and elements per thread, 1 or
 // kEPT.  One on a mesh too small to fill the GPU otherwise (choose_launch_shapes).
-// pdl: a programmatic dependent launch, for kernels of one element per thread:
+// pdl: a programmatic dependent launch, for a small FP32 model's kernels:
 // they may start while the stream's previous kernel runs and wait for it
 // (pdl_wait) before they read or write anything but the mesh.
 struct Blk {
@@ -343,9 +343,8 @@ template <class T>
 void launch_vertex(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Partials P, bool diag, Blk b,
                    cudaStream_t st);
 // the cell and vertex passes of one stage in one launch (they read only the
-// stage's input, nothing the other writes); b.ept 1
-template <class T>
-void launch_cell_vertex(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Partials P, bool diag,
+// stage's input, nothing the other writes); FP32, b.ept 1
+void launch_cell_vertex(const DevMesh& M, const ModelOpt& O, const StageIO<float>& S, RKStage rk, Partials P, bool diag,
                         Blk b, cudaStream_t st);
 template <class T>
 void launch_edge_pv(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Blk b, cudaStream_t st);
@@ -378,7 +377,7 @@ struct Products {
 };
 void launch_finalize(Partials P, const int* counts_host, double totalArea, double sumAreaTriangle, double dt,
                      bool step, bool diag, bool conserve, double* diag_out, cudaStream_t st, int scheme = 2,
-                     int members = 1, const Products* products = nullptr, bool pdl = false);
+                     int members = 1, const Products* products = nullptr, bool pdl = false);  // (pdl: with products)
 
 // conservative APVM (pv_scheme 2) after k_edge_pv: both tangent fluxes, their
 // curls and the three global sums, epsilon, and the correction of pv_edge

@@ -98,8 +98,6 @@ __device__ __forceinline__ void finish_step(const FinalizeArgs& a, const double*
 // step went from 118.3 to 102.8 us with the integer sums.
 __global__ void __launch_bounds__(256) k_finalize(Partials P0, FinalizeArgs a, double* out0, double* res0,
                                                   unsigned int* counter0) {
-  pdl_start();
-  pdl_wait();
   // one member per blockIdx.y: its partials, outputs, region sums and counter
   const Partials P = P0.at(blockIdx.y);
   double* out = out0 + (size_t)blockIdx.y * kDiagStride;
@@ -320,10 +318,6 @@ void launch_finalize(Partials P, const int* counts_host, double totalArea, doubl
     const int nbv = products->v && diag ? grid_for(products->nv, 256) : 0;
     launch(k_finalize_products, std::max(nbc + nbe + nbv, 1), Blk(256, 1, pdl), st, P, a, *products, nbc, nbe, nbv,
            diag_out, res, counter);
-    return;
-  }
-  if (pdl && members <= 1) {
-    launch(k_finalize, kFinalizeRegions * a.split, Blk(256, 1, true), st, P, a, diag_out, res, counter);
     return;
   }
   k_finalize<<<dim3(kFinalizeRegions * a.split, members > 1 ? members : 1), 256, 0, st>>>(P, a, diag_out, res,

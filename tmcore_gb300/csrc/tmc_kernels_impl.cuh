@@ -98,13 +98,12 @@ __device__ __forceinline__ void block_store(const A (&v)[N], const Partials& P, 
 template <class T>
 constexpr bool kF64 = std::is_same<T, double>::value;
 
-// Programmatic dependent launch (Blk::pdl): the kernels of one element per
-// thread of a single model let the next one start at once (pdl_start) and wait
-// for the previous one before they touch the state (pdl_wait), after the loads
-// of the mesh where those come first.  In a launch without the attribute both
-// do nothing.
-template <bool kB, int EPT>
-constexpr bool kPdl = !kB && EPT == 1;
+// Programmatic dependent launch (Blk::pdl): the kernels of a small FP32 model's
+// chain let the next one start at once (pdl_start) and wait for the previous one
+// before they touch the state (pdl_wait), after the loads of the mesh where
+// those come first.  In a launch without the attribute both do nothing.
+template <class T, bool kB, int EPT>
+constexpr bool kPdl = !kF64<T> && !kB && EPT == 1;
 // the state of a dependent launch is another kernel's output until pdl_wait:
 // plain loads, where a kernel alone reads its inputs through the read-only path
 template <bool kDep, class T>
@@ -409,10 +408,6 @@ template <class T, bool kB, int EPT>
 __global__ void __launch_bounds__(kMaxBlock) k_edge_prep(DevMesh M, ModelOpt O, StageIO<T> S0, Partials P0, int diag) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
-  if constexpr (kPdl<kB, EPT>) {
-    pdl_start();
-    pdl_wait();
-  }
   double en = 0.0;
   const CellSrc<T> C{S.gd_in, S.gdf_in, S.q_in, S.qr_in, nullptr};
   TMC_FOR_N(EPT, e, M.ne) {
@@ -445,13 +440,14 @@ __global__ void __launch_bounds__(kMaxBlock) k_edge_prep(DevMesh M, ModelOpt O, 
 // ---------------------------------------------------------------------------
 // cell: div of mass flux, kinetic energy, E, RK update of gd and tracers
 // ---------------------------------------------------------------------------
-template <class T, bool kB, int EPT>
+// (kDep, here and below: a dependent launch)
+template <class T, bool kB, int EPT, bool kDep>
 __device__ __forceinline__ void cell_body(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S0, RKStage rk,
                                           const Partials& P0, int diag, int b0 = 0) {
   const int bx = (int)blockIdx.x - b0;  // this block among the cells' blocks
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
-  if constexpr (kPdl<kB, EPT>) {
+  if constexpr (kDep) {
     pdl_start();
     pdl_wait();
   }
@@ -701,17 +697,17 @@ __device__ __forceinline__ void cell_body(const DevMesh& M, const ModelOpt& O, c
 template <class T, bool kB, int EPT>
 __global__ void __launch_bounds__(kMaxBlock) k_cell(DevMesh M, ModelOpt O, StageIO<T> S0, RKStage rk, Partials P0,
                                                     int diag) {
-  cell_body<T, kB, EPT>(M, O, S0, rk, P0, diag);
+  cell_body<T, kB, EPT, false>(M, O, S0, rk, P0, diag);
 }
 
 // ---------------------------------------------------------------------------
 // vertex: gd on vertices, vorticity, potential vorticity
 // ---------------------------------------------------------------------------
-template <class T, bool kB, int EPT>
+template <class T, bool kB, int EPT, bool kDep>
 __device__ __forceinline__ void vertex_body(const DevMesh& M, const StageIO<T>& S0, const Partials& P0, int diag) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
-  if constexpr (kPdl<kB, EPT>) pdl_start();
+  if constexpr (kDep) pdl_start();
   double pe = 0.0, av = 0.0;      // FP64 path
   float ph = 0.f, pl = 0.f, ah = 0.f, al = 0.f;  // FP32 path: compensated sums
   if constexpr (kF64<T>) {
@@ -727,7 +723,6 @@ __device__ __forceinline__ void vertex_body(const DevMesh& M, const StageIO<T>& 
         kt[i] = M.kite[(size_t)i * M.nv + v];
       }
       const double At = M.areaTriangle[v], rAt = M.invAreaTriangle[v], fv = M.fVertex[v];
-      if constexpr (kPdl<kB, EPT>) pdl_wait();
 #pragma unroll
       for (int i = 0; i < 3; ++i) gv = gv + S.gd_in[ci[i]] * kt[i];
       gv = f64::div_r(gv, At, rAt);
@@ -768,11 +763,11 @@ __device__ __forceinline__ void vertex_body(const DevMesh& M, const StageIO<T>& 
       const float iA = __ldg(M.invAreaTriangle_f + v);
       const float At = diag ? __ldg(M.areaTriangle_f + v) : 0.f;
       const float fv = __ldg(M.fVertex_f + v);
-      if constexpr (kPdl<kB, EPT>) pdl_wait();
+      if constexpr (kDep) pdl_wait();
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
-        g[i] = kPdl<kB, EPT> ? S.gdf_in[ci[i]] : __ldg(S.gdf_in + ci[i]);
-        uu[i] = kPdl<kB, EPT> ? S.u[ei[i]] : __ldg(S.u + ei[i]);
+        g[i] = state_load<kDep>(S.gdf_in + ci[i]);
+        uu[i] = state_load<kDep>(S.u + ei[i]);
       }
       const float gv = (g[0] * kt[0] + g[1] * kt[1] + g[2] * kt[2]) * iA;
       const float sv = ts[0] * uu[0] * dc[0] + ts[1] * uu[1] * dc[1] + ts[2] * uu[2] * dc[2];
@@ -809,25 +804,15 @@ __device__ __forceinline__ void vertex_body(const DevMesh& M, const StageIO<T>& 
 }
 template <class T, bool kB, int EPT>
 __global__ void __launch_bounds__(kMaxBlock) k_vertex(DevMesh M, StageIO<T> S0, Partials P0, int diag) {
-  vertex_body<T, kB, EPT>(M, S0, P0, diag);
-}
-// the cell and the vertex pass of a small model's stage in one launch: blocks
-// [0, nvb) take the vertices, the others the cells
-template <class T>
-__global__ void __launch_bounds__(kMaxBlock) k_cell_vertex(DevMesh M, ModelOpt O, StageIO<T> S, RKStage rk, Partials P,
-                                                           int diag, int nvb) {
-  if ((int)blockIdx.x < nvb)
-    vertex_body<T, false, 1>(M, S, P, diag);
-  else
-    cell_body<T, false, 1>(M, O, S, rk, P, diag, nvb);
+  vertex_body<T, kB, EPT, false>(M, S0, P0, diag);
 }
 
 // pv on cells: scalar_v2c_interp_operator as a gather (operators_mod.F90:125-141)
-template <class T, int EPT>
+template <class T>
 __global__ void __launch_bounds__(kMaxBlock) k_v2c(DevMesh M, const T* pv_v0, T* pv_c0, long long msv, long long msc) {
   const T* pv_v = pv_v0 + blockIdx.y * msv;
   T* pv_c = pv_c0 + blockIdx.y * msc;
-  TMC_FOR_N(EPT, c, M.nc) {
+  TMC_FOR_EPT(c, M.nc) {
     const T A = T(M.areaCell[c]);
     T s = T(0);
     for (int k = M.v2c_start[c]; k < M.v2c_start[c + 1]; ++k) s = s + pv_v[M.v2c_vertex[k]] * T(M.v2c_kite[k]) / A;
@@ -842,7 +827,7 @@ template <class T, bool kB, int EPT>
 __global__ void __launch_bounds__(kMaxBlock) k_edge_pv(DevMesh M, ModelOpt O, StageIO<T> S0) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const bool need_v = (O.pv_scheme >= 2) || (O.pv_scheme == 1 && O.apvm_weight != 0.0);
-  if constexpr (kPdl<kB, EPT>) {
+  if constexpr (kPdl<T, kB, EPT>) {
     pdl_start();
     if (need_v) pdl_wait();
   }
@@ -857,7 +842,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_edge_pv(DevMesh M, ModelOpt O, St
       v1[j] = e < M.ne ? M.verticesOnEdge[e] : 0;
       v2[j] = e < M.ne ? M.verticesOnEdge[M.ne + e] : 0;
     }
-    if constexpr (kPdl<kB, EPT>) pdl_wait();
+    if constexpr (kPdl<T, kB, EPT>) pdl_wait();
 #pragma unroll
     for (int j = 0; j < EPT; ++j) pe[j] = halve(S.pv_v[v1[j]] + S.pv_v[v2[j]]);
 #pragma unroll
@@ -979,11 +964,10 @@ __device__ __forceinline__ T upwind_sign(const DevMesh& M, const StageIO<T>& S, 
   const int ne = M.ne;
   if constexpr (kF64<T>) {
     const int n = M.nEdgesOnEdge[e];
-    if constexpr (kDep) pdl_wait();
     float s = 0.f, a = 0.f;
 #pragma unroll 5
     for (int i = 0; i < n; ++i) {
-      const float t = __fmul_rn(state_load<kDep>(S.uf + __ldg(M.edgesOnEdge + (size_t)i * ne + e)),
+      const float t = __fmul_rn(__ldg(S.uf + __ldg(M.edgesOnEdge + (size_t)i * ne + e)),
                                 __ldg(M.weightsOnEdge_f + (size_t)i * ne + e));
       s = __fadd_rn(s, t);
       a = __fadd_rn(a, fabsf(t));
@@ -1269,7 +1253,7 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
                                                const Partials& P0) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
-  if constexpr (kPdl<kB, EPT>) pdl_start();
+  if constexpr (kPdl<T, kB, EPT>) pdl_start();
   T rip = T(0), r44 = T(0);  // FP32 path: FP32 products and per-thread sums, FP64 across warps
   constexpr bool kPlain = kMode != kGeneral;
   const int mode = kPlain ? kMode : rk.mode;
@@ -1293,7 +1277,7 @@ __device__ __forceinline__ void edge_flux_body(const DevMesh& M, const ModelOpt&
     } else {
       dc = M.dcEdge[e];
     }
-    if constexpr (kPdl<kB, EPT>) pdl_wait();
+    if constexpr (kPdl<T, kB, EPT>) pdl_wait();
     const T pe = S.pv_e[e];
     T uu = T(0), ge = T(0), sq = T(0), hu = T(0);
     if constexpr (kF64<T>) {
@@ -1475,7 +1459,7 @@ template <class T, bool kB, int EPT>
 __global__ void __launch_bounds__(kMaxBlock) k_final_cells(DevMesh M, ModelOpt O, StageIO<T> S0, const double* diag0) {
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const double* diag = kB ? diag0 + (size_t)blockIdx.y * kDiagStride : diag0;
-  if constexpr (kPdl<kB, EPT>) {
+  if constexpr (kPdl<T, kB, EPT>) {
     pdl_start();
     pdl_wait();
   }
@@ -1535,7 +1519,7 @@ __global__ void __launch_bounds__(kB ? kMemberBlock : kMaxBlock, kB ? TMC_FINAL_
   const StageIO<T> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
   const double* diag = kB ? diag0 + (size_t)blockIdx.y * kDiagStride : diag0;
-  if constexpr (kPdl<kB, EPT>) {
+  if constexpr (kPdl<T, kB, EPT>) {
     pdl_start();
     pdl_wait();
   }
@@ -1667,11 +1651,11 @@ __device__ __forceinline__ void tracer_update_f(const StageIO<float>& S, size_t 
 // kMode as in edge_flux_body; with tracers the constant stages form the mass
 // flux from u and the two cells' gd (whose index the tracers need anyway)
 // instead of gathering it.
-template <int NTR, bool kB, int EPT, int kMode>
+template <int NTR, bool kB, int EPT, int kMode, bool kDep>
 __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<float>& S0, RKStage rk,
                                                const Partials& P0, int diag, int b0 = 0) {
   const int bx = (int)blockIdx.x - b0;  // this block among the cells' blocks
-  if constexpr (kPdl<kB, EPT>) pdl_start();
+  if constexpr (kDep) pdl_start();
   const StageIO<float> S = kB ? S0.at(blockIdx.y) : S0;
   const Partials P = kB ? P0.at(blockIdx.y) : P0;
   constexpr int NQ = NTR > 0 ? NTR : 1;
@@ -1693,7 +1677,7 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
     const float invAf = M.invAreaCell_f[c];
     const float Af = (mode >= 2) ? M.areaCell_f[c] : 0.f;
     float uu[kME], Fv[kME], dv[kME], ae[kME], qn[NQ][kME];
-    if constexpr (kPdl<kB, EPT>) {  // the mesh's values, then the previous kernel's
+    if constexpr (kDep) {  // the mesh's values, then the previous kernel's
 #pragma unroll
       for (int i = 0; i < kME; ++i) {
         dv[i] = M.dvEdge_f[ei[i]];
@@ -1724,7 +1708,7 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
     for (int i = 0; i < kME; ++i) {
       uu[i] = S.u[ei[i]];
       Fv[i] = kPlain && NTR > 0 ? S.gdf_in[ci[i]] : S.F[ei[i]];
-      if constexpr (!kPdl<kB, EPT>) {
+      if constexpr (!kDep) {
         dv[i] = M.dvEdge_f[ei[i]];
         ae[i] = M.areaEdge_f[ei[i]];
       }
@@ -1809,15 +1793,7 @@ __device__ __forceinline__ void cell_fast_body(const DevMesh& M, const StageIO<f
 template <int NTR, int EPT, int kMode>
 __global__ void __launch_bounds__(kCellBlock, TMC_CELL_SINGLE_MIN_BLOCKS) k_cell_fast(DevMesh M, StageIO<float> S0, RKStage rk, Partials P0,
                                                          int diag) {
-  cell_fast_body<NTR, false, EPT, kMode>(M, S0, rk, P0, diag);
-}
-template <int NTR, int kMode>
-__global__ void __launch_bounds__(kCellBlock, TMC_CELL_SINGLE_MIN_BLOCKS) k_cell_vertex_fast(DevMesh M, StageIO<float> S, RKStage rk,
-                                                         Partials P, int diag, int nvb) {
-  if ((int)blockIdx.x < nvb)
-    vertex_body<float, false, 1>(M, S, P, diag);
-  else
-    cell_fast_body<NTR, false, 1, kMode>(M, S, rk, P, diag, nvb);
+  cell_fast_body<NTR, false, EPT, kMode, false>(M, S0, rk, P0, diag);
 }
 // The tracer terms of the FP32 cell pass alone, for a stage whose cell pass
 // ran tracer-free (k_cell_fast<0>): the same loads and the same arithmetic
@@ -1864,7 +1840,7 @@ __global__ void __launch_bounds__(kCellBlock) k_tracers_fast(DevMesh M, StageIO<
 template <int NTR, int kMode>
 __global__ void __launch_bounds__(kMemberBlock, NTR == 0 ? TMC_CELL_MIN_BLOCKS : 3) k_cell_fast_members(DevMesh M, StageIO<float> S0, RKStage rk,
                                                                     Partials P0, int diag) {
-  cell_fast_body<NTR, true, kEPT, kMode>(M, S0, rk, P0, diag);
+  cell_fast_body<NTR, true, kEPT, kMode, false>(M, S0, rk, P0, diag);
 }
 
 template <class T>
@@ -1900,30 +1876,6 @@ void launch_cell(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKSta
   TMC_LAUNCH(k_cell, M.nc, M, O, S, rk, P, diag ? 1 : 0);
 }
 template <class T>
-void launch_cell_vertex(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Partials P, bool diag,
-                        Blk b, cudaStream_t st) {
-  const int nvb = grid_for(M.nv, b), g = nvb + grid_for(M.nc, b), dg = diag ? 1 : 0;
-  if constexpr (!kF64<T>) {
-    auto run = [&](auto ntr) {
-      on_mode(!S.gd_e, rk.mode, [&](auto m) {
-        constexpr int kMode = decltype(m)::value;
-        if constexpr (kMode != 0)
-          launch(k_cell_vertex_fast<decltype(ntr)::value, kMode>, g, b, st, M, S, rk, P, dg, nvb);
-      });
-    };
-    if (launch_cell_is_fast(O)) {
-      switch (O.n_tracers) {
-        case 0: run(std::integral_constant<int, 0>()); return;
-        case 1: run(std::integral_constant<int, 1>()); return;
-        case 2: run(std::integral_constant<int, 2>()); return;
-        case 4: run(std::integral_constant<int, 4>()); return;
-        default: break;
-      }
-    }
-  }
-  launch(k_cell_vertex<T>, g, b, st, M, O, S, rk, P, dg, nvb);
-}
-template <class T>
 void launch_tracers_fast(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, RKStage rk, Blk b,
                          cudaStream_t st) {
   if constexpr (!kF64<T>) {
@@ -1950,7 +1902,7 @@ void launch_vertex(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Par
 template <class T>
 void launch_edge_pv(const DevMesh& M, const ModelOpt& O, const StageIO<T>& S, Blk b, cudaStream_t st) {
   if ((O.pv_scheme == 1 && O.apvm_weight != 0.0) || O.pv_scheme == 2 || O.need_pv_c)
-    k_v2c<T, kEPT><<<dim3(grid_for(M.nc, b.bs), nmem(S)), b.bs, 0, st>>>(M, S.pv_v, S.pv_c, S.msv, S.msc);
+    k_v2c<T><<<dim3(grid_for(M.nc, b.bs), nmem(S)), b.bs, 0, st>>>(M, S.pv_v, S.pv_c, S.msv, S.msc);
   if (M.vfit_n) {
     const int bs = b.bs < 256 ? b.bs : 256;
     const dim3 gv(nblk(M.nv, bs), nmem(S)), ge(nblk(M.ne, bs), nmem(S));
@@ -2053,8 +2005,6 @@ void launch_to_f64(size_t n, const T* src, double* dst, cudaStream_t st) {
 #define TMC_INSTANTIATE_CELL(T) \
   template void launch_cell<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, Partials, bool, Blk, \
                                cudaStream_t);                                                                     \
-  template void launch_cell_vertex<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, Partials, bool, \
-                                      Blk, cudaStream_t);                                                          \
   template void launch_tracers_fast<T>(const DevMesh&, const ModelOpt&, const StageIO<T>&, RKStage, Blk,           \
                                        cudaStream_t);
 
