@@ -61,6 +61,7 @@ struct EngineBase {
   virtual void get_tracers_dev(double* raw_q) = 0;
   virtual void set_ghs_dev(const double* raw) = 0;
   virtual int launches_per_step() const = 0;
+  virtual int closure_tables() { return TMC_OK; }
   virtual void adv_set_initial_dev(const double* raw_q) = 0;  // adv model: gd <- q, wind at t = 0
   virtual void adv_get_dev(double* raw_q, double* raw_u) = 0;
   virtual void state_slot0(void** gd, void** iap, void** q, void** ghs) = 0;  // all members
@@ -899,27 +900,6 @@ struct EnsEngine : EngineBase {
     cdv = h->upload(v_cdv);
     cae = h->upload(v_cae);
     vdc = h->upload(v_vdc);
-    {
-      std::vector<ens::EdgeRec> rec(h->M.ne);
-      const size_t ne_ = h->M.ne;
-#pragma omp parallel for schedule(static)
-      for (int e = 0; e < h->M.ne; ++e) {
-        ens::EdgeRec& r = rec[e];
-        for (int k = 0; k < 10; ++k) {
-          r.e[k] = hm.edgesOnEdge[(size_t)k * ne_ + e];
-          r.w[k] = (float)hm.weightsOnEdge[(size_t)k * ne_ + e];
-        }
-        for (int s = 0; s < 2; ++s) {
-          r.c[s] = hm.cellsOnEdge[(size_t)s * ne_ + e];
-          r.v[s] = hm.verticesOnEdge[(size_t)s * ne_ + e];
-          r.f[s] = (float)hm.fVertex[r.v[s]];
-        }
-        r.dv = (float)hm.dvEdge[e];
-        r.dc = (float)hm.dcEdge[e];
-      }
-      if (!(edge_rec = h->upload(rec))) return TMC_E_CUDA;
-      if (!(v2c_kite = h->upload(std::vector<float>(hm.v2c_kite.begin(), hm.v2c_kite.end())))) return TMC_E_CUDA;
-    }
     if (h->O.pv_scheme == 3) {
       // the weights in FP32, as the FP32 single-model kernel converts them
       std::vector<float> wf(hm.vert2.w.begin(), hm.vert2.w.end());
@@ -970,6 +950,36 @@ struct EnsEngine : EngineBase {
     s.vdc = vdc;
     s.ffs = (size_t)h->M.nc * D.M;
     return s;
+  }
+
+  // the closure's mesh tables, on the first call that needs them (112 bytes per edge)
+  int closure_tables() override {
+    if (edge_rec && v2c_kite) return TMC_OK;
+    const HostMesh& hm = h->hm;
+    const size_t ne = h->M.ne;
+    std::vector<ens::EdgeRec> rec(ne);
+#pragma omp parallel for schedule(static)
+    for (int e = 0; e < h->M.ne; ++e) {
+      ens::EdgeRec& r = rec[e];
+      for (int k = 0; k < 10; ++k) {
+        r.e[k] = hm.edgesOnEdge[(size_t)k * ne + e];
+        r.w[k] = (float)hm.weightsOnEdge[(size_t)k * ne + e];
+      }
+      for (int s = 0; s < 2; ++s) {
+        r.c[s] = hm.cellsOnEdge[(size_t)s * ne + e];
+        r.v[s] = hm.verticesOnEdge[(size_t)s * ne + e];
+        r.f[s] = (float)hm.fVertex[r.v[s]];
+      }
+      r.dv = (float)hm.dvEdge[e];
+      r.dc = (float)hm.dcEdge[e];
+    }
+    if (!edge_rec) edge_rec = h->upload(rec);
+    if (!v2c_kite) v2c_kite = h->upload(std::vector<float>(hm.v2c_kite.begin(), hm.v2c_kite.end()));
+    if (!edge_rec || !v2c_kite) {
+      cudaGetLastError();
+      return h->fail(TMC_E_CUDA, "learned closure: device allocation failed");
+    }
+    return TMC_OK;
   }
 
   int launches_per_step() const override {
@@ -2121,6 +2131,8 @@ int tmc_set_closure(tmc_handle* h, const tmc_mlp* net) {
   if (net && (h->p.precision != TMC_FP32 || h->generic))
     return h->fail(TMC_E_UNSUP, "the learned closure runs in the FP32 CRK4 shallow-water step");
   if (sync(h, "tmc_set_closure")) return TMC_E_CUDA;
+  if (net)
+    if (int rc = h->eng->closure_tables()) return rc;
   h->closure = net;
   if (net) h->closure_net = tmc_mlp_net(net);
   h->O.need_pv_c = net ? 1 : 0;
@@ -2185,6 +2197,7 @@ int tmc_closure_features(tmc_handle* h, float* features, double* pv_edge) {
   if (h->p.precision != TMC_FP32 || h->generic)
     return h->fail(TMC_E_UNSUP, "closure features come from the FP32 CRK4 shallow-water step");
   if (!h->have_state) return h->fail(TMC_E_STATE, "no state set");
+  if (int rc = h->eng->closure_tables()) return rc;
   const int ne = h->M.ne;
   float *d_feat = nullptr, *d_pv = nullptr;
   if (cudaMalloc(&d_feat, sizeof(float) * (size_t)ne * mlp::kIn) != cudaSuccess ||
