@@ -272,12 +272,12 @@ def ensemble_model_bytes(nc: int, ne: int, nv: int, S: int, members: int) -> flo
 
 def inner_ensemble_pass_bytes(nc: int, ne: int, nv: int, members: int) -> dict:
     """Algorithmic bytes per launch of each pass of the member-innermost
-    ensemble step (every array once per pass, gathers at perfect reuse),
-    averaged over the four CRK4 stages: FP32 edge and vertex fields, gd and
-    its RK accumulator double-float (8 bytes), mesh tables once per pass.  A
-    fixed yardstick: the passes have since stopped moving gd_e, the cell pass's
-    F and the edge tendencies of stages 1 and 4 (about 15% of these bytes), so
-    a fraction by this model compares times, not DRAM throughput.
+    ensemble step as it was first built (every array once per pass, gathers at
+    perfect reuse), averaged over the four CRK4 stages: FP32 edge and vertex
+    fields, gd and its RK accumulator double-float (8 bytes), mesh tables once
+    per pass.  The passes have since stopped moving gd_e, the cell pass's F and
+    the edge tendencies of stages 1 and 4: inner_ensemble_moved_bytes has what
+    they move now; this one compares times over the versions.
     Per member and stage (modes 1 / 2-3 / 4):
       cell   u, F 8 Ne; gd old 8, acc 8 / 16 / 8, tend 0 / 4 / 4 in, gd h, ghs 8,
              E 4, acc 8, tend 4, next gd 8 / 8 / 0 out  (+4 Nc gd l on the diag stage)
@@ -298,8 +298,33 @@ def inner_ensemble_pass_bytes(nc: int, ne: int, nv: int, members: int) -> dict:
     return {k: mesh[k] + M * per[k] for k in per}
 
 
-def inner_ensemble_step_bytes(nc: int, ne: int, nv: int, members: int) -> float:
-    b = inner_ensemble_pass_bytes(nc, ne, nv, members)
+def inner_ensemble_moved_bytes(nc: int, ne: int, nv: int, members: int) -> dict:
+    """The same for the passes' present loads and stores.
+    Per member and stage (modes 1 / 2 / 3 / 4):
+      cell   u 4 Ne; gd h and ghs 8, gd old 8 / 8 / 8 / 0, acc 0 / 8 / 8 / 8, tend 0 / 0 / 4 / 4 in,
+             E 4, acc 8, tend 4, next gd 8 / 8 / 8 / 0 out  (+4 Nc gd l on the diag stage)
+      vertex gd h 4 Nc, u 4 Ne in, pv 4 Nv out
+      edge_pv pv 4 Nv in, pv_e 4 Ne out
+      flux   pv_e, u, F 12, tend 0 / 0 / 4 / 4, acc 0 / 4 / 4 / 4, old 4 / 4 / 4 / 0 in, acc 4,
+             tend 0 / 4 / 4 / 0, next u, F 8 / 8 / 8 / 0 out per edge; gd h, E, tend 12 and next
+             gd h 4 / 4 / 4 / 0 per cell
+      final  cells gd r/w 16, acc 8; edges iap r/w 8, acc 4, u, F 8, gd h 4 Nc.
+    Mesh: cell two index tables 48, nSign 6, dvEdge and areaEdge by cell 48, areas 24; vertex 67
+    with dcEdge by vertex 12; flux ten neighbours 80, cells 8, dcEdge, areaEdge 8; final 12."""
+    M = members
+    mesh = {"cell": 126 * nc, "vertex": 79 * nv, "edge_pv": 8 * ne, "edge_flux": 96 * ne, "final": 12 * ne}
+    per = {
+        "cell": (16 * ne + (40 + 48 + 52 + 36) * nc + 4 * nc) / 4.0,
+        "vertex": 4 * nc + 4 * ne + 4 * nv,
+        "edge_pv": 4 * nv + 4 * ne,
+        "edge_flux": ((28 + 36 + 40 + 24) * ne + (16 + 16 + 16 + 12) * nc) / 4.0,
+        "final": 28 * nc + 20 * ne,
+    }
+    return {k: mesh[k] + M * per[k] for k in per}
+
+
+def inner_ensemble_step_bytes(nc: int, ne: int, nv: int, members: int, passes=inner_ensemble_pass_bytes) -> float:
+    b = passes(nc, ne, nv, members)
     return 4 * (b["cell"] + b["vertex"] + b["edge_pv"] + b["edge_flux"]) + b["final"]
 
 
@@ -464,8 +489,8 @@ def run_ensemble(args, local, ics, peak):
            "scope_model_bytes_per_step": mb, "achieved_gbs": mb / step_s / 1e9, "frac": mb / step_s / 1e9 / peak,
            "gpu_launches": launches, "member0_beta": float(d[4]), "block_sizes": tuned}
     if lay == 1:
-        pb = inner_ensemble_pass_bytes(m.nCells, m.nEdges, m.nVertices, M)
-        sb = inner_ensemble_step_bytes(m.nCells, m.nEdges, m.nVertices, M)
+        pb = inner_ensemble_moved_bytes(m.nCells, m.nEdges, m.nVertices, M)
+        sb = inner_ensemble_step_bytes(m.nCells, m.nEdges, m.nVertices, M, inner_ensemble_moved_bytes)
         out["pass_model_bytes_per_step"] = sb
         out["pass_model_frac"] = sb / step_s / 1e9 / peak
         out["passes"] = {k: {"ms_per_launch": passes[k], "algorithmic_bytes_per_launch": pb[k],

@@ -730,7 +730,7 @@ __global__ void __launch_bounds__(kMaxBS) k_ens_edge_pv_up(DevMesh Mh, Dims D, I
 // operators_mod.F90:239-260), the gradient of E and the iap_u tendency
 // (calc_u_tend_on_edge, tmcore_swm_mod.F90:155-201), the RK update of iap_u
 // and the CRK4 inner products (time_scheme_mod.F90:109-154); stages 1-3 also
-// prepare the next stage's gd_edge, u and F from its gd and iap_u.
+// prepare the next stage's u and F from its gd and iap_u.
 // ---------------------------------------------------------------------------
 // The pass is bound by neither memory (DRAM 36%, L2 20%, L1 44% busy) but by
 // the overlap of its load and compute phases at 16 warps per SM, so what counts

@@ -26,11 +26,13 @@
 // stage's edges and the flux pass those of the next stage (prep_edge); small
 // FP32 models run cell and vertex in one launch.
 // Each thread handles kEPT elements (block-strided, so loads stay coalesced),
-// one on a small mesh (Blk).  Global sums (beta, invariants) are per-thread
-// sums and one sum per block; k_finalize adds the blocks' as integers over a
-// common scale, exactly, so in any order: deterministic.  An FP32 pass at one
-// element per thread stores its elements' terms and k_finalize_products sums
-// them in the four-element launch's order.
+// one on a small mesh (Blk).  Global sums (beta, invariants): a thread adds its
+// elements' terms; FP64 lanes and warps are added as integers over a common
+// scale (f64::warp_sum, exact to 64 bits below the largest term), FP32 ones by a
+// shuffle tree; k_finalize's threads add a few blocks' sums each in FP64 and
+// their sums as integers.  Every order is fixed: deterministic.  An FP32 pass at
+// one element per thread stores its elements' terms and k_finalize_products
+// sums them in the four-element launch's order.
 #pragma once
 
 #include <cstdint>
@@ -127,7 +129,8 @@ struct RKStage {
   double a_dt;
 };
 
-// Partial-sum regions (one double-double per block each).
+// Partial-sum regions, one (sum, compensation) pair per block each; the
+// compensation is zero but for compensated FP32 sums (block_store_ff).
 enum Region {
   R_IP_C = 0,  // inner product <t_prev, t> cells   (region + 2*(stage-2))
   R_IP_E = 1,  // inner product edges

@@ -92,10 +92,11 @@ __device__ __forceinline__ void finish_step(const FinalizeArgs& a, const double*
 // per-block partials into P.fin; the last block to finish (atomic counter, no
 // waiting) combines each region's a.split sums (a warp per region) and the
 // region sums into beta and the invariants (time_scheme_mod.F90:144-150;
-// tmcore_swm_mod.F90:215-255), and re-arms the counter.  The sums across
-// lanes are exact integer sums: with double-double shuffle trees on the
-// 2-lane FP64 pipe this launch took 24 us at every mesh size; a level-6 FP32
-// step went from 118.3 to 102.8 us with the integer sums.
+// tmcore_swm_mod.F90:215-255), and re-arms the counter.  A thread adds its few
+// blocks' sums in FP64, the lanes and warps are added as integers: with
+// double-double shuffle trees on the 2-lane FP64 pipe this launch took 24 us at
+// every mesh size; a level-6 FP32 step went from 118.3 to 102.8 us with the
+// integer sums.
 __global__ void __launch_bounds__(256) k_finalize(Partials P0, FinalizeArgs a, double* out0, double* res0,
                                                   unsigned int* counter0) {
   // one member per blockIdx.y: its partials, outputs, region sums and counter
