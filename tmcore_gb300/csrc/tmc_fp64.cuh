@@ -42,7 +42,8 @@ __device__ __forceinline__ double half(double x) {
 // sign * x for a sign of +1, -1 or 0 (an element that lists an edge which is not
 // its own)
 __device__ __forceinline__ double with_sign(double x, int sign) {
-  return __hiloint2double(sign ? __double2hiint(x) ^ (sign & 0x80000000) : 0, sign ? __double2loint(x) : 0);
+  const int mask = -(sign & 1);
+  return __hiloint2double((__double2hiint(x) ^ (sign & 0x80000000)) & mask, __double2loint(x) & mask);
 }
 
 // a / b rounded to nearest from r = RN(1/b), or from r = 0 (which makes it
