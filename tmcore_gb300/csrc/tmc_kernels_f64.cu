@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(256) k_finalize(Partials P0, FinalizeArgs a, d
 
 // The sum of `count` per-block pairs (their lo halves only if kLo, else zero) by
 // one warp, in every lane: K pairs per lane at a time, added exactly
-// (f64::warp_sum).  Level 6 has 41 to 120 pairs per region, level 7 up to 480;
+// (f64::warp_sum).  A region has up to 30 pairs at level 5, 120 at 6, 480 at 7;
 // meshes with more than 32 K add their rounds in double-double.
 template <int K, bool kLo>
 __device__ double region_sum(const double* reg, int count) {
@@ -279,11 +279,13 @@ __global__ void __launch_bounds__(256) k_finalize_products(Partials P, FinalizeA
   for (int q = threadIdx.x >> 5; q < kFinalizeRegions; q += blockDim.x >> 5) {
     const int n = ((q <= R_44_E) ? a.step : a.diag) ? a.counts[q] : 0;
     const double* const reg = P.region(q);
-    double s;
-    if (q <= R_44_E)  // the products' block sums have no lo half
-      s = n <= 4 * 32 ? region_sum<4, false>(reg, n) : region_sum<16, false>(reg, n);
-    else
-      s = n <= 4 * 32 ? region_sum<4, true>(reg, n) : region_sum<16, true>(reg, n);
+    auto sum = [&](auto lo) {  // as little code as the count allows: it runs once, and its fetch counts
+      constexpr bool kLo = decltype(lo)::value;
+      if (n <= 32) return region_sum<1, kLo>(reg, n);
+      return n <= 4 * 32 ? region_sum<4, kLo>(reg, n) : region_sum<16, kLo>(reg, n);
+    };
+    // (the products' block sums have no lo half)
+    const double s = q <= R_44_E ? sum(std::false_type()) : sum(std::true_type());
     if (lane == 0) rs[q] = res[q] = s;
   }
   __syncthreads();
