@@ -430,8 +430,8 @@ def run_mixed(args, local, ics_by_level, peak):
         res[layout] = (el / cycles, members, desc, bytes_cycle, alone, group_mode, by_mode, lanes_ms)
     lay = min(res, key=lambda k: res[k][0])  # the faster layout
     cyc_s, members, desc, bytes_cycle, alone, group_mode, by_mode, lanes_ms = res[lay]
-    pm = sum(2 ** (L - 4) * inner_ensemble_step_bytes(10 * 4 ** L + 2, 30 * 4 ** L,
-                                                                              20 * 4 ** L, len(ics))
+    pm = sum(2 ** (L - 4) * inner_ensemble_step_bytes(10 * 4 ** L + 2, 30 * 4 ** L, 20 * 4 ** L, len(ics),
+                                                      inner_ensemble_moved_bytes)
              for L, ics in ics_by_level.items())
     out = {"workload": "mixed batch " + ", ".join(desc) + ", one CUDA graph per 1200-s cycle",
            "member_layout": lay, "group_mode": group_mode,
