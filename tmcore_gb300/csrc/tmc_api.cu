@@ -1144,19 +1144,21 @@ int build_graph(tmc_handle* h, bool diag, cudaGraphExec_t* out, int first_stage 
   return TMC_OK;
 }
 
-// every edge's two sides belong to one vertex each that lists the edge, once
-// (k_vert_fit writes an edge's side from its vertex)
+// every edge is listed once by each of its two vertices, and the vertices list
+// nothing else (k_vert_fit writes an edge's side from its vertex)
 bool vertices_cover_edges(const HostMesh& hm) {
-  std::vector<uint8_t> seen((size_t)2 * hm.ne, 0);
-  for (int k = 0; k < 3; ++k)
-    for (int v = 0; v < hm.nv; ++v) {
-      const size_t q = (size_t)k * hm.nv + v, e = hm.edgesOnVertex[q];
-      if (hm.tSignEdge[q] == 0) return false;
-      const size_t side = (hm.tSignEdge[q] > 0 ? 0 : (size_t)hm.ne) + e;
-      if (hm.verticesOnEdge[side] != v || seen[side]) return false;
-      seen[side] = 1;
+  if (3 * (long long)hm.nv != 2 * (long long)hm.ne) return false;
+  int bad = 0;
+#pragma omp parallel for schedule(static) reduction(| : bad)
+  for (int e = 0; e < hm.ne; ++e)
+    for (int side = 0; side < 2; ++side) {
+      const size_t v = hm.verticesOnEdge[(size_t)side * hm.ne + e];
+      int listed = 0;
+      for (size_t k = 0; k < 3; ++k)
+        listed += hm.edgesOnVertex[k * hm.nv + v] == e && hm.tSignEdge[k * hm.nv + v] == (side ? -1 : 1);
+      bad |= listed != 1;
     }
-  return std::find(seen.begin(), seen.end(), 0) == seen.end();
+  return !bad;
 }
 
 // partial counts per region: the grid of the passes that write it
