@@ -1032,12 +1032,12 @@ __device__ __forceinline__ void ens_reduce(const Partials& P, int r, int count, 
     double v[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) v[q] = widen(sf[at(q, lane, w)]);
-    tot = f64::value(f64::warp_sum<8>(v));
+    tot = f64::value(f64::warp_sum(v));
   } else {
     double v[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) v[q] = sh[q][lane][w];
-    tot = f64::value(f64::warp_sum<4>(v));
+    tot = f64::value(f64::warp_sum(v));
   }
   const int mm = blockIdx.y * 32 + w;
   if (lane == 0 && mm < P.M) diag_out[(size_t)mm * kDiagStride + kDiagLen + r] = tot;

@@ -167,29 +167,26 @@ __device__ __forceinline__ double value(const Fixed& f) {
   return v.hi + v.lo;
 }
 
-// the sum over the warp of each lane's N terms, in every lane (all 32 lanes
-// call).  Many terms go through a loop: unrolled, 32 of them are 13 KB of code
-// that runs once, and fetching it took a level-7 step 2.4 us.
-template <int N>
-__device__ __forceinline__ Fixed warp_sum(const double (&v)[N]) {
-  static_assert(N <= 64, "the lanes' sums leave room for 6 bits above 32 terms");
-  constexpr int kUnroll = N <= 8 ? N : 1;
+// the sum over the warp of each lane's n <= 64 terms (the limbs leave 6 bits above
+// 32 terms), in every lane; all 32 lanes call, with the same n
+template <int kUnroll>
+__device__ __forceinline__ Fixed warp_sum(const double* v, int n) {
   const unsigned all = 0xffffffffu;
   int ex = 0;
 #pragma unroll kUnroll
-  for (int k = 0; k < N; ++k) ex = max(ex, (__double2hiint(v[k]) >> 20) & 0x7ff);
+  for (int k = 0; k < n; ++k) ex = max(ex, (__double2hiint(v[k]) >> 20) & 0x7ff);
   const int e = (int)__reduce_max_sync(all, (unsigned)ex);
   if ((unsigned)(e - 200) > 1700u) {  // zeros, extreme exponents, infinities, NaN: in FP64
-    double t = v[0];
+    double t = 0.0;
 #pragma unroll kUnroll
-    for (int k = 1; k < N; ++k) t += v[k];
+    for (int k = 0; k < n; ++k) t += v[k];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(all, t, off);
     return {(__int128)__double_as_longlong(t), -1};
   }
   unsigned __int128 acc = 0;
 #pragma unroll kUnroll
-  for (int k = 0; k < N; ++k) {
+  for (int k = 0; k < n; ++k) {
     const int hi = __double2hiint(v[k]), x = (hi >> 20) & 0x7ff;
     long long m = (long long)(((unsigned long long)(unsigned)(hi & 0xfffff) << 32) | (unsigned)__double2loint(v[k]));
     if (x) m |= 1ll << 52;
@@ -215,9 +212,13 @@ __device__ __forceinline__ Fixed warp_sum(const double (&v)[N]) {
                               ((unsigned __int128)s3 << 78) + ((unsigned __int128)(__int128)s4 << 104);
   return {(__int128)s, e};
 }
+template <int N>
+__device__ __forceinline__ Fixed warp_sum(const double (&v)[N]) {
+  return warp_sum<N>(v, N);
+}
 __device__ __forceinline__ Fixed warp_sum(double v) {
   const double t[1] = {v};
-  return warp_sum<1>(t);
+  return warp_sum(t);
 }
 
 }  // namespace f64

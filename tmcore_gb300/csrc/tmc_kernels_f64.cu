@@ -138,28 +138,29 @@ __global__ void __launch_bounds__(256) k_finalize(Partials P0, FinalizeArgs a, d
   if (threadIdx.x == 0) *counter = 0u;
 }
 
-// The sum of `count` per-block pairs (their lo halves only if kLo, else zero) by
-// one warp, in every lane: K pairs per lane at a time, added exactly
-// (f64::warp_sum).  A region has up to 30 pairs at level 5, 120 at 6, 480 at 7;
-// meshes with more than 32 K add their rounds in double-double.
-template <int K, bool kLo>
-__device__ double region_sum(const double* reg, int count) {
+// The sum of `count` per-block pairs (their lo halves only if `lo`, else they are
+// zero) by one warp, in every lane: up to 16 pairs per lane at a time, added
+// exactly (f64::warp_sum).  A region has up to 30 pairs at level 5, 120 at 6, 480
+// at 7; meshes with more than 512 add their rounds in double-double.  The terms
+// go through a loop: this code runs once per step and region, and what counts is
+// its fetch (16 pairs unrolled took a level-7 step 2.4 us, one unrolled form per
+// number of pairs a level-6 step 1.9 us).
+__device__ __forceinline__ double region_sum(const double* reg, int count, bool lo) {
+  constexpr int K = 16;
   const int lane = threadIdx.x & 31;
   f64::HiLo sum{0.0, 0.0};
   for (int i0 = 0; i0 < count; i0 += 32 * K) {
-    double t[kLo ? 2 * K : K];
+    const int m = min(K, (count - i0 + 31) / 32);  // pairs of a lane
+    double t[2 * K];
+    for (int k0 = 0; k0 < m; k0 += 8)  // eight loads in flight
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int i = i0 + 32 * k + lane;
-      if constexpr (kLo) {
+      for (int k = k0; k < k0 + 8; ++k) {
+        const int i = i0 + 32 * k + lane;
         const double2 p = i < count ? __ldcg(reinterpret_cast<const double2*>(reg) + i) : make_double2(0.0, 0.0);
-        t[k] = p.x;
-        t[K + k] = p.y;
-      } else {
-        t[k] = i < count ? __ldcg(reg + 2 * (size_t)i) : 0.0;
+        t[lo ? 2 * k : k] = p.x;
+        if (lo) t[2 * k + 1] = p.y;
       }
-    }
-    const f64::HiLo r = f64::split(f64::warp_sum(t));
+    const f64::HiLo r = f64::split(f64::warp_sum<1>(t, lo ? 2 * m : m));
     if (i0 == 0) {
       sum = r;
     } else {  // TwoSum (Knuth)
@@ -276,16 +277,19 @@ __global__ void __launch_bounds__(256) k_finalize_products(Partials P, FinalizeA
   __threadfence();
   __shared__ double rs[kFinalizeRegions];
   const int lane = threadIdx.x & 31;
-  for (int q = threadIdx.x >> 5; q < kFinalizeRegions; q += blockDim.x >> 5) {
-    const int n = ((q <= R_44_E) ? a.step : a.diag) ? a.counts[q] : 0;
-    const double* const reg = P.region(q);
-    auto sum = [&](auto lo) {  // as little code as the count allows: it runs once, and its fetch counts
-      constexpr bool kLo = decltype(lo)::value;
-      if (n <= 32) return region_sum<1, kLo>(reg, n);
-      return n <= 4 * 32 ? region_sum<4, kLo>(reg, n) : region_sum<16, kLo>(reg, n);
-    };
-    // (the products' block sums have no lo half)
-    const double s = q <= R_44_E ? sum(std::false_type()) : sum(std::true_type());
+  // warp w: the products' region w, whose block sums have no lo half, then an
+  // invariant (in warps whose first region is the cells', a third of the edges)
+  static_assert(R_44_E == 7 && kFinalizeRegions == 13, "eight warps, five invariants");
+  constexpr unsigned kNone = 15, kSecond = (unsigned)R_EN_E | kNone << 4 | (unsigned)R_PE << 8 |
+                                           (unsigned)R_EN_C << 12 | (unsigned)R_AV << 16 | kNone << 20 |
+                                           (unsigned)R_MASS << 24 | kNone << 28;
+  const unsigned warp = threadIdx.x >> 5;
+#pragma unroll 1
+  for (int round = 0; round < 2; ++round) {
+    const unsigned q = round ? kSecond >> (4 * warp) & 15u : warp;
+    if (q == kNone) break;
+    const int n = (round ? a.diag : a.step) ? a.counts[q] : 0;
+    const double s = region_sum(P.region(q), n, round != 0);
     if (lane == 0) rs[q] = res[q] = s;
   }
   __syncthreads();
